@@ -33,37 +33,47 @@ namespace iskra {
 // in push_t8.cu and push_t32.cu
 ISKRA_PUSH_TILE_TU(4, t16)
 cudaError_t push_tile_one_t8(cudaStream_t, bool, bool, const SpeciesDev &, const float2 *, const PushParams &, int,
-                             int, int *);
+                             int, int, int *);
 cudaError_t push_tile_two_t8(cudaStream_t, bool, const SpeciesDev &, const SpeciesDev &, const float2 *,
-                             const PushParams &, const PushParams &, int, int, int *, unsigned long long *);
+                             const PushParams &, const PushParams &, int, int, int, int *, unsigned long long *);
 cudaError_t push_tile_one_t32(cudaStream_t, bool, bool, const SpeciesDev &, const float2 *, const PushParams &, int,
-                              int, int *);
+                              int, int, int *);
 cudaError_t push_tile_two_t32(cudaStream_t, bool, const SpeciesDev &, const SpeciesDev &, const float2 *,
-                              const PushParams &, const PushParams &, int, int, int *, unsigned long long *);
+                              const PushParams &, const PushParams &, int, int, int, int *, unsigned long long *);
 
 cudaError_t push_tile_one(int ts, cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2,
-                          const PushParams &P, int ntiles, int blocks, int *err) {
+                          const PushParams &P, int ntiles, int parts, int blocks, int *err) {
   switch (ts) {
-    case 3: return push_tile_one_t8(st, push, trk, s, E2, P, ntiles, blocks, err);
-    case 4: return push_tile_one_t16(st, push, trk, s, E2, P, ntiles, blocks, err);
-    case 5: return push_tile_one_t32(st, push, trk, s, E2, P, ntiles, blocks, err);
+    case 3: return push_tile_one_t8(st, push, trk, s, E2, P, ntiles, parts, blocks, err);
+    case 4: return push_tile_one_t16(st, push, trk, s, E2, P, ntiles, parts, blocks, err);
+    case 5: return push_tile_one_t32(st, push, trk, s, E2, P, ntiles, parts, blocks, err);
   }
   return cudaErrorInvalidValue;
 }
 
 cudaError_t push_tile_two(int ts, cudaStream_t st, bool trk, const SpeciesDev &a, const SpeciesDev &b,
-                          const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles, int blocks,
+                          const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles, int parts, int blocks,
                           int *err, unsigned long long *step_ctr) {
   switch (ts) {
-    case 3: return push_tile_two_t8(st, trk, a, b, E2, Pa, Pb, ntiles, blocks, err, step_ctr);
-    case 4: return push_tile_two_t16(st, trk, a, b, E2, Pa, Pb, ntiles, blocks, err, step_ctr);
-    case 5: return push_tile_two_t32(st, trk, a, b, E2, Pa, Pb, ntiles, blocks, err, step_ctr);
+    case 3: return push_tile_two_t8(st, trk, a, b, E2, Pa, Pb, ntiles, parts, blocks, err, step_ctr);
+    case 4: return push_tile_two_t16(st, trk, a, b, E2, Pa, Pb, ntiles, parts, blocks, err, step_ctr);
+    case 5: return push_tile_two_t32(st, trk, a, b, E2, Pa, Pb, ntiles, parts, blocks, err, step_ctr);
   }
   return cudaErrorInvalidValue;
 }
 
-// one block per tile plus a grid-stride set for the unsorted tail
-static int push_blocks(Ctx *c) { return c->ntiles + c->num_sms; }
+// Blocks per tile of a push of nsp species: one where the tiles fill the
+// resident block slots of the chip; on grids of fewer tiles the particles of
+// a tile are split over as many blocks as the slots allow (a block takes at
+// least kPartMin of them, the others return at once).  One block per tile
+// left a 257 x 2 grid's push to 32 blocks of 6.5 k particles each (31 us, the
+// length of one block's serial pass): the step of that discharge (105 k + 105 k
+// particles) 126 -> 103 us, a 10 x 10 grid's (one tile, 20 k) 179 -> 146 us.
+static int push_parts(Ctx *c, int nsp) {
+  return std::max(1, std::min(64, c->num_sms * ISKRA_PUSH_MIN_BLOCKS / std::max(1, nsp * c->ntiles)));
+}
+// the tile blocks plus a grid-stride set for the unsorted tail
+static int push_blocks(Ctx *c, int nsp, int parts) { return nsp * c->ntiles * parts + c->num_sms; }
 
 static int sort_blocks(Ctx *c, Species &s) {
   long long want = (s.cap + 255) / 256;
@@ -113,8 +123,9 @@ int launch_advance(Ctx *c, int sid, float dt) {
   Species &s = c->species[sid];
   int rc = clear_acc(c, s);
   if (rc) return rc;
+  const int parts = push_parts(c, 1);
   ISKRA_CUDA(c, push_tile_one(c->tile_shift, c->stream, true, c->trk != nullptr, s.dev, c->E32, push_params(c, s, dt),
-                              c->ntiles, push_blocks(c), c->d_err));
+                              c->ntiles, parts, push_blocks(c, 1, parts), c->d_err));
   ISKRA_CUDA(c, cudaGetLastError());
   mark_pushed(s);
   return launch_surface_charge(c);  // hit! of floating electrodes, as part of advance!
@@ -132,9 +143,9 @@ int launch_advance_all(Ctx *c, float dt, unsigned long long *step_ctr, bool *fol
     if (!rc) rc = clear_acc(c, b);
     if (rc) return rc;
     const PushParams Pa = push_params(c, a, dt), Pb = push_params(c, b, dt);
-    const int blocks = 2 * c->ntiles + c->num_sms;
+    const int parts = push_parts(c, 2);
     ISKRA_CUDA(c, push_tile_two(c->tile_shift, c->stream, c->trk != nullptr, a.dev, b.dev, c->E32, Pa, Pb, c->ntiles,
-                                blocks, c->d_err, step_ctr));
+                                parts, push_blocks(c, 2, parts), c->d_err, step_ctr));
     ISKRA_CUDA(c, cudaGetLastError());
     mark_pushed(a);
     mark_pushed(b);
@@ -158,8 +169,9 @@ int launch_deposit(Ctx *c, int sid) {
   P.nx = c->nx;
   P.ny = c->ny;
   P.tiles_x = c->tiles_x;
-  ISKRA_CUDA(c, push_tile_one(c->tile_shift, c->stream, false, false, s.dev, c->E32, P, c->ntiles, push_blocks(c),
-                              c->d_err));
+  const int parts = push_parts(c, 1);
+  ISKRA_CUDA(c, push_tile_one(c->tile_shift, c->stream, false, false, s.dev, c->E32, P, c->ntiles, parts,
+                              push_blocks(c, 1, parts), c->d_err));
   ISKRA_CUDA(c, cudaGetLastError());
   s.acc_valid = true;
   s.acc_zero = false;

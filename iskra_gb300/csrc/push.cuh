@@ -203,6 +203,13 @@ __device__ __forceinline__ int apply_boundary(int &i, int P) {
 #ifndef ISKRA_PUSH_STAGES
 #define ISKRA_PUSH_STAGES 4
 #endif
+// Fewest particles worth a block of their own when a tile's particles are
+// split over several blocks (push_block): a block's staging of its window
+// and its node sums cost about what the push of a few hundred particles does.
+#ifndef ISKRA_PUSH_PART_MIN
+#define ISKRA_PUSH_PART_MIN 384
+#endif
+constexpr int kPartMin = ISKRA_PUSH_PART_MIN;
 // Each warp of a tile block streams its slice of particle records through a
 // ring of kStages shared-memory stages filled by asynchronous copies
 // (cp.async): kStages - 1 warp iterations (768 B each) are in flight while
@@ -552,15 +559,16 @@ __device__ __forceinline__ void push_warp(const SpeciesDev &s, float4 *__restric
 }
 
 // One block of the push: a tile block (tile >= 0) takes the particles the
-// last sort grouped in its tile: stage E at the window's nodes, push (each
+// last sort grouped in its tile -- all of them, or slice `part` of at most
+// `parts` of at least kPartMin particles: stage E at the window's nodes, push (each
 // warp a contiguous slice, streamed through its record ring), deposit into
 // the window, then add the window's nonzero node sums and cell counts to
-// the global accumulators.  A tail block (tile < 0, tail_block of
-// tail_blocks) walks the slots appended since that sort.  Integer sums: the
+// the global accumulators.  A tail block (tile < 0, `part` of `parts` tail
+// blocks) walks the slots appended since that sort.  Integer sums: the
 // density is the same bit for bit whichever block adds what.
 template <bool PUSH, int MX, int MY, bool TRK, int TS>
 __device__ __forceinline__ void push_block(const SpeciesDev &s, const PushParams &P, const float2 *__restrict__ E2,
-                                           TileShared<TS> &sh, int tile, int tail_block, int tail_blocks, int *err) {
+                                           TileShared<TS> &sh, int tile, int part, int parts, int *err) {
   constexpr int kWin = TileShared<TS>::kWin, kWinN = TileShared<TS>::kWinN, kWinCells = TileShared<TS>::kWinCells;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
@@ -571,7 +579,14 @@ __device__ __forceinline__ void push_block(const SpeciesDev &s, const PushParams
   int flags = 0;
   const int nx = P.nx;
   if (tile >= 0) {
-    const long long begin = s.tile_begin[tile], end = s.tile_begin[tile + 1];
+    long long begin = s.tile_begin[tile], end = s.tile_begin[tile + 1];
+    if (parts > 1) {  // slices in multiples of 32 slots
+      const long long len = end - begin;
+      const long long use = min((long long)parts, (len + kPartMin - 1) / kPartMin);
+      const long long slice = use > 0 ? ((len + use * 32 - 1) / (use * 32)) * 32 : 0;
+      begin += part * slice;
+      end = part < use ? min(end, begin + slice) : begin;
+    }
     if (begin < end) {  // block-uniform
       const int ox = ((tile % P.tiles_x) << TS) - kHalo, oy = ((tile / P.tiles_x) << TS) - kHalo;
       if (PUSH) {
@@ -755,8 +770,8 @@ __device__ __forceinline__ void push_block(const SpeciesDev &s, const PushParams
     }
   } else {
     const long long np = s.st->np, t0 = s.st->sorted_n;
-    const long long warp = (long long)tail_block * nwb + wib;
-    const long long nwarps = (long long)tail_blocks * nwb;
+    const long long warp = (long long)part * nwb + wib;
+    const long long nwarps = (long long)parts * nwb;
     for (long long base = t0 + warp * 32; base < np; base += nwarps * 32) {
       const long long p = base + lane;
       const bool v = p < np;
@@ -784,39 +799,39 @@ __device__ __forceinline__ void push_block(const SpeciesDev &s, const PushParams
 // registers out of the push without one)
 template <bool PUSH, int MX, int MY, bool TRK, int TS>
 __global__ void __launch_bounds__(kPushBlock, TRK ? ISKRA_PUSH_TRK_MIN_BLOCKS : ISKRA_PUSH_MIN_BLOCKS)
-    k_push(SpeciesDev s, const float2 *__restrict__ E2, PushParams P, int ntiles, int *err) {
+    k_push(SpeciesDev s, const float2 *__restrict__ E2, PushParams P, int ntiles, int parts, int *err) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char push_smem[];
   TileShared<TS> &sh = *reinterpret_cast<TileShared<TS> *>(push_smem);
-  const int b = blockIdx.x;
-  if (b < ntiles) push_block<PUSH, MX, MY, TRK, TS>(s, P, E2, sh, b, 0, 0, err);
-  else push_block<PUSH, MX, MY, TRK, TS>(s, P, E2, sh, -1, b - ntiles, gridDim.x - ntiles, err);
+  const int b = blockIdx.x, nt = ntiles * parts;
+  if (b < nt) push_block<PUSH, MX, MY, TRK, TS>(s, P, E2, sh, b / parts, b % parts, parts, err);
+  else push_block<PUSH, MX, MY, TRK, TS>(s, P, E2, sh, -1, b - nt, gridDim.x - nt, err);
 }
 
 // Two species in one launch (the step's electrons and ions): their pushes
 // are independent until ρ is formed, so the second species' tiles fill the
 // SMs as the first species' tiles drain instead of waiting for a second
-// launch.  Blocks [0, ntiles) first species' tiles, [ntiles, 2 ntiles) the
-// second's, the rest both tails.
+// launch.  Blocks [0, ntiles parts) first species' tiles, the next as many
+// the second's, the rest both tails.
 // step_ctr (optional): the step counter, advanced here when no MCC set reads
 // it earlier in the step (saves the step's opening launch).
 template <int MX, int MY, bool TRK, int TS>
 __global__ void __launch_bounds__(kPushBlock, TRK ? ISKRA_PUSH_TRK_MIN_BLOCKS : ISKRA_PUSH_MIN_BLOCKS)
     k_push2(SpeciesDev s0, SpeciesDev s1, const float2 *__restrict__ E2, PushParams P0, PushParams P1, int ntiles,
-            int *err, unsigned long long *step_ctr) {
+            int parts, int *err, unsigned long long *step_ctr) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char push_smem[];
   TileShared<TS> &sh = *reinterpret_cast<TileShared<TS> *>(push_smem);
-  const int b = blockIdx.x;
+  const int b = blockIdx.x, nt = ntiles * parts;
   if (step_ctr && b == 0 && threadIdx.x == 0) *step_ctr += 1ull;
-  if (b < ntiles) {
-    push_block<true, MX, MY, TRK, TS>(s0, P0, E2, sh, b, 0, 0, err);
-  } else if (b < 2 * ntiles) {
-    push_block<true, MX, MY, TRK, TS>(s1, P1, E2, sh, b - ntiles, 0, 0, err);
+  if (b < nt) {
+    push_block<true, MX, MY, TRK, TS>(s0, P0, E2, sh, b / parts, b % parts, parts, err);
+  } else if (b < 2 * nt) {
+    push_block<true, MX, MY, TRK, TS>(s1, P1, E2, sh, (b - nt) / parts, (b - nt) % parts, parts, err);
   } else {
-    const int tb = b - 2 * ntiles, nt = gridDim.x - 2 * ntiles;
-    push_block<true, MX, MY, TRK, TS>(s0, P0, E2, sh, -1, tb, nt, err);
-    push_block<true, MX, MY, TRK, TS>(s1, P1, E2, sh, -1, tb, nt, err);
+    const int tb = b - 2 * nt, tails = gridDim.x - 2 * nt;
+    push_block<true, MX, MY, TRK, TS>(s0, P0, E2, sh, -1, tb, tails, err);
+    push_block<true, MX, MY, TRK, TS>(s1, P1, E2, sh, -1, tb, tails, err);
   }
 }
 
@@ -835,17 +850,17 @@ struct PushTile {
   }
   // one species: push (push = true) or deposit only
   static cudaError_t one(cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2,
-                         const PushParams &P, int ntiles, int blocks, int *err) {
+                         const PushParams &P, int ntiles, int parts, int blocks, int *err) {
     if (!push) {
       auto kern = k_push<false, 0, 0, false, TS>;
       prepare(kern);
-      return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, err);
+      return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, parts, err);
     }
 #define ISKRA_PUSH_CASE(MX, MY)                                                                \
   if (P.mode_x == MX && P.mode_y == MY) {                                                      \
     auto kern = trk ? k_push<true, MX, MY, true, TS> : k_push<true, MX, MY, false, TS>;        \
     prepare(kern);                                                                             \
-    return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, err);             \
+    return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, parts, err);             \
   }
     ISKRA_PUSH_CASE(0, 0) ISKRA_PUSH_CASE(0, 1) ISKRA_PUSH_CASE(0, 2)
     ISKRA_PUSH_CASE(1, 0) ISKRA_PUSH_CASE(1, 1) ISKRA_PUSH_CASE(1, 2)
@@ -855,13 +870,13 @@ struct PushTile {
   }
   // two species with the same boundary rules in one launch
   static cudaError_t two(cudaStream_t st, bool trk, const SpeciesDev &a, const SpeciesDev &b, const float2 *E2,
-                         const PushParams &Pa, const PushParams &Pb, int ntiles, int blocks, int *err,
+                         const PushParams &Pa, const PushParams &Pb, int ntiles, int parts, int blocks, int *err,
                          unsigned long long *step_ctr) {
 #define ISKRA_PUSH2_CASE(MX, MY)                                                                          \
   if (Pa.mode_x == MX && Pa.mode_y == MY) {                                                               \
     auto kern = trk ? k_push2<MX, MY, true, TS> : k_push2<MX, MY, false, TS>;                             \
     prepare(kern);                                                                                        \
-    return launch_pdl(kern, blocks, kPushBlock, kSmem, st, a, b, E2, Pa, Pb, ntiles, err, step_ctr);         \
+    return launch_pdl(kern, blocks, kPushBlock, kSmem, st, a, b, E2, Pa, Pb, ntiles, parts, err, step_ctr);         \
   }
     ISKRA_PUSH2_CASE(0, 0) ISKRA_PUSH2_CASE(0, 1) ISKRA_PUSH2_CASE(0, 2)
     ISKRA_PUSH2_CASE(1, 0) ISKRA_PUSH2_CASE(1, 1) ISKRA_PUSH2_CASE(1, 2)
@@ -873,19 +888,19 @@ struct PushTile {
 
 // entry points of the per-tile-size translation units
 cudaError_t push_tile_one(int ts, cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2,
-                          const PushParams &P, int ntiles, int blocks, int *err);
+                          const PushParams &P, int ntiles, int parts, int blocks, int *err);
 cudaError_t push_tile_two(int ts, cudaStream_t st, bool trk, const SpeciesDev &a, const SpeciesDev &b,
-                          const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles, int blocks,
+                          const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles, int parts, int blocks,
                           int *err, unsigned long long *step_ctr);
 #define ISKRA_PUSH_TILE_TU(TS, NAME)                                                                          \
   cudaError_t push_tile_one_##NAME(cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2, \
-                                   const PushParams &P, int ntiles, int blocks, int *err) {                    \
-    return PushTile<TS>::one(st, push, trk, s, E2, P, ntiles, blocks, err);                                    \
+                                   const PushParams &P, int ntiles, int parts, int blocks, int *err) {                    \
+    return PushTile<TS>::one(st, push, trk, s, E2, P, ntiles, parts, blocks, err);                                    \
   }                                                                                                            \
   cudaError_t push_tile_two_##NAME(cudaStream_t st, bool trk, const SpeciesDev &a, const SpeciesDev &b,         \
                                    const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles,   \
-                                   int blocks, int *err, unsigned long long *step_ctr) {                       \
-    return PushTile<TS>::two(st, trk, a, b, E2, Pa, Pb, ntiles, blocks, err, step_ctr);                        \
+                                   int parts, int blocks, int *err, unsigned long long *step_ctr) {            \
+    return PushTile<TS>::two(st, trk, a, b, E2, Pa, Pb, ntiles, parts, blocks, err, step_ctr);                        \
   }
 
 }  // namespace iskra
