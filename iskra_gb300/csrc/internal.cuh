@@ -324,6 +324,7 @@ struct Species {
   bool acc_valid = false;      // acc holds the unconsumed deposit of the current positions
   bool acc_zero = true;        // acc is all zero
   bool n_valid = true;         // n matches the current positions
+  long long tail = 0;          // at most this many particles sampled outside steps since the last sort
 };
 
 struct Poisson;                // poisson.cu

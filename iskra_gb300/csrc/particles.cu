@@ -605,6 +605,7 @@ int launch_sort(Ctx *c, int sid) {
   k_scatter<<<blocks, 256, 0, c->stream>>>(s.dev, c->tiles_x, c->tile_shift, c->cell_cursor);
   k_sort_finish<<<1, 1, 0, c->stream>>>(s.dev.st, c->cell_count + nk);
   ISKRA_CUDA(c, cudaGetLastError());
+  s.tail = 0;
   return ISKRA_OK;
 }
 

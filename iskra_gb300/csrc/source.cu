@@ -194,7 +194,9 @@ int iskra_source_sample(iskra_ctx *h, int src, double dt, uint64_t seed) {
   Source &S = sources_of(c)[src];
   // one-off samples take their call number as the step word, with the top
   // bit set so they never share a key with a step's sample
-  return launch_source(c, src, dt, seed, nullptr, (1ull << 63) | S.calls++);
+  const int rc = launch_source(c, src, dt, seed, nullptr, (1ull << 63) | S.calls++);
+  if (rc == ISKRA_OK) c->species[S.sid].tail += std::max(0LL, (long long)std::floor(S.rate * dt));
+  return rc;
 }
 
 int iskra_source_set_every_step(iskra_ctx *h, int src, int on) {

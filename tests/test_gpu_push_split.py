@@ -43,3 +43,32 @@ def test_split_tiles_match_the_oracle(orc, lib, nx, ny, n):
     ref = orc.density(nx, ny, dx, dx, np.asfortranarray(x1), w, (0, 0, 0, 0))
     assert np.max(np.abs(dens - ref)) <= 1e-9 * np.max(np.abs(ref))
     ctx.close()
+
+
+@pytest.mark.parametrize("n,cap", [(65535, 70000), (65536, 70000), (65536, 8 * 65536), (65536, 8 * 65536 + 1)])
+def test_steps_after_a_source_fill_do_not_depend_on_its_sort(lib, n, cap):
+    """A species filled by a source is sorted once before its first step when
+    the fill is large (at least 65536 particles and an eighth of the
+    capacity): same fields, bit for bit, as with an explicit sort or none."""
+    out = []
+    for how in ("auto", "sorted", "never"):
+        ctx = make_ctx(65, 33, 1e-4, 1e-4)
+        sid = ctx.species_create(-QE, ME, 1e3, cap)
+        ctx.set_boundary(sid, lib.BND_DISCARD, lib.BND_WRAP)
+        src = ctx.source_create(sid, (n + 0.5) / 1e-11, [64e-4, 32e-4], [6e5, 6e5, 6e5])
+        ctx.source_sample(src, 1e-11, seed=5)
+        ctx.poisson_create(8.8541878128e-12)
+        col = np.zeros((65, 33), bool)
+        col[0, :] = True
+        ctx.apply_dirichlet(col, 0.0)
+        if how == "sorted":
+            ctx.sort(sid)
+        if how == "never":
+            ctx.set_sort_every(0)
+        ctx.step(1e-11, 3, seed=1, rtol=1e-8)
+        x, v, _ = by_id(*ctx.download(sid))
+        out.append((x, v, ctx.field(lib.FIELD_RHO), ctx.field(lib.FIELD_PHI)))
+        ctx.close()
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert np.array_equal(a, b)
