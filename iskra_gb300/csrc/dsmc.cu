@@ -468,6 +468,7 @@ int iskra_dsmc_create(iskra_ctx *h, int source, int target, const double *g, con
   ISKRA_CUDA(c, cudaMemcpy(d->d_tab, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
   ISKRA_CUDA(c, cudaMemset(d->remaining, 0, nn * sizeof(double)));
   ISKRA_CUDA(c, cudaMemset(d->nu, 0, nn * sizeof(unsigned)));
+  ISKRA_CUDA(c, setup_copies_done());
   if (!c->dsmcs) {
     c->dsmcs = new (std::nothrow) std::vector<Dsmc *>();
     if (!c->dsmcs) {

@@ -371,7 +371,7 @@ static int ens_update_keys(Ens *e) {
   for (int m = 0; m < (int)e->mcc.size(); m++) {
     std::vector<uint2> k(e->R);
     for (int r = 0; r < e->R; r++) mcc_key(e->seeds[r], mcc_set_index(e->c, m), k[r].x, k[r].y);
-    ENS_CUDA(e, cudaMemcpy(e->mcc[m].keys, k.data(), e->R * sizeof(uint2), cudaMemcpyHostToDevice));
+    ENS_CUDA(e, cudaMemcpyAsync(e->mcc[m].keys, k.data(), e->R * sizeof(uint2), cudaMemcpyHostToDevice, e->c->stream));
   }
   e->keys_valid = true;
   return ISKRA_OK;
@@ -528,7 +528,7 @@ int iskra_ens_set_drive_amplitude(iskra_ens *h, int group, const double *amp) {
   std::vector<double> a((size_t)e->R * e->ngroups);
   ENS_CUDA(e, cudaMemcpy(a.data(), e->amp, a.size() * sizeof(double), cudaMemcpyDeviceToHost));
   for (int r = 0; r < e->R; r++) a[(size_t)r * e->ngroups + group] = amp[r];
-  ENS_CUDA(e, cudaMemcpy(e->amp, a.data(), a.size() * sizeof(double), cudaMemcpyHostToDevice));
+  ENS_CUDA(e, cudaMemcpyAsync(e->amp, a.data(), a.size() * sizeof(double), cudaMemcpyHostToDevice, e->c->stream));
   return ISKRA_OK;
 }
 
@@ -552,7 +552,7 @@ int iskra_ens_upload(iskra_ens *h, int run, int sid, const double *x, const doub
   if (id)
     for (int64_t p = 0; p < np; p++) maxid = std::max(maxid, id[p]);
   s0.next_id = maxid + 1;
-  ENS_CUDA(e, cudaMemcpy(q.st + run, &s0, sizeof(s0), cudaMemcpyHostToDevice));
+  ENS_CUDA(e, cudaMemcpyAsync(q.st + run, &s0, sizeof(s0), cudaMemcpyHostToDevice, e->c->stream));
   return ISKRA_OK;
 }
 

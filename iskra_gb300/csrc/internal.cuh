@@ -515,6 +515,13 @@ inline cudaError_t launch_pdl(void (*kern)(K...), dim3 grid, dim3 block, size_t 
   return cudaLaunchKernelEx(&cfg, kern, static_cast<A &&>(args)...);
 }
 
+// Copies and memsets of a setup call run on the legacy stream, which the
+// (non-blocking) stream of a context does not wait for, and cudaMemcpy of up
+// to 64 KB of pageable memory returns before the device has the data: a setup
+// call ends with this wait.  Copies of a call that is made again and again go
+// on the context's stream instead.
+inline cudaError_t setup_copies_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // ---- helpers (ctx.cu) ----
 int set_err(Ctx *c, int code, const std::string &msg);
 int cuda_check(Ctx *c, cudaError_t e, const char *what);

@@ -1362,6 +1362,7 @@ int iskra_lws_create(iskra_ctx *h, int capacity, uint64_t seed) {
   }
   c->lws = L;
   rc = cuda_check(c, cudaMemcpy(L->w32, w0.data(), kParams * sizeof(float), cudaMemcpyHostToDevice), "weights");
+  if (!rc) rc = cuda_check(c, setup_copies_done(), "weights");
   if (rc) return rc;
   rc = lws_sync_weights(c, L);
   if (rc) return rc;
@@ -1410,7 +1411,7 @@ int iskra_lws_weights(iskra_ctx *h, float *w_out, const float *w_in) {
   Ctx *c = &h->c;
   ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
   if (w_in) {
-    ISKRA_CUDA(c, cudaMemcpy(L->w32, w_in, kParams * sizeof(float), cudaMemcpyHostToDevice));
+    ISKRA_CUDA(c, cudaMemcpyAsync(L->w32, w_in, kParams * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     int rc = lws_sync_weights(c, L);
     if (rc) return rc;
     ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1425,7 +1426,7 @@ int iskra_lws_forward(iskra_ctx *h, const float *in, float *out) {
   Ctx *c = &h->c;
   const size_t P = (size_t)L->H * L->W;
   ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
-  ISKRA_CUDA(c, cudaMemcpy(L->x, in, P * sizeof(float), cudaMemcpyHostToDevice));
+  ISKRA_CUDA(c, cudaMemcpyAsync(L->x, in, P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   int rc = lws_forward(c, L);
   if (rc) return rc;
   ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1439,10 +1440,10 @@ int iskra_lws_loss_grad(iskra_ctx *h, const float *in, const float *target, doub
   Ctx *c = &h->c;
   const size_t P = (size_t)L->H * L->W;
   ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
-  ISKRA_CUDA(c, cudaMemcpy(L->x, in, P * sizeof(float), cudaMemcpyHostToDevice));
+  ISKRA_CUDA(c, cudaMemcpyAsync(L->x, in, P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   // the target is staged in the (P doubles) harvest buffer
-  ISKRA_CUDA(c, cudaMemcpy(L->prev, target, P * sizeof(float), cudaMemcpyHostToDevice));
-  ISKRA_CUDA(c, cudaMemset(L->loss, 0, sizeof(double)));
+  ISKRA_CUDA(c, cudaMemcpyAsync(L->prev, target, P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+  ISKRA_CUDA(c, cudaMemsetAsync(L->loss, 0, sizeof(double), c->stream));
   int rc = lws_forward(c, L);
   if (rc) return rc;
   rc = lws_backward(c, L, (const float *)L->prev, 1.f);

@@ -871,6 +871,7 @@ int iskra_mcc_create(iskra_ctx *h, int src, int nproc, const int *types, const d
   cudaMemcpy(m->gas_n, nf.data(), nf.size() * sizeof(float), cudaMemcpyHostToDevice);
   cudaMemset(m->counts, 0, kMaxProc * sizeof(unsigned long long));
   cudaMemset(m->nu, 0, (size_t)c->nn * nproc * sizeof(unsigned int));
+  setup_copies_done();
   c->mccs.push_back(m);
   *mid = (int)c->mccs.size() - 1;
   if (max_sigma_g) *max_sigma_g = best;

@@ -600,6 +600,7 @@ int mg_build(Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::v
     cudaMemcpy(m->dlv, m->lv.data(), L * sizeof(MgLevel), cudaMemcpyHostToDevice);
     m->bottom = l0;
   }
+  setup_copies_done();
   *out = m;
   return ISKRA_OK;
 }

@@ -1827,6 +1827,7 @@ static int build_device(Ctx *c, Poisson *P) {
   if (!P->xh) ISKRA_CUDA(c, cudaMalloc(&P->xh, nn * sizeof(double)));
   // a new operator: the next step solve starts from ϕ itself
   ISKRA_CUDA(c, cudaMemset(&P->scal->hist, 0, sizeof(int)));
+  ISKRA_CUDA(c, setup_copies_done());
   P->dirty = false;
   return ISKRA_OK;
 }
@@ -2650,6 +2651,7 @@ int poisson_upload_fp64(Ctx *c) {
   if (P->cr64_d) return ISKRA_OK;
   ISKRA_CUDA(c, cudaMalloc(&P->cr64_d, std::max<size_t>(1, P->cr64.size()) * sizeof(double)));
   ISKRA_CUDA(c, cudaMemcpy(P->cr64_d, P->cr64.data(), P->cr64.size() * sizeof(double), cudaMemcpyHostToDevice));
+  ISKRA_CUDA(c, setup_copies_done());
   return ISKRA_OK;
 }
 
@@ -2690,8 +2692,7 @@ int iskra_poisson_apply_dirichlet(iskra_ctx *h, const uint8_t *nodes, double phi
     P->dirty = true;
     return ISKRA_OK;
   }
-  ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
-  ISKRA_CUDA(c, cudaMemcpy(P->bfix_d, P->bfix.data(), P->nn * sizeof(double), cudaMemcpyHostToDevice));
+  ISKRA_CUDA(c, cudaMemcpyAsync(P->bfix_d, P->bfix.data(), P->nn * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   return fixed_to_x_now(c);
 }
 
@@ -2830,8 +2831,9 @@ int iskra_poisson_solve_host(iskra_ctx *h, const double *f, double rtol, int max
   // the device ρ holds -f: b[ρ] = f/ε0 = -ρ/ε0
   std::vector<double> negf(c->nn);
   for (int k = 0; k < c->nn; k++) negf[k] = -f[k];
-  ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
-  ISKRA_CUDA(c, cudaMemcpy(c->rho, negf.data(), c->nn * sizeof(double), cudaMemcpyHostToDevice));
+  // on the stream of the solve: a cudaMemcpy of up to 64 KB can return before
+  // the device has the data, and the solve then read the previous ρ
+  ISKRA_CUDA(c, cudaMemcpyAsync(c->rho, negf.data(), c->nn * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   c->rho64_valid = true;
   c->rho_df_valid = false;
   int rc = solve_sync(c, rtol, maxit, iters, relres);

@@ -181,6 +181,7 @@ int iskra_source_create(iskra_ctx *h, int sid, double rate, const double wx[2], 
   }
   if (cudaMalloc(&S.d, sizeof(SourceDev)) != cudaSuccess) return set_err(c, ISKRA_ENOMEM, "source scratch");
   ISKRA_CUDA(c, cudaMemset(S.d, 0, sizeof(SourceDev)));
+  ISKRA_CUDA(c, setup_copies_done());
   sources_of(c).push_back(S);
   if (src) *src = (int)sources_of(c).size() - 1;
   return ISKRA_OK;

@@ -245,6 +245,7 @@ int iskra_circuit_create(iskra_ctx *h, double R, double L, double C, double amp,
     if (wall >= 0) seen[s] = st.absorbed[wall];
   }
   ISKRA_CUDA(c, cudaMemcpy(c->cir_seen, seen.data(), kMaxSpecies * sizeof(unsigned long long), cudaMemcpyHostToDevice));
+  ISKRA_CUDA(c, setup_copies_done());
   c->has_circuit = true;
   invalidate_graphs(c);
   return ISKRA_OK;

@@ -87,6 +87,7 @@ static int tracker_upload(Ctx *c) {
   unsigned char kinds[kMaxSurfaces] = {};
   for (size_t f = 0; f < t->kind.size(); f++) kinds[f] = (unsigned char)t->kind[f];
   ISKRA_CUDA(c, cudaMemcpy(t->d_kind, kinds, kMaxSurfaces, cudaMemcpyHostToDevice));
+  ISKRA_CUDA(c, setup_copies_done());
   invalidate_graphs(c);  // captured pushes hold the tracker pointers (or none)
   return ISKRA_OK;
 }
