@@ -82,6 +82,7 @@ struct Poisson {
   double pcg_graph_rtol = 0;
   // ---- device representation ----
   bool separable = false, singular = false, cyclic = false;
+  bool sep_form = false;        // the operator separates (direct_solve decides whether it is solved so)
   int nclass = 0;
   uint16_t *cls = nullptr;      // nn
   RowClass *classes = nullptr;
@@ -101,11 +102,11 @@ struct Poisson {
   PoissonScal *scal_h = nullptr;  // pinned
   double dsum = 0;              // Σ d over free rows (singular projection)
   // separable solver
-  int N = 0, K = 0, logN = 0;   // N = ny, K = N/2+1
+  int N = 0, K = 0, log2p = 0, odd = 1;  // N = ny = 2^log2p odd, K = N/2+1
   // (FP32 correction: factors computed in FP64 on the host, stored rounded)
   float *r32 = nullptr;         // nn scaled residual, input of the correction
   float2 *spec = nullptr;       // nx*K
-  float2 *tw = nullptr;         // N/2 twiddles exp(-2πi m/N)
+  float2 *tw = nullptr;         // N/2 twiddles exp(-2πi m/N), then the odd factor's exp(-2πi m/odd)
   float *low = nullptr, *up = nullptr;        // nx
   float *inv = nullptr, *cp = nullptr, *q = nullptr;  // nx*K
   float *gk = nullptr;          // 2K: 1/(1+v.q) and β/γ per mode (x-periodic)
@@ -686,20 +687,94 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 
 __device__ __forceinline__ unsigned bitrev(unsigned v, int bits) { return __brev(v) >> (32 - bits); }
 
-// in-place radix-2 DIT FFT of TP length-N columns held in shared memory with
-// column stride S (input in bit-reversed order), twiddles tw (N/2, shared);
-// the inverse uses conjugate twiddles and leaves the 1/N to the caller
-__device__ void fft_columns(float2 *buf, int TP, int N, int S, int logN, const float2 *tw, bool inverse) {
+// Transform length N = 2^log2p odd.  A power of two (odd == 1) is radix-2
+// butterflies alone; any other ny takes its odd factor as dense DFTs first
+// (ODD instantiations of the kernels), so that operators of every ny are
+// solved directly instead of by multigrid CG (35 iterations of ~33 launches
+// on a 301 x 97 slab: 3.6 ms per step).
+struct FftPlan {
+  int N, log2p, odd;
+  const float2 *tw;   // N/2 twiddles exp(-2 pi i p / N)
+  const float2 *twm;  // odd twiddles exp(-2 pi i p / odd) (odd > 1)
+};
+
+// position of input j in the buffer: subsequence j mod 2^log2p (bit-reversed),
+// its elements contiguous
+template <bool ODD>
+__device__ __forceinline__ int fft_pos(int j, const FftPlan &F) {
+  if (!ODD) return (int)bitrev((unsigned)j, F.log2p);
+  const int r = F.log2p ? (int)bitrev((unsigned)(j & ((1 << F.log2p) - 1)), F.log2p) : 0;
+  return r * F.odd + (j >> F.log2p);
+}
+
+// Dense DFTs of length m = odd over the m-element runs of TP columns (column
+// stride S), src -> dst.  Outputs q and m - q share their products: with
+// s_t = z_t + z_(m-t), d_t = z_t - z_(m-t),
+//   Z_q, Z_(m-q) = z_0 + sum_t s_t cos(2 pi t q / m) -+ i d_t sin(2 pi t q / m)
+// (four FMAs per t for the two).  m^2/4 terms per run: at the m of real grids
+// (up to a few hundred) a few microseconds for the whole grid, bound by the
+// shared-memory reads of the twiddle at (t q) mod m.
+__device__ void dft_runs(const float2 *__restrict__ src, float2 *__restrict__ dst, int TP, const FftPlan &F, int S,
+                         const float2 *twm, bool inverse) {
+  const int m = F.odd, hm = (m - 1) >> 1, runs = 1 << F.log2p;
+  const int per = runs * (hm + 1);
+  for (int b = threadIdx.x; b < TP * per; b += blockDim.x) {
+    const int col = b / per, r = (b - col * per) / (hm + 1), q = b - col * per - r * (hm + 1);
+    const float2 *z = src + col * S + r * m;
+    float2 *o = dst + col * S + r * m;
+    float ar = z[0].x, ai = z[0].y, br = 0.f, bi = 0.f;
+    int at = 0;
+    for (int t = 1; t <= hm; t++) {
+      at += q;
+      if (at >= m) at -= m;
+      const float2 w = twm[at];  // cos, -sin
+      const float2 u = z[t], v = z[m - t];
+      ar = fmaf(u.x + v.x, w.x, ar);
+      ai = fmaf(u.y + v.y, w.x, ai);
+      br = fmaf(u.x - v.x, w.y, br);
+      bi = fmaf(u.y - v.y, w.y, bi);
+    }
+    // Z_q = a + i b for the forward transform (w.y = -sin), conjugated twiddles inverse
+    const float sg = inverse ? -1.f : 1.f;
+    o[q] = make_float2(ar - sg * bi, ai + sg * br);
+    if (q) o[m - q] = make_float2(ar + sg * bi, ai - sg * br);
+  }
+  __syncthreads();
+}
+
+// FFT of TP length-N columns held in shared memory with column stride S
+// (input at fft_pos): dense DFTs of the odd factor (buf -> alt), then radix-2
+// DIT stages in place, twiddles tw (N/2, shared); the inverse uses conjugate
+// twiddles and leaves the 1/N to the caller.  Returns the buffer that holds
+// the result.
+template <bool ODD>
+__device__ float2 *fft_columns(float2 *buf, float2 *alt, int TP, const FftPlan &F, int S, const float2 *tw,
+                               const float2 *twm, bool inverse) {
+  const int N = F.N, logN = F.log2p;
+  if (ODD) {
+    dft_runs(buf, alt, TP, F, S, twm, inverse);
+    buf = alt;
+  }
   const int hlog = logN - 1, hn = N >> 1;
-  const int total = TP * hn;
+  const int total = logN > 0 ? TP * hn : 0;
   for (int s = 1; s <= logN; s++) {
-    const int half = 1 << (s - 1);
+    const int half = ODD ? F.odd << (s - 1) : 1 << (s - 1);
     const int tws = logN - s;  // twiddle index = pos << tws
     for (int b = threadIdx.x; b < total; b += blockDim.x) {
-      const int col = b >> hlog;
-      const int kk = b & (hn - 1);
-      const int pos = kk & (half - 1);
-      const int i1 = ((kk >> (s - 1)) << s) + pos, i2 = i1 + half;
+      int col, kk, pos, i1;
+      if (ODD) {
+        col = b / hn;
+        kk = b - col * hn;
+        const int g = kk / half;
+        pos = kk - g * half;
+        i1 = 2 * g * half + pos;
+      } else {
+        col = b >> hlog;
+        kk = b & (hn - 1);
+        pos = kk & (half - 1);
+        i1 = ((kk >> (s - 1)) << s) + pos;
+      }
+      const int i2 = i1 + half;
       float2 w = tw[pos << tws];
       if (inverse) w.y = -w.y;
       float2 *c = buf + col * S;
@@ -710,45 +785,62 @@ __device__ void fft_columns(float2 *buf, int TP, int N, int S, int logN, const f
     }
     __syncthreads();
   }
+  return buf;
+}
+
+// shared memory of a transform block: TP columns of stride N + 1, N/2
+// twiddles and, with an odd factor, as many columns again and its twiddles
+struct FftShared {
+  float2 *buf, *tw, *alt, *twm;
+};
+template <bool ODD>
+__device__ __forceinline__ FftShared fft_shared(float2 *base, int TP, const FftPlan &F) {
+  FftShared q;
+  const int cols = TP * (F.N + 1);
+  q.buf = base;
+  q.tw = base + cols;
+  q.alt = ODD ? q.tw + (F.N >> 1) : nullptr;
+  q.twm = ODD ? q.alt + cols : nullptr;
+  for (int t = threadIdx.x; t < (F.N >> 1); t += blockDim.x) q.tw[t] = __ldg(F.tw + t);
+  if (ODD)
+    for (int t = threadIdx.x; t < F.odd; t += blockDim.x) q.twm[t] = __ldg(F.twm + t);
+  return q;
 }
 
 // r (nx, ny) -> spec[i K + k], k = 0..N/2: forward FFT along y of the 2 TP
 // columns of work item `item` (columns 2 TP item ...), two per complex
-// transform.  fbuf: TP columns of stride N + 1, then N/2 twiddles.  Ends with
-// a block barrier (the next item may reuse fbuf).
-__device__ __forceinline__ void fft_fwd_item(int item, const float *__restrict__ r, int nx, int N, int logN, int TP,
-                                             const float2 *__restrict__ tw, float2 *__restrict__ spec,
-                                             float2 *fbuf) {
-  const int S = N + 1, W = 2 * TP, K = (N >> 1) + 1;
+// transform.
+template <bool ODD>
+__device__ __forceinline__ void fft_fwd_item(int item, const float *__restrict__ r, int nx, const FftPlan &F, int TP,
+                                             float2 *__restrict__ spec, float2 *base) {
+  const int N = F.N, S = N + 1, W = 2 * TP, K = (N >> 1) + 1;
   const int i0 = item * W;
-  float2 *tws = fbuf + TP * S;
-  for (int t = threadIdx.x; t < (N >> 1); t += blockDim.x) tws[t] = __ldg(tw + t);
+  const FftShared q = fft_shared<ODD>(base, TP, F);
   for (int t = threadIdx.x; t < W * N; t += blockDim.x) {
     const int j = t / W, c = t - j * W;
     const int i = i0 + c;
     const float v = i < nx ? r[i + (size_t)nx * j] : 0.f;
-    reinterpret_cast<float *>(fbuf + (c >> 1) * S + bitrev(j, logN))[c & 1] = v;
+    reinterpret_cast<float *>(q.buf + (c >> 1) * S + fft_pos<ODD>(j, F))[c & 1] = v;
   }
   __syncthreads();
-  fft_columns(fbuf, TP, N, S, logN, tws, false);
+  const float2 *z = fft_columns<ODD>(q.buf, q.alt, TP, F, S, q.tw, q.twm, false);
   for (int t = threadIdx.x; t < TP * K; t += blockDim.x) {
     const int p = t / K, k = t - p * K;
-    const float2 zk = fbuf[p * S + k];
-    const float2 zm = fbuf[p * S + ((N - k) & (N - 1))];
+    const float2 zk = z[p * S + k];
+    const float2 zm = z[p * S + (k ? N - k : 0)];
     const int ia = i0 + 2 * p;
     if (ia < nx) spec[(size_t)ia * K + k] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
     if (ia + 1 < nx) spec[(size_t)(ia + 1) * K + k] = make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
   }
-  __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_fft_fwd(const float *__restrict__ r, int nx, int N, int logN, int TP,
-                                                 const float2 *__restrict__ tw, float2 *__restrict__ spec,
-                                                 const PoissonScal *__restrict__ sc) {
+template <bool ODD>
+__global__ void __launch_bounds__(256) k_fft_fwd(const float *__restrict__ r, int nx, FftPlan F, int TP,
+                                                 float2 *__restrict__ spec, const PoissonScal *__restrict__ sc) {
   pdl_wait();
-  extern __shared__ float2 fbuf[];  // TP columns of stride S, then N/2 twiddles
+  extern __shared__ float2 fbuf[];
   if (sc->done) return;
-  fft_fwd_item(blockIdx.x, r, nx, N, logN, TP, tw, spec, fbuf);
+  fft_fwd_item<ODD>(blockIdx.x, r, nx, F, TP, spec, fbuf);
 }
 
 // Per Fourier mode and real/imaginary part (one thread each): Thomas forward
@@ -909,15 +1001,14 @@ __global__ void __launch_bounds__(256) k_tridiag_cr(CrArgs A, const PoissonScal 
 }
 
 // spec -> δ (nx, ny) by the inverse of k_fft_fwd for work item `item`; x +=
-// δ on free rows.  Ends with a block barrier.
-template <bool DF>
-__device__ __forceinline__ void fft_inv_item(int item, const float2 *__restrict__ spec, int nx, int N, int logN,
-                                             int TP, const float2 *__restrict__ tw, const uint16_t *__restrict__ cls,
-                                             float2 *__restrict__ xd, double *__restrict__ x64, float2 *fbuf) {
-  const int S = N + 1, W = 2 * TP, K = (N >> 1) + 1;
+// δ on free rows.
+template <bool DF, bool ODD>
+__device__ __forceinline__ void fft_inv_item(int item, const float2 *__restrict__ spec, int nx, const FftPlan &F,
+                                             int TP, const uint16_t *__restrict__ cls, float2 *__restrict__ xd,
+                                             double *__restrict__ x64, float2 *base) {
+  const int N = F.N, S = N + 1, W = 2 * TP, K = (N >> 1) + 1;
   const int i0 = item * W;
-  float2 *tws = fbuf + TP * S;
-  for (int t = threadIdx.x; t < (N >> 1); t += blockDim.x) tws[t] = __ldg(tw + t);
+  const FftShared q = fft_shared<ODD>(base, TP, F);
   // the update's ϕ values and row classes, fetched before the transform
   constexpr int kPre = 8;
   float2 xp[kPre];
@@ -941,7 +1032,7 @@ __device__ __forceinline__ void fft_inv_item(int item, const float2 *__restrict_
     }
   }
   for (int t = threadIdx.x; t < TP * N; t += blockDim.x) {
-    const int p = t >> logN, k = t & (N - 1);
+    const int p = ODD ? t / N : t >> F.log2p, k = ODD ? t - p * N : t & (N - 1);
     const int ia = i0 + 2 * p;
     const bool hi = k >= K;
     const int kk = hi ? N - k : k;
@@ -952,18 +1043,18 @@ __device__ __forceinline__ void fft_inv_item(int item, const float2 *__restrict_
       a.y = -a.y;
       b.y = -b.y;
     }
-    fbuf[p * S + bitrev(k, logN)] = make_float2(a.x - b.y, a.y + b.x);
+    q.buf[p * S + fft_pos<ODD>(k, F)] = make_float2(a.x - b.y, a.y + b.x);
   }
   __syncthreads();
-  fft_columns(fbuf, TP, N, S, logN, tws, true);
-  const float invN = 1.f / (float)N;  // N is a power of two: exact
+  const float2 *zb = fft_columns<ODD>(q.buf, q.alt, TP, F, S, q.tw, q.twm, true);
+  const float invN = 1.f / (float)N;  // (exact for a power of two)
 #pragma unroll
   for (int u = 0; u < kPre; u++) {
     const int t = threadIdx.x + u * blockDim.x;
     const int j = t / W, c = t - j * W;
     const int i = i0 + c;
     if (freep[u]) {
-      const float2 z = fbuf[(c >> 1) * S + j];
+      const float2 z = zb[(c >> 1) * S + j];
       const float dz = (c & 1 ? z.y : z.x) * invN;
       if (DF) xd[i + (size_t)nx * j] = df_add_f(xp[u], dz);
       else x64[i + (size_t)nx * j] = xq[u] + (double)dz;
@@ -975,25 +1066,23 @@ __device__ __forceinline__ void fft_inv_item(int item, const float2 *__restrict_
     if (i < nx) {
       const size_t kk = i + (size_t)nx * j;
       if (!(cls[kk] & kFixedBit)) {
-        const float2 z = fbuf[(c >> 1) * S + j];
+        const float2 z = zb[(c >> 1) * S + j];
         const float dz = (c & 1 ? z.y : z.x) * invN;
         if (DF) xd[kk] = df_add_f(xd[kk], dz);
         else x64[kk] += (double)dz;
       }
     }
   }
-  __syncthreads();
 }
 
-template <bool DF>
-__global__ void __launch_bounds__(256) k_fft_inv_update(const float2 *__restrict__ spec, int nx, int N, int logN,
-                                                        int TP, const float2 *__restrict__ tw,
+template <bool DF, bool ODD>
+__global__ void __launch_bounds__(256) k_fft_inv_update(const float2 *__restrict__ spec, int nx, FftPlan F, int TP,
                                                         const uint16_t *__restrict__ cls, float2 *__restrict__ xd,
                                                         double *__restrict__ x64, const PoissonScal *__restrict__ sc) {
   pdl_wait();
-  extern __shared__ float2 fbuf[];  // TP columns of stride S, then N/2 twiddles
+  extern __shared__ float2 fbuf[];
   if (sc->done) return;
-  fft_inv_item<DF>(blockIdx.x, spec, nx, N, logN, TP, tw, cls, xd, x64, fbuf);
+  fft_inv_item<DF, ODD>(blockIdx.x, spec, nx, F, TP, cls, xd, x64, fbuf);
 }
 
 // mean-zero projection of x over nodes (singular case)
@@ -1369,11 +1458,24 @@ static RowEff effective_row(const Poisson *P, int r) {
   return e;
 }
 
-static int fft_smem_attr(Ctx *c, int N);
+static int fft_smem_attr(Ctx *c);
 
-static int build_device(Ctx *c, Poisson *P) {
+// Whether a separable operator is solved directly (FFT along y, cyclic
+// reduction along x) for tolerance rtol.  A power-of-two ny always is.  Any
+// other ny is down to a tolerance of 1e-9 (301 x 97 slab: a step took
+// 3.66 ms with multigrid CG, 0.10 ms directly); tighter ones keep CG, whose
+// recursively updated residual reaches tolerances below the rounding floor
+// of the recomputed one, and so does a context with a learned warm start,
+// which works on CG solves.
+static bool direct_solve(Ctx *c, const Poisson *P, double rtol) {
+  return P->sep_form && ((P->ny & (P->ny - 1)) == 0 || (!c->lws && rtol >= 1e-9));
+}
+
+// Effective rows and the symmetrising scale d of the free rows (breadth-first
+// propagation); *any_fixed: some row is an identity row.
+static int scaled_rows(Ctx *c, const Poisson *P, std::vector<RowEff> &rows, std::vector<double> &d, bool *any_fixed) {
   const int nx = P->nx, ny = P->ny, nn = P->nn;
-  std::vector<RowEff> rows(nn);
+  rows.resize(nn);
   for (int r = 0; r < nn; r++) {
     rows[r] = effective_row(P, r);
     if (rows[r].sig_dof == -2) return set_err(c, ISKRA_EINVAL, "a row couples to more than one σ dof");
@@ -1397,12 +1499,11 @@ static int build_device(Ctx *c, Poisson *P) {
     if (nb(r, 3) == col) a += e.cN;
     return a;
   };
-  // symmetrising scale by breadth-first propagation over free rows
-  std::vector<double> d(nn, 0.0);
+  d.assign(nn, 0.0);
   std::vector<int> queue;
   queue.reserve(nn);
-  bool any_fixed = false;
-  for (int r = 0; r < nn; r++) any_fixed |= rows[r].fixed;
+  *any_fixed = false;
+  for (int r = 0; r < nn; r++) *any_fixed |= rows[r].fixed;
   for (int r0 = 0; r0 < nn; r0++) {
     if (rows[r0].fixed || d[r0] != 0.0) continue;
     d[r0] = 1.0;
@@ -1426,6 +1527,39 @@ static int build_device(Ctx *c, Poisson *P) {
         }
       }
     }
+  }
+  return ISKRA_OK;
+}
+
+// The multigrid hierarchy of the CG path, from the scaled rows (host work).
+static int build_mg(Ctx *c, Poisson *P, const std::vector<RowEff> &rows, const std::vector<double> &d) {
+  const int nn = P->nn;
+  std::vector<double> s0(nn, 0.0), sW(nn, 0.0), sE(nn, 0.0), sS(nn, 0.0), sN(nn, 0.0);
+  std::vector<char> free_row(nn, 0);
+  int per_x = 0, per_y = 0;
+  for (int r = 0; r < nn; r++) {
+    per_x |= P->C[(size_t)r * 7 + 5] != 0.0;
+    per_y |= P->C[(size_t)r * 7 + 6] != 0.0;
+    const RowEff &e = rows[r];
+    if (e.fixed) continue;
+    free_row[r] = 1;
+    s0[r] = -d[r] * e.c0;
+    sW[r] = -d[r] * e.cW;
+    sE[r] = -d[r] * e.cE;
+    sS[r] = -d[r] * e.cS;
+    sN[r] = -d[r] * e.cN;
+  }
+  return mg_build(c, P->nx, P->ny, s0, sW, sE, sS, sN, free_row, per_x, per_y, &P->mg);
+}
+
+static int build_device(Ctx *c, Poisson *P) {
+  const int nx = P->nx, ny = P->ny, nn = P->nn;
+  std::vector<RowEff> rows;
+  std::vector<double> d;
+  bool any_fixed = false;
+  {
+    const int rc = scaled_rows(c, P, rows, d, &any_fixed);
+    if (rc) return rc;
   }
   for (int r = 0; r < nn; r++)
     if (!rows[r].fixed && (!(d[r] > 0) || !(-d[r] * rows[r].c0 > 0)))
@@ -1491,7 +1625,7 @@ static int build_device(Ctx *c, Poisson *P) {
   P->nclass = (int)classes.size();
   P->rho_fixed = rho_fixed;
   // ---- separability: per column i, every j gives the same scaled row ----
-  bool sep = P->method == 0 && ny >= 2 && (ny & (ny - 1)) == 0 && ny <= 4096;
+  bool sep = P->method == 0 && ny >= 2 && ny <= 4096;
   std::vector<double> s0(nx), sW(nx), sE(nx), ey(nx);
   std::vector<int> colfixed(nx);
   for (int i = 0; i < nx && sep; i++) {
@@ -1513,29 +1647,15 @@ static int build_device(Ctx *c, Poisson *P) {
       ey[i] = -d[i] * e0.cS;
     }
   }
-  P->separable = sep;
+  P->sep_form = sep;
+  P->separable = direct_solve(c, P, 1.0);
   // ---- multigrid preconditioner of the CG path ----
   mg_destroy(P->mg);
   P->mg = nullptr;
   if (P->pcg_graph) cudaGraphExecDestroy(P->pcg_graph);
   P->pcg_graph = nullptr;
-  if (!sep && !singular && P->method != 1) {
-    std::vector<double> s0(nn, 0.0), sW(nn, 0.0), sE(nn, 0.0), sS(nn, 0.0), sN(nn, 0.0);
-    std::vector<char> free_row(nn, 0);
-    int per_x = 0, per_y = 0;
-    for (int r = 0; r < nn; r++) {
-      per_x |= P->C[(size_t)r * 7 + 5] != 0.0;
-      per_y |= P->C[(size_t)r * 7 + 6] != 0.0;
-      const RowEff &e = rows[r];
-      if (e.fixed) continue;
-      free_row[r] = 1;
-      s0[r] = -d[r] * e.c0;
-      sW[r] = -d[r] * e.cW;
-      sE[r] = -d[r] * e.cE;
-      sS[r] = -d[r] * e.cS;
-      sN[r] = -d[r] * e.cN;
-    }
-    int rc = mg_build(c, nx, ny, s0, sW, sE, sS, sN, free_row, per_x, per_y, &P->mg);
+  if (!P->separable && !singular && P->method != 1) {
+    const int rc = build_mg(c, P, rows, d);
     if (rc) return rc;
   }
   // ---- device upload ----
@@ -1634,11 +1754,14 @@ static int build_device(Ctx *c, Poisson *P) {
   P->low = P->up = P->inv = P->cp = P->q = P->gk = nullptr;
   if (sep) {
     const int N = ny, K = N / 2 + 1;
-    int logN = 0;
-    while ((1 << logN) < N) logN++;
     P->N = N;
     P->K = K;
-    P->logN = logN;
+    P->log2p = 0;
+    P->odd = N;
+    while (P->odd % 2 == 0) {
+      P->odd /= 2;
+      P->log2p++;
+    }
     // tridiagonal couplings per column (k-independent); fixed columns decouple
     std::vector<double> lo(nx, 0.0), upv(nx, 0.0);
     double corner_lo = 0.0, corner_up = 0.0;  // T[0][nx-1], T[nx-1][0]
@@ -1770,10 +1893,14 @@ static int build_device(Ctx *c, Poisson *P) {
       for (size_t n = 0; n < v.size(); n++) o[n] = make_float2((float)v[n].x, (float)v[n].y);
       return o;
     };
-    std::vector<float2> tw(N / 2 > 0 ? N / 2 : 1);
+    std::vector<float2> tw(N / 2 + P->odd);
     for (int m = 0; m < N / 2; m++) {
       const double ang = -2.0 * M_PI * m / N;
       tw[m] = make_float2((float)std::cos(ang), (float)std::sin(ang));
+    }
+    for (int m = 0; m < P->odd; m++) {
+      const double ang = -2.0 * M_PI * m / P->odd;
+      tw[N / 2 + m] = make_float2((float)std::cos(ang), (float)std::sin(ang));
     }
     P->cr64.clear();
     for (const double2 &v : cr_fwd) P->cr64.insert(P->cr64.end(), {v.x, v.y});
@@ -1819,7 +1946,7 @@ static int build_device(Ctx *c, Poisson *P) {
     }
   }
   if (sep) {
-    int rc = fft_smem_attr(c, P->N);
+    int rc = fft_smem_attr(c);
     if (rc) return rc;
     if (!P->xd) ISKRA_CUDA(c, cudaMalloc(&P->xd, nn * sizeof(float2)));
     if (!P->bd) ISKRA_CUDA(c, cudaMalloc(&P->bd, nn * sizeof(float2)));
@@ -1882,16 +2009,19 @@ static int fixed_to_x_now(Ctx *c) {
 
 // Column pairs per FFT block: about two blocks per SM (at least one pair),
 // at most 64 KB of float2 per block.
-static int fft_tp(int N, int nx, int sms) {
+static int fft_tp(int N, int odd, int nx, int sms) {
   int tp = nx / (4 * sms);
-  const int cap = (65536 / (int)sizeof(float2) - N / 2) / (N + 1);
+  const int fixed = N / 2 + (odd > 1 ? odd : 0);
+  const int cap = (65536 / (int)sizeof(float2) - fixed) / ((odd > 1 ? 2 : 1) * (N + 1));
   if (tp > cap) tp = cap;
   if (tp > 16) tp = 16;
   if (tp < 1) tp = 1;
   return tp;
 }
 
-static size_t fft_smem(int N, int tp) { return ((size_t)tp * (N + 1) + N / 2) * sizeof(float2); }
+static size_t fft_smem(int N, int odd, int tp) {
+  return ((size_t)(odd > 1 ? 2 : 1) * tp * (N + 1) + N / 2 + (odd > 1 ? odd : 0)) * sizeof(float2);
+}
 
 // Shared memory of one cyclic-reduction mode: 2 columns of nx floats and its
 // coefficients (nf + nb float2, nb float; nf, nb < nx).
@@ -1913,11 +2043,19 @@ static size_t cr_smem(const Poisson *P, int G) {
   return (size_t)G * (2 * P->nx * sizeof(float) + (P->cr_nf + P->cr_nb) * sizeof(float2) + P->cr_nb * sizeof(float));
 }
 
-static int fft_smem_attr(Ctx *c, int N) {
-  const int smem = (int)fft_smem(N, fft_tp(N, c->ps->nx, c->num_sms));
-  ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+static int fft_smem_attr(Ctx *c) {
+  Poisson *P = c->ps;
+  const int smem = (int)fft_smem(P->N, P->odd, fft_tp(P->N, P->odd, P->nx, c->num_sms));
+  constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (P->odd > 1) {
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_fwd<true>, kAttr, smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<true, true>, kAttr, smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<false, true>, kAttr, smem));
+  } else {
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_fwd<false>, kAttr, smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<true, false>, kAttr, smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<false, false>, kAttr, smem));
+  }
   const int G = cr_modes_per_block(c->ps->nx, c->ps->K, c->num_sms);
   const int crsm = (int)cr_smem(c->ps, G);
   if (G && crsm > 48 * 1024)
@@ -1954,9 +2092,9 @@ struct SepShape {
 static SepShape sep_shape(Ctx *c) {
   Poisson *P = c->ps;
   SepShape sh;
-  sh.TP = fft_tp(P->N, P->nx, c->num_sms);
+  sh.TP = fft_tp(P->N, P->odd, P->nx, c->num_sms);
   sh.fb = (P->nx + 2 * sh.TP - 1) / (2 * sh.TP);
-  sh.smem = fft_smem(P->N, sh.TP);
+  sh.smem = fft_smem(P->N, P->odd, sh.TP);
   sh.G = cr_modes_per_block(P->nx, P->K, c->num_sms);
   return sh;
 }
@@ -2039,12 +2177,14 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
   const SweepLoop none{};
   if (P->separable) {
     const SepShape sh = sep_shape(c);
-    const int N = P->N, K = P->K;
+    const int K = P->K;
+    const FftPlan F{P->N, P->log2p, P->odd, P->tw, P->tw + P->N / 2};
+    const bool odd = P->odd > 1;
     for (int s = 0; s < count; s++) {
       const bool last = s == count - 1;
       const PoissonScal *sc = P->scal;
-      ISKRA_CUDA(c, launch_pdl(k_fft_fwd, sh.fb, 256, sh.smem, st, (const float *)P->r32, P->nx, N, P->logN, sh.TP,
-                               (const float2 *)P->tw, P->spec, sc));
+      ISKRA_CUDA(c, launch_pdl(odd ? k_fft_fwd<true> : k_fft_fwd<false>, sh.fb, 256, sh.smem, st,
+                               (const float *)P->r32, P->nx, F, sh.TP, P->spec, sc));
       if (sh.G) {
         ISKRA_CUDA(c, launch_pdl(k_tridiag_cr, (K + sh.G - 1) / sh.G, 256, cr_smem(P, sh.G), st, cr_args(P, sh.G),
                                  sc));
@@ -2054,16 +2194,16 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
                                  (const float *)P->q, (const float *)P->gk, (int)P->cyclic, P->pin_k0, sc));
       }
       if (P->df_mode) {
-        ISKRA_CUDA(c, launch_pdl(k_fft_inv_update<true>, sh.fb, 256, sh.smem, st, (const float2 *)P->spec, P->nx, N,
-                                 P->logN, sh.TP, (const float2 *)P->tw, (const uint16_t *)P->cls, P->xd,
-                                 (double *)nullptr, sc));
+        ISKRA_CUDA(c, launch_pdl(odd ? k_fft_inv_update<true, true> : k_fft_inv_update<true, false>, sh.fb, 256,
+                                 sh.smem, st, (const float2 *)P->spec, P->nx, F, sh.TP, (const uint16_t *)P->cls,
+                                 P->xd, (double *)nullptr, sc));
         ISKRA_CUDA(c, launch_pdl(k_residual_df<false, true>, B, T, 0, st, op, (const float2 *)P->xd,
                                  (const double *)nullptr, (const float2 *)nullptr, make_float2(0.f, 0.f), nie,
                                  P->bd, P->scal, P->r32, P->part, nn,
                                  (int)P->singular, rtol2, eout(c, true), last ? loop : none));
       } else {
-        ISKRA_CUDA(c, launch_pdl(k_fft_inv_update<false>, sh.fb, 256, sh.smem, st, (const float2 *)P->spec, P->nx,
-                                 N, P->logN, sh.TP, (const float2 *)P->tw, (const uint16_t *)P->cls,
+        ISKRA_CUDA(c, launch_pdl(odd ? k_fft_inv_update<false, true> : k_fft_inv_update<false, false>, sh.fb, 256,
+                                 sh.smem, st, (const float2 *)P->spec, P->nx, F, sh.TP, (const uint16_t *)P->cls,
                                  (float2 *)nullptr, P->x, sc));
         ISKRA_CUDA(c, launch_pdl(k_residual<false, true>, B, T, 0, st, op, (const double *)P->x,
                                  (const double *)c->rho, nie, P->scal, (double *)nullptr, P->r32, P->part, nn,
@@ -2104,9 +2244,11 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
 
 // Sweeps a step graph runs per solve (each skipped on the device once the
 // residual meets rtol): one FP32 correction reduces the residual by about
-// 10^-5 (cold start) and the step starts from the previous potential.
-static int graph_sweeps(double rtol) {
-  const int n = (int)std::ceil(std::log(rtol) / std::log(1e-5));
+// 10^-5 (cold start) and the step starts from the previous potential.  One
+// more with an odd factor in ny (CG, which solved those operators before,
+// had no such limit).
+static int graph_sweeps(const Poisson *P, double rtol) {
+  const int n = (int)std::ceil(std::log(rtol) / std::log(1e-5)) + (P->odd > 1 ? 1 : 0);
   return std::max(2, std::min(8, n));
 }
 
@@ -2135,7 +2277,7 @@ int poisson_solve_graph(Ctx *c, double rtol) {
   if (rc) return rc;
   Poisson *P = c->ps;
   if (!P->separable) return set_err(c, ISKRA_EINVAL, "graph solve needs a separable operator");
-  const int n = graph_sweeps(rtol);
+  const int n = graph_sweeps(P, rtol);
   const SweepLoop none{}, last{c->d_err};
   rc = queue_prologue(c, rtol, c->graph_dt, none, true);
   if (rc) return rc;
@@ -2268,7 +2410,7 @@ static int solve_sync(Ctx *c, double rtol, int maxit, int *iters, double *relres
         }
       }
     }
-    if (P->mg) {
+    if (P->mg && !P->separable) {
       // multigrid CG: the start (V-cycle of the first residual) queued, then
       // the iteration's kernels replayed as one graph
       if (first) {
@@ -2367,10 +2509,34 @@ int poisson_sync_x(Ctx *c) {
 // mix 1/Δx and 1/Δx^2 scales) keep the FP64 state.
 static bool want_df(const Poisson *P, double rtol) { return P->separable && P->nsig == 0 && rtol >= 1e-9; }
 
+// Puts the solver that direct_solve picks in effect (outside stream capture);
+// the multigrid hierarchy is built when CG first needs it.
+static int choose_solver(Ctx *c, double rtol) {
+  Poisson *P = c->ps;
+  const bool direct = direct_solve(c, P, rtol);
+  if (P->dirty || direct == P->separable) return ISKRA_OK;
+  int rc = poisson_sync_x(c);
+  if (rc) return rc;
+  if (!direct && !P->mg && !P->singular) {
+    std::vector<RowEff> rows;
+    std::vector<double> d;
+    bool any_fixed = false;
+    rc = scaled_rows(c, P, rows, d, &any_fixed);
+    if (!rc) rc = build_mg(c, P, rows, d);
+    if (rc) return rc;
+  }
+  ISKRA_CUDA(c, cudaMemsetAsync(&P->scal->hist, 0, sizeof(int), c->stream));
+  P->separable = direct;
+  invalidate_graphs(c);
+  return ISKRA_OK;
+}
+
 // Switches the authoritative state (outside stream capture; stream-ordered).
 int poisson_set_precision(Ctx *c, double rtol) {
   Poisson *P = c->ps;
   if (!P) return ISKRA_OK;
+  const int rc = choose_solver(c, rtol);
+  if (rc) return rc;
   const bool df = want_df(P, rtol);
   if (df == P->df_mode) return ISKRA_OK;
   if (df) {
@@ -2595,8 +2761,9 @@ int launch_field_runs(Ctx *c, int R, FieldRunsHost &H, cudaStream_t st) {
   int rc = poisson_prepare(c);
   if (rc) return rc;
   Poisson *P = c->ps;
-  if (!P->separable || P->cyclic || P->singular || P->N > 16 || P->nsig > 0 || P->rho_fixed)
-    return set_err(c, ISKRA_EINVAL, "ensemble field solve needs a separable, non-periodic-x operator with ny <= 16");
+  if (!P->separable || P->odd > 1 || P->cyclic || P->singular || P->N > 16 || P->nsig > 0 || P->rho_fixed)
+    return set_err(c, ISKRA_EINVAL, "ensemble field solve needs a separable, non-periodic-x operator with ny <= 16, "
+                                    "a power of two");
   const int nx = P->nx, K = P->K, nn = P->nn;
   if (!P->cr64_d) return set_err(c, ISKRA_EINVAL, "FP64 factors not uploaded (poisson_upload_fp64)");
   FieldRuns F{};
@@ -2647,7 +2814,8 @@ int poisson_upload_fp64(Ctx *c) {
   int rc = poisson_prepare(c);
   if (rc) return rc;
   Poisson *P = c->ps;
-  if (!P->separable) return set_err(c, ISKRA_EINVAL, "ensemble field solve needs a separable operator");
+  if (!P->separable || P->odd > 1)
+    return set_err(c, ISKRA_EINVAL, "ensemble field solve needs a separable operator with ny a power of two");
   if (P->cr64_d) return ISKRA_OK;
   ISKRA_CUDA(c, cudaMalloc(&P->cr64_d, std::max<size_t>(1, P->cr64.size()) * sizeof(double)));
   ISKRA_CUDA(c, cudaMemcpy(P->cr64_d, P->cr64.data(), P->cr64.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -2796,6 +2964,7 @@ int iskra_poisson_set_method(iskra_ctx *h, int method, int *active) {
     c->ps->dirty = true;
   }
   int rc = poisson_prepare(c);
+  if (!rc) rc = choose_solver(c, 1.0);
   if (rc) return rc;
   if (active) *active = c->ps->separable ? 0 : (c->ps->mg ? 2 : 1);
   return ISKRA_OK;
