@@ -334,7 +334,9 @@ struct Mg;                     // multigrid.cu (V-cycle preconditioner of CG sol
 int mg_build(struct Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::vector<double> &sW,
              const std::vector<double> &sE, const std::vector<double> &sS, const std::vector<double> &sN,
              const std::vector<char> &free_row, int per_x, int per_y, Mg **out);
-int mg_queue_cycle(struct Ctx *c, Mg *m, const double *r, double *z, const int *skip);
+struct PcgDots;
+int mg_queue_cycle(struct Ctx *c, Mg *m, const double *r, double *z, const int *skip, const PcgDots &D,
+                   bool *dots_done);
 int mg_levels(const Mg *m);
 void mg_destroy(Mg *m);
 struct CircuitDev {            // device-resident circuit state (FP64)
@@ -521,6 +523,127 @@ inline cudaError_t launch_pdl(void (*kern)(K...), dim3 grid, dim3 block, size_t 
 // call ends with this wait.  Copies of a call that is made again and again go
 // on the context's stream instead.
 inline cudaError_t setup_copies_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
+// ---- FP64 reductions of the solvers ----
+__device__ __forceinline__ double block_sum(double v, double *sh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) sh[wid] = v;
+  __syncthreads();
+  double t = 0;
+  if (threadIdx.x < 32) {
+    t = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  }
+  __syncthreads();
+  return t;  // valid in thread 0
+}
+
+// deterministic sum of partials (every block computes the same value)
+static __device__ __forceinline__ double sum_partials(const double *__restrict__ part, int n, double *sh) {
+  double v = 0;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) v += __ldcg(part + k);  // written by other blocks
+  double t = block_sum(v, sh);
+  if (threadIdx.x == 0) sh[32] = t;
+  __syncthreads();
+  double r = sh[32];
+  __syncthreads();
+  return r;
+}
+
+
+// Scalars of the multigrid-preconditioned CG iteration (poisson.cu,
+// multigrid.cu).  Each dot product is finished by the last block of the kernel
+// that forms its partials, so that the kernels that use it read one value: every
+// block of the consumer summing the partials itself cost ~10 us of FP64 issue
+// per kernel at 912 blocks.
+constexpr int kPcgPartials = 1024;
+struct PcgScal {
+  double rz, alpha, beta;
+  unsigned tick_ap, tick_up, tick_z;  // blocks finished, per kernel
+  int par;                            // which of the two direction buffers holds p
+};
+struct PcgDots {
+  const double *ap = nullptr;  // S p of the iteration
+  double *part = nullptr;      // 2 kPcgPartials: partials of z.r and z.Sp
+  PcgScal *s = nullptr;
+  int init = 0;                // the start of a solve: z.r only, beta = 0
+};
+// Block sums of K values per thread, K <= 2, by shared memory (buf: K blockDim
+// doubles): warp q adds up the threads' values of sum q, a few per lane, then
+// across its lanes; the sums come back to every thread.  A shuffle tree in every
+// warp issues five FP64 additions per warp and value on a pipe that takes 16
+// cycles each (23 warps: ~1 us a block and SM), this one about one per warp.
+template <int K>
+static __device__ __forceinline__ void block_sums(const double (&v)[K], double *buf, double (&out)[K]) {
+  __shared__ double res[K];
+  const int T = blockDim.x, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < K; q++) buf[q * T + threadIdx.x] = v[q];
+  __syncthreads();
+  if (wid < K) {
+    double a[4] = {0, 0, 0, 0};  // (short chains: an FP64 addition's latency is ~40 cycles)
+    for (int k = lane; k < T; k += 128)
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (k + 32 * u < T) a[u] += buf[wid * T + k + 32 * u];
+    double t = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) res[wid] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < K; q++) out[q] = res[q];
+  __syncthreads();
+}
+// The grid's sums of K values per thread: block sums to part[q kPcgPartials +
+// block]; in the last block to finish (ticket), true, with the totals in out
+// (added up in block order); false in the others.  The ticket is reset.
+template <int K>
+static __device__ __forceinline__ bool grid_sums(const double (&v)[K], double *buf, double *part, unsigned *ticket,
+                                                 double (&out)[K]) {
+  __shared__ int last;
+  double t[K];
+  block_sums<K>(v, buf, t);
+  if (gridDim.x == 1) {
+#pragma unroll
+    for (int q = 0; q < K; q++) out[q] = t[q];
+    return true;
+  }
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 0; q < K; q++) part[q * kPcgPartials + blockIdx.x] = t[q];
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  if (threadIdx.x == 0) *ticket = 0u;
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    t[q] = 0;
+    for (int k = threadIdx.x; k < gridDim.x; k += blockDim.x) t[q] += __ldcg(part + q * kPcgPartials + k);
+  }
+  block_sums<K>(t, buf, out);
+  return true;
+}
+// z.r and z.Sp summed up; the last block forms rz and the Polak-Ribiere
+// beta = z_new.(r_new - r_old) / rz_old = -alpha z_new.(S p) / rz_old, which
+// tolerates the FP32 rounding of the cycle.  (Every thread of the block; buf: 2
+// blockDim doubles.)
+static __device__ __forceinline__ void pcg_finish_dots(const PcgDots &D, double zr, double za, double *buf) {
+  const double v[2] = {zr, za};
+  double t[2];
+  if (grid_sums<2>(v, buf, D.part, &D.s->tick_z, t) && threadIdx.x == 0) {
+    const double rz = D.s->rz;
+    D.s->beta = !D.init && rz != 0 ? -D.s->alpha * t[1] / rz : 0.0;
+    D.s->rz = t[0];
+  }
+}
 
 // ---- helpers (ctx.cu) ----
 int set_err(Ctx *c, int code, const std::string &msg);

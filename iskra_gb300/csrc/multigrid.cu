@@ -24,6 +24,11 @@
 // dense inverse.  The cycle is symmetric (same smoother before and after,
 // restriction = P^T, exact coarsest solve), so it is a fixed SPD
 // preconditioner up to FP32 rounding.
+//
+// Launches: one per level and leg.  k_mg_down does a level's two sweeps from
+// zero, its residual and the restriction on shared-memory tiles with a halo;
+// k_mg_up the prolongation and two sweeps; the smallest levels and the
+// coarsest solve are one block (k_mg_bottom).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -32,9 +37,12 @@
 
 namespace iskra {
 
-constexpr int kMgCoarsest = 400;  // nodes of the level solved by its dense inverse
+// Nodes of the level solved by its dense inverse: a grid of up to 400 nodes as
+// it is (its inverse then makes the whole cycle exact), the coarsest of several
+// levels at most 128, so that its inverse fits the bottom block's shared memory
+// (64 KB) beside the levels above it.
+constexpr int kMgCoarsest = 128, kMgSingle = 400;
 constexpr float kMgOmega = 0.7f;
-constexpr int kMgSweeps = 2;
 
 struct MgLevel {
   int nx = 0, ny = 0, n = 0;
@@ -43,13 +51,14 @@ struct MgLevel {
   int five = 0;                // no corner couplings (5-point stencil)
   float *coef = nullptr;       // 9 x n: offset o = (dy + 1) 3 + (dx + 1), node-major
   float *dinv = nullptr;       // omega / diagonal, 0 on nodes outside the correction
-  float *x = nullptr, *x2 = nullptr, *b = nullptr, *r = nullptr;
+  float *x = nullptr, *x2 = nullptr, *b = nullptr;
 };
 
 struct Mg {
   std::vector<MgLevel> lv;
   MgLevel *dlv = nullptr;      // device copy of lv (the single-block bottom reads it)
   int bottom = 0;              // first level of the single-block bottom (0: none)
+  size_t bottom_smem = 0;      // its shared memory
   float *cinv = nullptr;       // dense inverse of the coarsest level (n x n)
 };
 
@@ -61,7 +70,6 @@ void mg_destroy(Mg *m) {
     cudaFree(l.x);
     cudaFree(l.x2);
     cudaFree(l.b);
-    cudaFree(l.r);
   }
   cudaFree(m->cinv);
   cudaFree(m->dlv);
@@ -102,217 +110,225 @@ __host__ __device__ __forceinline__ int axis_parents(int i, int n, int nc, int c
 }
 
 // ---- kernels (FP32) ----------------------------------------------------------
-// Node kernels run one thread per node on (32 x 8)-thread blocks over the
-// level's grid; every stencil load is issued unconditionally (a zero
-// coefficient multiplies a finite x) so that the loads of a node overlap.
-// FIVE: the level has no corner couplings (level 0, the 5-point operator):
-// the four corner planes are neither read nor multiplied.
-constexpr int kMgBx = 32, kMgBy = 8;
-
+// Every stencil load is issued unconditionally (a zero coefficient multiplies a
+// finite x) so that the loads of a node overlap.  FIVE: the level has no corner
+// couplings (level 0, the 5-point operator): the four corner planes are neither
+// read nor multiplied.
 __device__ __forceinline__ int wrap_idx(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
+// any position of a tile and its halo to its node (tiles may be wider than the grid)
+__device__ __forceinline__ int wrap_any(int i, int n) {
+  if ((unsigned)i < (unsigned)n) return i;
+  const int m = i % n;
+  return m < 0 ? m + n : m;
+}
 
-// (A x)_k with x(m) the iterate at node m
-template <bool FIVE, class X>
-__device__ __forceinline__ float apply9x(const float *__restrict__ coef, X x, int k, int i, int j, int nx, int ny,
-                                         int n) {
-  const int iw = wrap_idx(i - 1, nx), ie = wrap_idx(i + 1, nx);
-  const int rs = nx * wrap_idx(j - 1, ny), rc = nx * j, rn = nx * wrap_idx(j + 1, ny);
-  float a = coef[(size_t)4 * n + k] * x(k);
-  a = fmaf(coef[(size_t)1 * n + k], x(i + rs), a);
-  a = fmaf(coef[(size_t)3 * n + k], x(iw + rc), a);
-  a = fmaf(coef[(size_t)5 * n + k], x(ie + rc), a);
-  a = fmaf(coef[(size_t)7 * n + k], x(i + rn), a);
+// a node's stencil coefficients in registers
+template <bool FIVE>
+struct MgStencil {
+  float c[FIVE ? 5 : 9];
+};
+template <bool FIVE>
+__device__ __forceinline__ MgStencil<FIVE> mg_stencil(const float *__restrict__ coef, int k, int n) {
+  MgStencil<FIVE> S;
+  constexpr int o[9] = {4, 1, 3, 5, 7, 0, 2, 6, 8};
+#pragma unroll
+  for (int q = 0; q < (FIVE ? 5 : 9); q++) S.c[q] = __ldg(coef + (size_t)o[q] * n + k);
+  return S;
+}
+// (A x) at a node from shared memory: x points at the node's value, rows W apart
+template <bool FIVE>
+__device__ __forceinline__ float apply9t(const MgStencil<FIVE> &S, const float *x, int W) {
+  float a = S.c[0] * x[0];
+  a = fmaf(S.c[1], x[-W], a);
+  a = fmaf(S.c[2], x[-1], a);
+  a = fmaf(S.c[3], x[1], a);
+  a = fmaf(S.c[4], x[W], a);
   if (!FIVE) {
-    a = fmaf(coef[(size_t)0 * n + k], x(iw + rs), a);
-    a = fmaf(coef[(size_t)2 * n + k], x(ie + rs), a);
-    a = fmaf(coef[(size_t)6 * n + k], x(iw + rn), a);
-    a = fmaf(coef[(size_t)8 * n + k], x(ie + rn), a);
+    a = fmaf(S.c[FIVE ? 0 : 5], x[-W - 1], a);
+    a = fmaf(S.c[FIVE ? 0 : 6], x[-W + 1], a);
+    a = fmaf(S.c[FIVE ? 0 : 7], x[W - 1], a);
+    a = fmaf(S.c[FIVE ? 0 : 8], x[W + 1], a);
   }
   return a;
-}
-template <bool FIVE>
-__device__ __forceinline__ float apply9(const float *__restrict__ coef, const float *__restrict__ x, int k, int i,
-                                        int j, int nx, int ny, int n) {
-  return apply9x<FIVE>(coef, [&](int m) { return x[m]; }, k, i, j, nx, ny, n);
-}
-
-// One damped-Jacobi sweep at node (i, j): xo = xi + dinv (b - A xi).
-// xi == nullptr: the first sweep from x = 0 (xo = dinv b); with r64 given it
-// also forms the level-0 right-hand side b = (float) r64 (the FP64 scaled
-// residual of the CG iteration).  z64 given: the last sweep of the cycle
-// writes the result in FP64 there instead of xo.
-template <bool FIVE>
-__device__ __forceinline__ void smooth_node(const float *__restrict__ coef, const float *__restrict__ dinv,
-                                            const float *__restrict__ xi, float *__restrict__ xo,
-                                            float *__restrict__ b, int nx, int ny, int i, int j,
-                                            const double *__restrict__ r64, double *__restrict__ z64) {
-  const int n = nx * ny, k = i + nx * j;
-  const float dk = dinv[k];
-  if (!xi) {
-    float bk;
-    if (r64) {
-      bk = (float)r64[k];
-      b[k] = bk;
-    } else {
-      bk = b[k];
-    }
-    xo[k] = dk * bk;
-    return;
-  }
-  const float ax = apply9<FIVE>(coef, xi, k, i, j, nx, ny, n);
-  const float v = dk != 0.f ? xi[k] + dk * (b[k] - ax) : 0.f;
-  if (z64) z64[k] = (double)v;
-  else xo[k] = v;
-}
-
-// The first two sweeps at node (i, j): the first from x = 0 is pointwise
-// (x0 = dinv b), so the second forms x0 at the stencil's nodes itself --
-// the same products as two sweeps, without the first one's launch and its
-// pass over x.  r64 given: level 0, b = (float) r64 (also stored in b).
-template <bool FIVE>
-__device__ __forceinline__ void smooth01_node(const float *__restrict__ coef, const float *__restrict__ dinv,
-                                              float *__restrict__ xo, float *__restrict__ b, int nx, int ny, int i,
-                                              int j, const double *__restrict__ r64) {
-  const int n = nx * ny, k = i + nx * j;
-  auto bval = [&](int m) { return r64 ? (float)r64[m] : b[m]; };
-  auto x0 = [&](int m) { return __fmul_rn(dinv[m], bval(m)); };  // as the first sweep stores it
-  const float dk = dinv[k], bk = bval(k);
-  if (r64) b[k] = bk;
-  const float ax = apply9x<FIVE>(coef, x0, k, i, j, nx, ny, n);
-  xo[k] = dk != 0.f ? fmaf(dk, bk - ax, __fmul_rn(dk, bk)) : 0.f;
-}
-
-// r = b - A x at node (i, j) of the correction's nodes
-template <bool FIVE>
-__device__ __forceinline__ void residual_node(const float *__restrict__ coef, const float *__restrict__ dinv,
-                                              const float *__restrict__ x, const float *__restrict__ b,
-                                              float *__restrict__ r, int nx, int ny, int i, int j) {
-  const int n = nx * ny, k = i + nx * j;
-  const float ax = apply9<FIVE>(coef, x, k, i, j, nx, ny, n);
-  r[k] = dinv[k] != 0.f ? b[k] - ax : 0.f;
 }
 
 struct MgXfer {
   int nx, ny, ncx, ncy, cx, cy, per_x, per_y;
 };
 
-// coarse b = P^T r at coarse node (I, J) (gathered from its fine candidates)
-__device__ __forceinline__ void restrict_node(const float *__restrict__ r, float *__restrict__ bc, const MgXfer &T,
-                                              int I, int J) {
+// Weight along one axis of fine index f = 2I + d in coarse index I's restriction
+// (axis_parents transposed): 1 at d = 0, 1/2 beside it, 1 on an open far end's
+// last odd node, 0 outside the axis.
+__device__ __forceinline__ float restrict_weight(int f, int d, int n, int nc, int per) {
+  if (d == 0) return 1.f;
+  if (!per && (f < 0 || f >= n)) return 0.f;
+  return !per && d > 0 && (f + 1) >> 1 >= nc ? 1.f : 0.5f;
+}
+
+// coarse b = P^T r at coarse node (I, J), gathered from its fine candidates
+// 2I-1, 2I, 2I+1 (I itself on an axis that is not coarsened); r(fi, fj) takes
+// the candidates as formed, wrapping at a periodic end is the caller's
+template <class R>
+__device__ __forceinline__ float restrict_at(R r, const MgXfer &T, int I, int J) {
   float s = 0.f;
-  // fine candidates along each axis: 2I-1, 2I, 2I+1 (wrapped), or I itself
-  int fi[3], fj[3];
-  int ni = 0, nj = 0;
-  if (T.cx) {
-    for (int d = -1; d <= 1; d++) {
-      int f = 2 * I + d;
-      if (f < 0 || f >= T.nx) {
-        if (!T.per_x) continue;
-        f = wrap_idx(f, T.nx);
-      }
-      fi[ni++] = f;
-    }
-  } else {
-    fi[ni++] = I;
-  }
-  if (T.cy) {
-    for (int d = -1; d <= 1; d++) {
-      int f = 2 * J + d;
-      if (f < 0 || f >= T.ny) {
-        if (!T.per_y) continue;
-        f = wrap_idx(f, T.ny);
-      }
-      fj[nj++] = f;
-    }
-  } else {
-    fj[nj++] = J;
-  }
-  for (int b2 = 0; b2 < nj; b2++) {
-    int cj[2];
-    float wj[2];
-    const int pj = axis_parents(fj[b2], T.ny, T.ncy, T.cy, T.per_y, cj, wj);
-    float wy = 0.f;
-    for (int q = 0; q < pj; q++)
-      if (cj[q] == J) wy += wj[q];
+#pragma unroll
+  for (int dj = -1; dj <= 1; dj++) {
+    if (!T.cy && dj) continue;
+    const int fj = T.cy ? 2 * J + dj : J;
+    const float wy = restrict_weight(fj, dj, T.ny, T.ncy, T.per_y);
     if (wy == 0.f) continue;
-    for (int a2 = 0; a2 < ni; a2++) {
-      int ci[2];
-      float wi[2];
-      const int pi = axis_parents(fi[a2], T.nx, T.ncx, T.cx, T.per_x, ci, wi);
-      float wx = 0.f;
-      for (int q = 0; q < pi; q++)
-        if (ci[q] == I) wx += wi[q];
-      if (wx != 0.f) s = fmaf(wx * wy, r[fi[a2] + T.nx * fj[b2]], s);
+#pragma unroll
+    for (int di = -1; di <= 1; di++) {
+      if (!T.cx && di) continue;
+      const int fi = T.cx ? 2 * I + di : I;
+      const float wx = restrict_weight(fi, di, T.nx, T.ncx, T.per_x);
+      if (wx != 0.f) s = fmaf(wx * wy, r(fi, fj), s);
     }
   }
-  bc[I + T.ncx * J] = s;
+  return s;
 }
 
-// x += P xc at fine node (i, j) of the correction's nodes
-__device__ __forceinline__ void prolong_node(float *__restrict__ x, const float *__restrict__ dinv,
-                                             const float *__restrict__ xc, const MgXfer &T, int i, int j) {
-  const int k = i + T.nx * j;
-  if (dinv[k] == 0.f) return;
-  int ci[2], cj[2];
-  float wi[2], wj[2];
-  const int pi = axis_parents(i, T.nx, T.ncx, T.cx, T.per_x, ci, wi);
-  const int pj = axis_parents(j, T.ny, T.ncy, T.cy, T.per_y, cj, wj);
-  float v = 0.f;
-  for (int b2 = 0; b2 < pj; b2++)
-    for (int a2 = 0; a2 < pi; a2++) v = fmaf(wi[a2] * wj[b2], xc[ci[a2] + T.ncx * cj[b2]], v);
-  x[k] += v;
+// the parents of fine index i along one axis (axis_parents): c0, and c1 >= 0
+// when two share it equally
+__device__ __forceinline__ void prolong_parents(int i, int nc, int coarsened, int per, int &c0, int &c1) {
+  c0 = coarsened ? i >> 1 : i;
+  c1 = -1;
+  if (coarsened && (i & 1)) {
+    const int hi = (i + 1) >> 1;
+    c1 = hi < nc ? hi : per ? 0 : -1;
+  }
 }
+
+// (P xc) at fine node (i, j)
+__device__ __forceinline__ float prolong_at(const float *xc, const MgXfer &T, int i, int j) {
+  int i0, i1, j0, j1;
+  prolong_parents(i, T.ncx, T.cx, T.per_x, i0, i1);
+  prolong_parents(j, T.ncy, T.cy, T.per_y, j0, j1);
+  const float w = (i1 >= 0 ? 0.5f : 1.f) * (j1 >= 0 ? 0.5f : 1.f);
+  float v = w * xc[i0 + T.ncx * j0];
+  if (i1 >= 0) v = fmaf(w, xc[i1 + T.ncx * j0], v);
+  if (j1 >= 0) {
+    v = fmaf(w, xc[i0 + T.ncx * j1], v);
+    if (i1 >= 0) v = fmaf(w, xc[i1 + T.ncx * j1], v);
+  }
+  return v;
+}
+
+// ---- downward leg of a level: two sweeps from zero, residual, restriction ----
+// A block takes 16 x 8 coarse nodes.  On a shared-memory tile of the fine nodes
+// under them: x0 = dinv b (the first sweep from x = 0 is pointwise) with a halo
+// of 3, the second sweep x1 with a halo of 2, the residual with a halo of 1,
+// then the coarse b.  One thread per tile node keeps the node's coefficients and
+// b in registers through both stencil passes, and all its loads are issued at
+// once: a level costs one memory latency and four barriers.  (A first version
+// with 256 threads looping over the tile took 13 us on every level, the latency
+// of its nine dependent rounds of loads.)  x1 of the tile's own fine nodes goes
+// to memory for the upward leg.  At 1024 x 1024 16 us where the three kernels it
+// replaces took 30, on levels of a few thousand nodes 4-5 us against 15.  r64 given: level 0, b = (float) r64 (the FP64
+// scaled residual of the CG iteration).
+constexpr int kDownCx = 16, kDownCy = 8;
+constexpr int kDownW = 2 * kDownCx + 5, kDownH = 2 * kDownCy + 5;  // x0 region of a doubly coarsened level
+constexpr int kDownThreads = (kDownW * kDownH + 31) / 32 * 32;
 
 template <bool FIVE>
-__global__ void __launch_bounds__(kMgBx * kMgBy) k_mg_smooth(const float *__restrict__ coef,
-                                                             const float *__restrict__ dinv,
-                                                             const float *__restrict__ xi, float *__restrict__ xo,
-                                                             float *__restrict__ b, int nx, int ny, const int *skip,
-                                                             const double *__restrict__ r64, double *__restrict__ z64) {
+__global__ void __launch_bounds__(kDownThreads) k_mg_down(const float *__restrict__ coef,
+                                                            const float *__restrict__ dinv, float *__restrict__ x,
+                                                            const float *__restrict__ b, float *__restrict__ bc,
+                                                            MgXfer T, const int *skip,
+                                                            const double *__restrict__ r64) {
+  __shared__ float s0[kDownThreads], s1[kDownThreads];
+  const int nx = T.nx, ny = T.ny, n = nx * ny;
+  const int l = threadIdx.x, ly = l / kDownW, lx = l - kDownW * ly;
+  const int I0 = blockIdx.x * kDownCx, J0 = blockIdx.y * kDownCy;
+  const int fx = T.cx ? 2 * I0 : I0, fy = T.cy ? 2 * J0 : J0;  // first own fine node
+  const int ox = T.cx ? 2 * kDownCx : kDownCx, oy = T.cy ? 2 * kDownCy : kDownCy;  // own fine nodes per axis
+  const int gx = fx - T.cx - 2, gy = fy - T.cy - 2;            // node of tile position (0, 0)
+  const int W = (T.cx ? 2 * kDownCx + 1 : kDownCx) + 4, H = (T.cy ? 2 * kDownCy + 1 : kDownCy) + 4;
+  const int k = wrap_any(gx + lx, nx) + nx * wrap_any(gy + ly, ny);
+  // coefficients: written by the operator build, read before the wait
+  const MgStencil<FIVE> S = mg_stencil<FIVE>(coef, k, n);
+  const float dk = __ldg(dinv + k);
   pdl_wait();
   if (*skip) return;
-  const int i = blockIdx.x * kMgBx + threadIdx.x, j = blockIdx.y * kMgBy + threadIdx.y;
-  if (i < nx && j < ny) smooth_node<FIVE>(coef, dinv, xi, xo, b, nx, ny, i, j, r64, z64);
+  const float bk = r64 ? (float)r64[k] : b[k];
+  const float x0 = __fmul_rn(dk, bk);
+  s0[l] = x0;
+  __syncthreads();
+  if (lx >= 1 && lx < W - 1 && ly >= 1 && ly < H - 1) {
+    const float v = dk != 0.f ? fmaf(dk, bk - apply9t(S, s0 + l, kDownW), x0) : 0.f;
+    s1[l] = v;
+    const int ux = gx + lx - fx, uy = gy + ly - fy;
+    if ((unsigned)ux < (unsigned)ox && (unsigned)uy < (unsigned)oy && fx + ux < nx && fy + uy < ny) x[k] = v;
+  }
+  __syncthreads();
+  if (lx >= 2 && lx < W - 2 && ly >= 2 && ly < H - 2)
+    s0[l] = dk != 0.f ? bk - apply9t(S, s1 + l, kDownW) : 0.f;  // (x0 is used up)
+  __syncthreads();
+  const int I = I0 + lx, J = J0 + ly;
+  if (lx < kDownCx && ly < kDownCy && I < T.ncx && J < T.ncy)
+    bc[I + T.ncx * J] = restrict_at([&](int fi, int fj) { return s0[fi - gx + kDownW * (fj - gy)]; }, T, I, J);
 }
+
+// ---- upward leg of a level: prolongation and two sweeps ----
+// A block takes 32 x 16 nodes, one thread per node of the tile and its halo of
+// two: x + P xc, the first sweep with a halo of 1, the second into xo (another
+// array than x: neighbouring blocks read x); coefficients and b in registers for
+// both sweeps (four to five us on small levels against 12 in three launches).
+// Level 0 (r64, z64 given) reads b = (float) r64, writes the result
+// in FP64 and adds up z.r and z.Sp of the CG iteration (pcg_finish_dots).
+constexpr int kUpX = 32, kUpY = 16, kUpW = kUpX + 4, kUpH = kUpY + 4;
+constexpr int kUpThreads = (kUpW * kUpH + 31) / 32 * 32;
 
 template <bool FIVE>
-__global__ void __launch_bounds__(kMgBx * kMgBy) k_mg_smooth01(const float *__restrict__ coef,
-                                                               const float *__restrict__ dinv, float *__restrict__ xo,
-                                                               float *__restrict__ b, int nx, int ny, const int *skip,
-                                                               const double *__restrict__ r64) {
-  pdl_wait();
-  if (*skip) return;
-  const int i = blockIdx.x * kMgBx + threadIdx.x, j = blockIdx.y * kMgBy + threadIdx.y;
-  if (i < nx && j < ny) smooth01_node<FIVE>(coef, dinv, xo, b, nx, ny, i, j, r64);
-}
-
-template <bool FIVE>
-__global__ void __launch_bounds__(kMgBx * kMgBy) k_mg_residual(const float *__restrict__ coef,
-                                                               const float *__restrict__ dinv,
-                                                               const float *__restrict__ x,
-                                                               const float *__restrict__ b, float *__restrict__ r,
-                                                               int nx, int ny, const int *skip) {
-  pdl_wait();
-  if (*skip) return;
-  const int i = blockIdx.x * kMgBx + threadIdx.x, j = blockIdx.y * kMgBy + threadIdx.y;
-  if (i < nx && j < ny) residual_node<FIVE>(coef, dinv, x, b, r, nx, ny, i, j);
-}
-
-__global__ void __launch_bounds__(kMgBx * kMgBy) k_mg_restrict(const float *__restrict__ r, float *__restrict__ bc,
-                                                               MgXfer T, const int *skip) {
-  pdl_wait();
-  if (*skip) return;
-  const int I = blockIdx.x * kMgBx + threadIdx.x, J = blockIdx.y * kMgBy + threadIdx.y;
-  if (I < T.ncx && J < T.ncy) restrict_node(r, bc, T, I, J);
-}
-
-__global__ void __launch_bounds__(kMgBx * kMgBy) k_mg_prolong(float *__restrict__ x, const float *__restrict__ dinv,
-                                                              const float *__restrict__ xc, MgXfer T,
-                                                              const int *skip) {
-  pdl_wait();
-  if (*skip) return;
-  const int i = blockIdx.x * kMgBx + threadIdx.x, j = blockIdx.y * kMgBy + threadIdx.y;
-  if (i < T.nx && j < T.ny) prolong_node(x, dinv, xc, T, i, j);
+__global__ void __launch_bounds__(kUpThreads) k_mg_up(const float *__restrict__ coef, const float *__restrict__ dinv,
+                                                      const float *__restrict__ x, const float *__restrict__ b,
+                                                      const float *__restrict__ xc, float *__restrict__ xo, MgXfer T,
+                                                      const int *skip, const double *__restrict__ r64,
+                                                      double *__restrict__ z64, PcgDots D) {
+  __shared__ float sa[kUpThreads], sx[kUpThreads];
+  __shared__ double red[2 * kUpThreads];
+  const int nx = T.nx, ny = T.ny, n = nx * ny;
+  const int tiles_x = (nx + kUpX - 1) / kUpX, tiles = tiles_x * ((ny + kUpY - 1) / kUpY);
+  const int l = threadIdx.x, ly = l / kUpW, lx = l - kUpW * ly;
+  double zr = 0, za = 0;
+  bool waited = false;
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int ty = tile / tiles_x;
+    const int gx = (tile - ty * tiles_x) * kUpX - 2 + lx, gy = ty * kUpY - 2 + ly;
+    const int i = wrap_any(gx, nx), j = wrap_any(gy, ny), k = i + nx * j;
+    const bool own = lx >= 2 && lx < kUpX + 2 && ly >= 2 && ly < kUpY + 2 && gx < nx && gy < ny;
+    const MgStencil<FIVE> S = mg_stencil<FIVE>(coef, k, n);
+    const float dk = __ldg(dinv + k);
+    if (!waited) {
+      pdl_wait();
+      if (*skip) return;
+      waited = true;
+    }
+    const double rk = r64 ? r64[k] : 0.0;
+    const double apk = own && z64 && !D.init ? D.ap[k] : 0.0;
+    const float bk = r64 ? (float)rk : b[k];
+    float v = x[k];
+    if (dk != 0.f) v += prolong_at(xc, T, i, j);
+    sa[l] = v;
+    __syncthreads();
+    if (lx >= 1 && lx < kUpW - 1 && ly >= 1 && ly < kUpH - 1) {
+      v = dk != 0.f ? v + dk * (bk - apply9t(S, sa + l, kUpW)) : 0.f;
+      sx[l] = v;
+    }
+    __syncthreads();
+    if (own) {
+      v = dk != 0.f ? v + dk * (bk - apply9t(S, sx + l, kUpW)) : 0.f;
+      if (z64) {
+        const double z = (double)v;
+        z64[k] = z;
+        zr = fma(z, rk, zr);
+        za = fma(z, apk, za);
+      } else {
+        xo[k] = v;
+      }
+    }
+  }
+  if (z64) pcg_finish_dots(D, zr, za, red);
 }
 
 // coarsest level: x = Ainv b (one warp per row)
@@ -335,56 +351,165 @@ __global__ void __launch_bounds__(256) k_mg_coarse(const float *__restrict__ inv
   }
 }
 
-// The smallest levels of the cycle in one block: levels l0 .. L-1 (each of at
+// The smallest levels of the cycle in one block: levels l0 .. L-1 (together at
 // most kMgBottomNodes nodes) get the same sweeps, residuals, transfers and
 // coarsest solve as the per-level kernels, separated by block barriers
-// instead of launches -- at a few hundred to a thousand nodes a launch
-// costs more than the level's work.  Leaves the correction in lv[l0].x.
-constexpr int kMgBottomNodes = 1024;
+// instead of launches -- at a few thousand nodes a launch costs more than the
+// level's work.  The levels' coefficients and vectors and the coarsest inverse
+// live in shared memory (14 words a node, staged once, before the kernel waits
+// for its predecessor): read from L2 in each of the cycle's phases they made the
+// block 18 us (1024 + 256 nodes) to 30 us (1075 + 300) of dependent loads; now 12
+// and 14.
+// Leaves the correction in lv[l0].x.
+constexpr int kMgBottomNodes = 2400;
+constexpr int kMgBottomWords = 14;  // per node: 9 coefficients, dinv, b, x, x2, r
 constexpr int kMgBottomThreads = 1024;
 
-__global__ void __launch_bounds__(kMgBottomThreads) k_mg_bottom(const MgLevel *__restrict__ lv, int l0, int L,
-                                                                const float *__restrict__ cinv, const int *skip) {
-  pdl_wait();
-  if (*skip) return;
-  const int tid = threadIdx.x, nt = blockDim.x;
+// shared-memory view of one bottom level
+struct MgSh {
+  float *coef, *dinv, *b, *x, *x2, *r;
+  int nx, ny, n;
+};
+__device__ __forceinline__ MgSh mg_sh(float *base, const MgLevel &D) {
+  MgSh q;
+  q.nx = D.nx;
+  q.ny = D.ny;
+  q.n = D.n;
+  q.coef = base;
+  q.dinv = base + 9 * D.n;
+  q.b = base + 10 * D.n;
+  q.x = base + 11 * D.n;
+  q.x2 = base + 12 * D.n;
+  q.r = base + 13 * D.n;
+  return q;
+}
+__device__ __forceinline__ float mg_apply(const MgSh &q, const float *x, int i, int j) {
+  const int iw = wrap_idx(i - 1, q.nx), ie = wrap_idx(i + 1, q.nx), k = i + q.nx * j, n = q.n;
+  const float *xs = x + q.nx * wrap_idx(j - 1, q.ny), *x0 = x + q.nx * j, *xn = x + q.nx * wrap_idx(j + 1, q.ny);
+  float a = q.coef[4 * n + k] * x0[i];
+  a = fmaf(q.coef[1 * n + k], xs[i], a);
+  a = fmaf(q.coef[3 * n + k], x0[iw], a);
+  a = fmaf(q.coef[5 * n + k], x0[ie], a);
+  a = fmaf(q.coef[7 * n + k], xn[i], a);
+  a = fmaf(q.coef[0 * n + k], xs[iw], a);
+  a = fmaf(q.coef[2 * n + k], xs[ie], a);
+  a = fmaf(q.coef[6 * n + k], xn[iw], a);
+  return fmaf(q.coef[8 * n + k], xn[ie], a);
+}
+// f(i, j, k) for every node of a level: thread (x, y) of a 32-wide block takes
+// nodes (x + 32 a, y + rows b)
+template <class F>
+__device__ __forceinline__ void mg_nodes(int nx, int ny, F f) {
+  for (int j = threadIdx.x >> 5; j < ny; j += blockDim.x >> 5)
+    for (int i = threadIdx.x & 31; i < nx; i += 32) f(i, j, i + nx * j);
+}
+
+// One cycle on the levels l0 .. L-1 held in shared memory (base), the
+// right-hand side in the first one's b; cinv: the coarsest inverse (shared or
+// global memory).  Ends with a block barrier.
+__device__ __forceinline__ void mg_bottom_cycle(float *base, const MgLevel *__restrict__ lv, int l0, int L,
+                                                const float *cinv) {
   auto xfer = [&](int l) {
     const MgLevel &F = lv[l], &C = lv[l + 1];
     return MgXfer{F.nx, F.ny, C.nx, C.ny, F.cx, F.cy, F.per_x, F.per_y};
   };
-  auto smooth = [&](const MgLevel &D, const float *src, float *dst) {
-    for (int k = tid; k < D.n; k += nt)
-      smooth_node<false>(D.coef, D.dinv, src, dst, D.b, D.nx, D.ny, k % D.nx, k / D.nx, nullptr, nullptr);
-    __syncthreads();
-  };
+  float *at = base;
   for (int l = l0; l + 1 < L; l++) {
-    const MgLevel &D = lv[l];
-    for (int s = 0; s < kMgSweeps; s++) smooth(D, s == 0 ? nullptr : ((s & 1) ? D.x2 : D.x), (s & 1) ? D.x : D.x2);
-    for (int k = tid; k < D.n; k += nt) residual_node<false>(D.coef, D.dinv, D.x, D.b, D.r, D.nx, D.ny, k % D.nx, k / D.nx);
+    const MgSh q = mg_sh(at, lv[l]);
+    at += kMgBottomWords * q.n;
+    const MgSh C = mg_sh(at, lv[l + 1]);
+    mg_nodes(q.nx, q.ny, [&](int, int, int k) { q.x2[k] = __fmul_rn(q.dinv[k], q.b[k]); });
     __syncthreads();
-    const MgLevel &C = lv[l + 1];
+    mg_nodes(q.nx, q.ny, [&](int i, int j, int k) {
+      q.x[k] = q.dinv[k] != 0.f ? fmaf(q.dinv[k], q.b[k] - mg_apply(q, q.x2, i, j), q.x2[k]) : 0.f;
+    });
+    __syncthreads();
+    mg_nodes(q.nx, q.ny, [&](int i, int j, int k) {
+      q.r[k] = q.dinv[k] != 0.f ? q.b[k] - mg_apply(q, q.x, i, j) : 0.f;
+    });
+    __syncthreads();
     const MgXfer T = xfer(l);
-    for (int k = tid; k < C.n; k += nt) restrict_node(D.r, C.b, T, k % C.nx, k / C.nx);
+    mg_nodes(C.nx, C.ny, [&](int I, int J, int k) {
+      C.b[k] = restrict_at([&](int fi, int fj) { return q.r[wrap_idx(fi, T.nx) + T.nx * wrap_idx(fj, T.ny)]; }, T, I,
+                           J);
+    });
     __syncthreads();
   }
   {
-    const MgLevel &C = lv[L - 1];
-    const int lane = tid & 31;
-    for (int row = tid >> 5; row < C.n; row += nt >> 5) {
+    // eight lanes per row
+    const MgSh C = mg_sh(at, lv[L - 1]);
+    const int sub = threadIdx.x & 7;
+    for (int row0 = 0; row0 < C.n; row0 += blockDim.x >> 3) {
+      const int row = row0 + (threadIdx.x >> 3);
       float acc = 0.f;
-      for (int c = lane; c < C.n; c += 32) acc = fmaf(cinv[(size_t)row * C.n + c], C.b[c], acc);
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-      if (lane == 0) C.x[row] = acc;
+      if (row < C.n)
+        for (int c = sub; c < C.n; c += 8) acc = fmaf(cinv[row * C.n + c], C.b[c], acc);
+      for (int o = 4; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, 8);
+      if (sub == 0 && row < C.n) C.x[row] = acc;
     }
     __syncthreads();
   }
   for (int l = L - 2; l >= l0; l--) {
-    const MgLevel &D = lv[l];
+    at -= kMgBottomWords * lv[l].n;
+    const MgSh q = mg_sh(at, lv[l]);
+    const MgSh C = mg_sh(at + kMgBottomWords * q.n, lv[l + 1]);
     const MgXfer T = xfer(l);
-    for (int k = tid; k < D.n; k += nt) prolong_node(D.x, D.dinv, lv[l + 1].x, T, k % D.nx, k / D.nx);
+    mg_nodes(q.nx, q.ny, [&](int i, int j, int k) {
+      if (q.dinv[k] != 0.f) q.x[k] += prolong_at(C.x, T, i, j);
+    });
     __syncthreads();
-    for (int s = 0; s < kMgSweeps; s++) smooth(D, (s & 1) ? D.x2 : D.x, (s & 1) ? D.x : D.x2);
+    mg_nodes(q.nx, q.ny, [&](int i, int j, int k) {
+      q.x2[k] = q.dinv[k] != 0.f ? q.x[k] + q.dinv[k] * (q.b[k] - mg_apply(q, q.x, i, j)) : 0.f;
+    });
+    __syncthreads();
+    mg_nodes(q.nx, q.ny, [&](int i, int j, int k) {
+      q.x[k] = q.dinv[k] != 0.f ? q.x2[k] + q.dinv[k] * (q.b[k] - mg_apply(q, q.x2, i, j)) : 0.f;
+    });
+    __syncthreads();
   }
+}
+
+// coefficients of the levels l0 .. L-1 and the coarsest inverse into shared
+// memory (one cp.async group, for the caller to wait for); returns the inverse's
+// place
+__device__ __forceinline__ float *mg_bottom_stage(float *base, const MgLevel *__restrict__ lv, int l0, int L,
+                                                  const float *__restrict__ cinv) {
+  // asynchronous 4-byte copies: all in flight together (the planes of odd-sized
+  // levels have no common 16-byte alignment)
+  auto copy = [](float *dst, const float *src, int n) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst + t)),
+                   "l"(src + t)
+                   : "memory");
+  };
+  float *at = base;
+  for (int l = l0; l < L; l++) {
+    const MgLevel &D = lv[l];
+    copy(at, D.coef, 9 * D.n);
+    copy(at + 9 * D.n, D.dinv, D.n);
+    at += kMgBottomWords * D.n;
+  }
+  const int nc = lv[L - 1].n;
+  copy(at, cinv, nc * nc);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  return at;
+}
+
+__global__ void __launch_bounds__(kMgBottomThreads) k_mg_bottom(const MgLevel *__restrict__ lv, int l0, int L,
+                                                                const float *__restrict__ cinv, const int *skip) {
+  extern __shared__ float mg_smem[];
+  const float *ci = mg_bottom_stage(mg_smem, lv, l0, L, cinv);  // (written by the operator build)
+  pdl_wait();
+  if (*skip) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // no copy is in flight when the block ends
+    return;
+  }
+  const MgLevel &D = lv[l0];
+  for (int k = threadIdx.x; k < D.n; k += blockDim.x) mg_smem[10 * D.n + k] = D.b[k];
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  mg_bottom_cycle(mg_smem, lv, l0, L, ci);
+  for (int k = threadIdx.x; k < D.n; k += blockDim.x) D.x[k] = mg_smem[11 * D.n + k];
 }
 
 // ---- host: hierarchy --------------------------------------------------------
@@ -539,7 +664,7 @@ int mg_build(Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::v
     if (free_row[nn_]) L0.coef[(size_t)7 * n0 + k] += sN[k];
   }
   std::vector<int> cxs, cys;
-  while (H.back().nx * H.back().ny > kMgCoarsest) {
+  while (H.back().nx * H.back().ny > (H.size() == 1 ? kMgSingle : kMgCoarsest)) {
     const HostLevel &F = H.back();
     const int cx = can_coarsen(F.nx, F.per_x), cy = can_coarsen(F.ny, F.per_y);
     if (!cx && !cy) break;
@@ -571,8 +696,7 @@ int mg_build(Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::v
               cudaMalloc(&D.dinv, D.n * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&D.x, D.n * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&D.x2, D.n * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&D.b, D.n * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&D.r, D.n * sizeof(float)) == cudaSuccess;
+              cudaMalloc(&D.b, D.n * sizeof(float)) == cudaSuccess;
     if (!ok) {
       mg_destroy(m);
       return set_err(c, ISKRA_ENOMEM, "multigrid levels");
@@ -587,18 +711,25 @@ int mg_build(Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::v
   }
   cudaMemcpy(m->cinv, inv.data(), inv.size() * sizeof(float), cudaMemcpyHostToDevice);
   // the single-block bottom: the smallest levels (from level 1 on, so that
-  // level 0's FP64 conversions stay in its own kernels), if more than the
-  // coarsest one qualifies
+  // level 0's FP64 conversions stay in its own kernels) that fit its shared
+  // memory together
   const int L = (int)m->lv.size();
-  int l0 = L;
-  while (l0 > 1 && m->lv[l0 - 1].n <= kMgBottomNodes) l0--;
-  if (l0 <= L - 2) {
-    if (cudaMalloc(&m->dlv, L * sizeof(MgLevel)) != cudaSuccess) {
-      mg_destroy(m);
-      return set_err(c, ISKRA_ENOMEM, "multigrid level table");
+  if (L > 1) {
+    int l0 = L, nodes = 0;
+    const int nc = m->lv[L - 1].n;
+    if (nc <= kMgCoarsest)
+      while (l0 > 1 && nodes + m->lv[l0 - 1].n <= kMgBottomNodes) nodes += m->lv[--l0].n;
+    if (l0 < L) {
+      if (cudaMalloc(&m->dlv, L * sizeof(MgLevel)) != cudaSuccess) {
+        mg_destroy(m);
+        return set_err(c, ISKRA_ENOMEM, "multigrid level table");
+      }
+      cudaMemcpy(m->dlv, m->lv.data(), L * sizeof(MgLevel), cudaMemcpyHostToDevice);
+      m->bottom = l0;
+      m->bottom_smem = ((size_t)nodes * kMgBottomWords + (size_t)nc * nc) * sizeof(float);
+      cudaFuncSetAttribute(k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (kMgBottomNodes * kMgBottomWords + kMgCoarsest * kMgCoarsest) * (int)sizeof(float));
     }
-    cudaMemcpy(m->dlv, m->lv.data(), L * sizeof(MgLevel), cudaMemcpyHostToDevice);
-    m->bottom = l0;
   }
   setup_copies_done();
   *out = m;
@@ -607,80 +738,44 @@ int mg_build(Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::v
 
 int mg_levels(const Mg *m) { return m ? (int)m->lv.size() : 0; }
 
-static dim3 mg_grid2(int nx, int ny) { return dim3((nx + kMgBx - 1) / kMgBx, (ny + kMgBy - 1) / kMgBy); }
-
-static int mg_smooth(Ctx *c, const MgLevel &D, const float *src, float *dst, const int *skip, const double *r64,
-                     double *z64) {
-  const dim3 g = mg_grid2(D.nx, D.ny), t(kMgBx, kMgBy);
-  if (D.five)
-    ISKRA_CUDA(c, launch_pdl(k_mg_smooth<true>, g, t, 0, c->stream, (const float *)D.coef, (const float *)D.dinv, src,
-                             dst, D.b, D.nx, D.ny, skip, r64, z64));
-  else
-    ISKRA_CUDA(c, launch_pdl(k_mg_smooth<false>, g, t, 0, c->stream, (const float *)D.coef, (const float *)D.dinv, src,
-                             dst, D.b, D.nx, D.ny, skip, r64, z64));
-  return ISKRA_OK;
-}
-
 // z = M^-1 r: one V(2,2) cycle on the scaled residual r (FP64, free rows);
-// every kernel returns at once while *skip is set (a converged solve).  The
-// first sweep of level 0 converts r to FP32, the last one writes z in FP64.
-int mg_queue_cycle(Ctx *c, Mg *m, const double *r, double *z, const int *skip) {
+// every kernel returns at once while *skip is set (a converged solve).  Level
+// 0 reads r in FP64 and writes z in FP64 with the dot products of D; a
+// hierarchy of one level leaves those to the caller (*dots_done = false).
+int mg_queue_cycle(Ctx *c, Mg *m, const double *r, double *z, const int *skip, const PcgDots &D, bool *dots_done) {
   cudaStream_t st = c->stream;
   const int L = (int)m->lv.size();
-  const dim3 t(kMgBx, kMgBy);
+  *dots_done = L > 1;
   auto xfer = [&](int l) {
     const MgLevel &F = m->lv[l], &C = m->lv[l + 1];
     return MgXfer{F.nx, F.ny, C.nx, C.ny, F.cx, F.cy, F.per_x, F.per_y};
   };
-  // down: smooth from zero (sweeps alternate x2 <- x <- ..., ending in x),
-  // residual, restrict
-  static_assert(kMgSweeps % 2 == 0, "an even sweep count leaves the iterate in x");
   const int lb = m->bottom ? m->bottom : L - 1;  // first level not run by per-level kernels
   for (int l = 0; l < lb; l++) {
-    MgLevel &D = m->lv[l];
-    // the first two sweeps in one launch (into x), then the rest alternating
-    const double *r64 = l == 0 ? r : nullptr;
-    if (D.five)
-      ISKRA_CUDA(c, launch_pdl(k_mg_smooth01<true>, mg_grid2(D.nx, D.ny), t, 0, st, (const float *)D.coef,
-                               (const float *)D.dinv, D.x, D.b, D.nx, D.ny, skip, r64));
-    else
-      ISKRA_CUDA(c, launch_pdl(k_mg_smooth01<false>, mg_grid2(D.nx, D.ny), t, 0, st, (const float *)D.coef,
-                               (const float *)D.dinv, D.x, D.b, D.nx, D.ny, skip, r64));
-    for (int s = 2; s < kMgSweeps; s++) {
-      const float *src = (s & 1) ? D.x2 : D.x;
-      float *dst = (s & 1) ? D.x : D.x2;
-      const int rc = mg_smooth(c, D, src, dst, skip, nullptr, nullptr);
-      if (rc) return rc;
-    }
-    if (D.five)
-      ISKRA_CUDA(c, launch_pdl(k_mg_residual<true>, mg_grid2(D.nx, D.ny), t, 0, st, (const float *)D.coef,
-                               (const float *)D.dinv, (const float *)D.x, (const float *)D.b, D.r, D.nx, D.ny, skip));
-    else
-      ISKRA_CUDA(c, launch_pdl(k_mg_residual<false>, mg_grid2(D.nx, D.ny), t, 0, st, (const float *)D.coef,
-                               (const float *)D.dinv, (const float *)D.x, (const float *)D.b, D.r, D.nx, D.ny, skip));
-    const MgLevel &C = m->lv[l + 1];
-    ISKRA_CUDA(c, launch_pdl(k_mg_restrict, mg_grid2(C.nx, C.ny), t, 0, st, (const float *)D.r, C.b, xfer(l), skip));
+    MgLevel &F = m->lv[l], &C = m->lv[l + 1];
+    const dim3 g((C.nx + kDownCx - 1) / kDownCx, (C.ny + kDownCy - 1) / kDownCy);
+    ISKRA_CUDA(c, launch_pdl(F.five ? k_mg_down<true> : k_mg_down<false>, g, kDownThreads, 0, st,
+                             (const float *)F.coef, (const float *)F.dinv, F.x, (const float *)F.b, C.b, xfer(l), skip,
+                             l == 0 ? r : nullptr));
   }
   if (m->bottom) {
-    ISKRA_CUDA(c, launch_pdl(k_mg_bottom, 1, kMgBottomThreads, 0, st, (const MgLevel *)m->dlv, m->bottom, L,
-                             (const float *)m->cinv, skip));
+    ISKRA_CUDA(c, launch_pdl(k_mg_bottom, 1, kMgBottomThreads, m->bottom_smem, st, (const MgLevel *)m->dlv, m->bottom,
+                             L, (const float *)m->cinv, skip));
   } else {
     MgLevel &C = m->lv[L - 1];
     ISKRA_CUDA(c, launch_pdl(k_mg_coarse, std::max(1, std::min(c->num_sms * 2, (C.n + 7) / 8)), 256, 0, st,
                              (const float *)m->cinv, (const float *)C.b, C.x, C.n, skip, L == 1 ? r : nullptr,
                              L == 1 ? z : nullptr));
   }
-  // up: prolong, smooth
   for (int l = lb - 1; l >= 0; l--) {
-    MgLevel &D = m->lv[l];
-    ISKRA_CUDA(c, launch_pdl(k_mg_prolong, mg_grid2(D.nx, D.ny), t, 0, st, D.x, (const float *)D.dinv,
-                             (const float *)m->lv[l + 1].x, xfer(l), skip));
-    for (int s = 0; s < kMgSweeps; s++) {
-      const float *src = (s & 1) ? D.x2 : D.x;
-      float *dst = (s & 1) ? D.x : D.x2;
-      const int rc = mg_smooth(c, D, src, dst, skip, nullptr, (l == 0 && s == kMgSweeps - 1) ? z : nullptr);
-      if (rc) return rc;
-    }
+    MgLevel &F = m->lv[l];
+    // the coarser level's correction: in x2 from its own k_mg_up, in x from the bottom
+    const float *xc = l + 1 < lb ? m->lv[l + 1].x2 : m->lv[l + 1].x;
+    const int tiles = ((F.nx + kUpX - 1) / kUpX) * ((F.ny + kUpY - 1) / kUpY);
+    const int g = l == 0 ? std::min(tiles, std::min(kPcgPartials, c->num_sms * 2)) : tiles;  // 736 threads: 2 per SM
+    ISKRA_CUDA(c, launch_pdl(F.five ? k_mg_up<true> : k_mg_up<false>, g, kUpThreads, 0, st, (const float *)F.coef,
+                             (const float *)F.dinv, (const float *)F.x, (const float *)F.b, xc, F.x2, xfer(l), skip,
+                             l == 0 ? r : nullptr, l == 0 ? z : nullptr, D));
   }
   ISKRA_CUDA(c, cudaGetLastError());
   return ISKRA_OK;

@@ -43,6 +43,7 @@ struct RowClass {
   int rho;                    // b = -ρ/ε0 (ρ dof) else b = bfix
   float nd32;                 // -d in FP32 (scaling of the FP32 residual)
   float2 c0f, cWf, cEf, cSf, cNf;  // the coefficients as double-float pairs
+  double s0, sW, sE, sS, sN;  // the scaled row -d c (the symmetric operator of CG), 0 on identity rows
 };
 
 struct DriveGroup {
@@ -97,6 +98,8 @@ struct Poisson {
   bool df_mode = false;         // the solver's state is xd (double-float), x a view
   bool x_stale = false;         // (df_mode) x lags xd
   double *r = nullptr, *z = nullptr, *p = nullptr, *ap = nullptr;  // nn
+  double *p2 = nullptr;         // second direction buffer of the multigrid CG
+  PcgScal *pcg = nullptr;       // its scalars
   double *part = nullptr;       // reduction partials (kPartials * 4)
   PoissonScal *scal = nullptr;
   PoissonScal *scal_h = nullptr;  // pinned
@@ -158,6 +161,8 @@ void poisson_destroy(Poisson *p) {
   cudaFree(p->z);
   cudaFree(p->p);
   cudaFree(p->ap);
+  cudaFree(p->p2);
+  cudaFree(p->pcg);
   cudaFree(p->part);
   cudaFree(p->scal);
   if (p->scal_h) cudaFreeHost(p->scal_h);
@@ -289,34 +294,6 @@ __global__ void k_extrapolate(const uint16_t *__restrict__ cls, void *__restrict
     sc->hticket = 0u;
     sc->hist = 1;
   }
-}
-
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-  }
-  __syncthreads();
-  return t;  // valid in thread 0
-}
-
-// deterministic sum of partials (every block computes the same value)
-__device__ double sum_partials(const double *__restrict__ part, int n, double *sh) {
-  double v = 0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) v += __ldcg(part + k);  // written by other blocks
-  double t = block_sum(v, sh);
-  if (threadIdx.x == 0) sh[32] = t;
-  __syncthreads();
-  double r = sh[32];
-  __syncthreads();
-  return r;
 }
 
 // Σ d_k b_k over free rows (singular case only: no fixed rows exist)
@@ -1206,83 +1183,133 @@ __global__ void k_cg_rz0(const double *__restrict__ part, int nparts, PoissonSca
 }
 
 // ---- flexible PCG with the multigrid preconditioner (multigrid.cu) ----
-// z = M^-1 r comes from a V-cycle between k_pcg_update and k_pcg_dots; the
-// direction update is Polak-Ribiere, beta = z_new.(r_new - r_old) / rz_old
-// = -alpha z_new.(S p) / rz_old, which tolerates the FP32 rounding of the
-// cycle.  Iteration: k_cg_ap, k_pcg_update, cycle, k_pcg_dots, k_pcg_dir.
-__global__ void k_pcg_init(OpView op, const double *__restrict__ r, const double *__restrict__ z,
-                           double *__restrict__ p, double *__restrict__ part, int nn) {
-  __shared__ double sh[40];
+// Iteration: k_pcg_ap (direction, S p, alpha), k_pcg_update (x, r, the
+// convergence test), the cycle z = M^-1 r, whose last kernel also forms z.r and
+// z.Sp and beta (pcg_finish_dots).  A converged iteration runs no cycle.
+
+// p = z + beta p, ap = S p, alpha = rz / p.Sp.  A block forms p on a 32 x 16 tile
+// and a halo of one node in shared memory, one thread per node (1.2x the
+// additions), so that the direction update costs no pass of its own; p
+// alternates between two buffers (s->par), since neighbouring blocks read the
+// old one.  Bound by GB300's FP64 rate (~7 FP64 instructions per node, 12 us at
+// 1024 x 1024) and its memory traffic: 26 us there with cold caches, where the
+// direction and S p kernels it replaces took 43 us.
+constexpr int kApX = 32, kApY = 16, kApW = kApX + 2, kApH = kApY + 2;
+constexpr int kApThreads = (kApW * kApH + 31) / 32 * 32;
+__device__ __forceinline__ int tile_node(int i, int n) {
+  if ((unsigned)i < (unsigned)n) return i;
+  const int m = i % n;
+  return m < 0 ? m + n : m;
+}
+__global__ void __launch_bounds__(kApThreads) k_pcg_ap(OpView op, const double *__restrict__ z,
+                                                       double *__restrict__ pa, double *__restrict__ pb,
+                                                       double *__restrict__ ap, double *__restrict__ part,
+                                                       const int *skip, PcgScal *s) {
+  __shared__ double sp[kApThreads];
+  __shared__ double red[kApThreads];
+  const int nx = op.nx, ny = op.ny;
+  const int l = threadIdx.x, ly = l / kApW, lx = l - kApW * ly;
+  const int tiles_x = (nx + kApX - 1) / kApX, tiles = tiles_x * ((ny + kApY - 1) / kApY);
+  pdl_wait();
+  if (*skip) return;
+  const double beta = s->beta;
+  const int par = s->par;
+  const double *po = par ? pb : pa;
+  double *pn = par ? pa : pb;
   double v = 0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    const double zz = (op.cls[k] & kFixedBit) ? 0.0 : z[k];
-    p[k] = zz;
-    v += r[k] * zz;
-  }
-  double t = block_sum(v, sh);
-  if (threadIdx.x == 0) part[2 * kPartials + blockIdx.x] = t;
-}
-
-// α = rz/pAp; x += αp; r -= αAp; partial ||res||²; α kept for the direction
-__global__ void k_pcg_update(OpView op, double *__restrict__ x, double *__restrict__ r, const double *__restrict__ p,
-                             const double *__restrict__ ap, double *__restrict__ part, int nparts, int nn,
-                             PoissonScal *__restrict__ sc) {
-  __shared__ double sh[40];
-  if (sc->done) return;
-  const double rz = sc->rz;
-  const double pap = sum_partials(part + kPartials, nparts, sh);
-  const double alpha = pap != 0 ? rz / pap : 0.0;
-  double w2 = 0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int ty = tile / tiles_x;
+    const int gx = (tile - ty * tiles_x) * kApX - 1 + lx, gy = ty * kApY - 1 + ly;
+    const int k = tile_node(gx, nx) + nx * tile_node(gy, ny);
+    const bool own = lx >= 1 && lx <= kApX && ly >= 1 && ly <= kApY && gx < nx && gy < ny;
     const RowClass &C = op.classes[op.cls[k] & kClassMask];
-    if (C.fixed) continue;
-    x[k] += alpha * p[k];
-    const double rr = r[k] - alpha * ap[k];
-    r[k] = rr;
-    const double res = rr * C.inv_d;
-    w2 += res * res;
+    double p = z[k];
+    if (beta != 0) p = fma(beta, po[k], p);
+    sp[l] = p;
+    __syncthreads();
+    if (own) {
+      double a = C.s0 * p;  // (zeros on identity rows)
+      a = fma(C.sW, sp[l - 1], a);
+      a = fma(C.sE, sp[l + 1], a);
+      a = fma(C.sS, sp[l - kApW], a);
+      a = fma(C.sN, sp[l + kApW], a);
+      pn[k] = p;
+      ap[k] = a;
+      v = fma(p, a, v);
+    }
+    __syncthreads();
   }
-  double t2 = block_sum(w2, sh);
-  if (threadIdx.x == 0) part[3 * kPartials + blockIdx.x] = t2;
-  if (blockIdx.x == 0 && threadIdx.x == 0) sc->pap = alpha;
+  const double part_v[1] = {v};
+  double pap[1];
+  if (grid_sums<1>(part_v, red, part, &s->tick_ap, pap) && threadIdx.x == 0)
+    s->alpha = pap[0] != 0 ? s->rz / pap[0] : 0.0;
 }
 
-// partials of z.r (part[2K..]) and z.Sp (part[K..], after k_pcg_update read pAp)
-__global__ void k_pcg_dots(const double *__restrict__ r, const double *__restrict__ z, const double *__restrict__ ap,
-                           double *__restrict__ part, int nn, const PoissonScal *__restrict__ sc) {
-  __shared__ double sh[40];
+// x += alpha p; r -= alpha S p; the convergence test on the unscaled residual.
+// A thread takes four nodes with all their loads in flight together.
+__global__ void __launch_bounds__(256) k_pcg_update(OpView op, double *__restrict__ x, double *__restrict__ r,
+                                                    const double *__restrict__ pa, const double *__restrict__ pb,
+                                                    const double *__restrict__ ap, double *__restrict__ part, int nn,
+                                                    PoissonScal *sc, PcgScal *s, double rtol2) {
+  pdl_wait();
   if (sc->done) return;
-  double a = 0, b = 0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    a += z[k] * r[k];
-    b += z[k] * ap[k];
+  __shared__ double red[256];
+  const double alpha = s->alpha;
+  const double *p = s->par ? pa : pb;  // the buffer k_pcg_ap wrote
+  double w2 = 0;
+  constexpr int U = 4;
+  const int stride = gridDim.x * blockDim.x;
+  for (int k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < nn; k0 += U * stride) {
+    double xk[U], rk[U], pk[U], ak[U], dk[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int k = k0 + u * stride;
+      dk[u] = 0.0;
+      if (k < nn) {
+        const unsigned ck = op.cls[k];
+        xk[u] = x[k];
+        rk[u] = r[k];
+        pk[u] = p[k];
+        ak[u] = ap[k];
+        if (!(ck & kFixedBit)) dk[u] = op.classes[ck & kClassMask].inv_d;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int k = k0 + u * stride;
+      if (dk[u] != 0.0) {  // a free row
+        x[k] = fma(alpha, pk[u], xk[u]);
+        const double rr = fma(-alpha, ak[u], rk[u]);
+        r[k] = rr;
+        const double res = rr * dk[u];
+        w2 = fma(res, res, w2);
+      }
+    }
   }
-  const double ta = block_sum(a, sh), tb = block_sum(b, sh);
-  if (threadIdx.x == 0) {
-    part[2 * kPartials + blockIdx.x] = ta;
-    part[kPartials + blockIdx.x] = tb;
-  }
-}
-
-// β (Polak-Ribiere), p = z + βp on free rows, convergence on the unscaled residual
-__global__ void k_pcg_dir(OpView op, const double *__restrict__ z, double *__restrict__ p, double *__restrict__ part,
-                          int nparts, int nn, PoissonScal *sc, double rtol2) {
-  __shared__ double sh[40];
-  if (sc->done) return;
-  const double rz = sc->rz, alpha = sc->pap;
-  const double rzn = sum_partials(part + 2 * kPartials, nparts, sh);
-  const double zap = sum_partials(part + kPartials, nparts, sh);
-  const double res2 = sum_partials(part + 3 * kPartials, nparts, sh);
-  const double beta = rz != 0 ? -alpha * zap / rz : 0.0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x)
-    p[k] = (op.cls[k] & kFixedBit) ? 0.0 : z[k] + beta * p[k];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    sc->rz_new = rzn;
+  const double part_w[1] = {w2};
+  double res[1];
+  if (grid_sums<1>(part_w, red, part, &s->tick_up, res) && threadIdx.x == 0) {
+    const double res2 = res[0];
+    s->par ^= 1;
     sc->res2 = res2;
     sc->relres = sc->rhs2 > 0 ? sqrt(res2 / sc->rhs2) : sqrt(res2);
     sc->iters += 1;
     if ((sc->rhs2 > 0 && res2 <= rtol2 * sc->rhs2) || res2 == 0.0) sc->done = 1;
   }
+}
+
+// z.r and z.Sp of a hierarchy of one level (its coarsest solve forms no sums)
+__global__ void __launch_bounds__(256) k_pcg_dots(const double *__restrict__ r, const double *__restrict__ z, int nn,
+                                                  const int *skip, PcgDots D) {
+  pdl_wait();
+  if (*skip) return;
+  __shared__ double red[512];
+  double a = 0, b = 0;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
+    a = fma(z[k], r[k], a);
+    if (!D.init) b = fma(z[k], D.ap[k], b);
+  }
+  pcg_finish_dots(D, a, b, red);
 }
 
 // ===========================================================================
@@ -1611,6 +1638,13 @@ static int build_device(Ctx *c, Poisson *P) {
       rc.cEf = split(e.cE);
       rc.cSf = split(e.cS);
       rc.cNf = split(e.cN);
+      if (!e.fixed) {
+        rc.s0 = -rc.d * e.c0;
+        rc.sW = -rc.d * e.cW;
+        rc.sE = -rc.d * e.cE;
+        rc.sS = -rc.d * e.cS;
+        rc.sN = -rc.d * e.cN;
+      }
       rc.sig_coef = e.sig_coef;
       rc.sig_dof = e.sig_dof;
       rc.fixed = e.fixed;
@@ -1697,6 +1731,9 @@ static int build_device(Ctx *c, Poisson *P) {
     ISKRA_CUDA(c, cudaMalloc(&P->z, nn * sizeof(double)));
     ISKRA_CUDA(c, cudaMalloc(&P->p, nn * sizeof(double)));
     ISKRA_CUDA(c, cudaMalloc(&P->ap, nn * sizeof(double)));
+    ISKRA_CUDA(c, cudaMalloc(&P->p2, nn * sizeof(double)));
+    ISKRA_CUDA(c, cudaMalloc(&P->pcg, sizeof(PcgScal)));
+    ISKRA_CUDA(c, cudaMemset(P->pcg, 0, sizeof(PcgScal)));
     ISKRA_CUDA(c, cudaMalloc(&P->part, 4 * kPartials * sizeof(double)));
     ISKRA_CUDA(c, cudaMalloc(&P->scal, sizeof(PoissonScal)));
     ISKRA_CUDA(c, cudaMallocHost(&P->scal_h, sizeof(PoissonScal)));
@@ -2213,19 +2250,31 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
   } else if (P->mg) {  // flexible PCG, one multigrid V-cycle per iteration
     const int *skip = &P->scal->done;
     const int G = P->cg_blocks;
+    const int tiles = ((P->nx + kApX - 1) / kApX) * ((P->ny + kApY - 1) / kApY);
+    PcgDots D;
+    D.ap = P->ap;
+    D.part = P->part;
+    D.s = P->pcg;
+    auto cycle = [&](int init) {
+      D.init = init;
+      bool dots = false;
+      const int rc = mg_queue_cycle(c, P->mg, P->r, P->z, skip, D, &dots);
+      if (rc || dots) return rc;
+      ISKRA_CUDA(c, launch_pdl(k_pcg_dots, std::min(G, kPcgPartials), T, 0, st, (const double *)P->r,
+                               (const double *)P->z, nn, skip, D));
+      return (int)ISKRA_OK;
+    };
     if (reset_cg) {  // rhs2 is already in scal
-      int rc = mg_queue_cycle(c, P->mg, P->r, P->z, skip);
+      const int rc = cycle(1);
       if (rc) return rc;
-      k_pcg_init<<<G, T, 0, st>>>(op, P->r, P->z, P->p, P->part, nn);
-      k_cg_rz0<<<1, T, 0, st>>>(P->part, G, P->scal);
     }
     for (int s = 0; s < count; s++) {
-      k_cg_ap<<<G, T, 0, st>>>(op, P->p, P->ap, P->part, nn, P->scal);
-      k_pcg_update<<<G, T, 0, st>>>(op, P->x, P->r, P->p, P->ap, P->part, G, nn, P->scal);
-      int rc = mg_queue_cycle(c, P->mg, P->r, P->z, skip);
+      ISKRA_CUDA(c, launch_pdl(k_pcg_ap, std::min(tiles, std::min(kPcgPartials, c->num_sms * 3)), kApThreads, 0, st, op, (const double *)P->z, P->p, P->p2,
+                               P->ap, P->part, skip, P->pcg));
+      ISKRA_CUDA(c, launch_pdl(k_pcg_update, G, T, 0, st, op, P->x, P->r, (const double *)P->p, (const double *)P->p2,
+                               (const double *)P->ap, P->part, nn, P->scal, P->pcg, rtol2));
+      const int rc = cycle(0);
       if (rc) return rc;
-      k_pcg_dots<<<G, T, 0, st>>>(P->r, P->z, P->ap, P->part, nn, P->scal);
-      k_pcg_dir<<<G, T, 0, st>>>(op, P->z, P->p, P->part, G, nn, P->scal, rtol2);
     }
   } else {
     if (reset_cg) {  // rhs2 is already in scal
@@ -2374,7 +2423,10 @@ static int solve_sync(Ctx *c, double rtol, int maxit, int *iters, double *relres
   int done_it = 0;
   const SweepLoop none{};
   for (;;) {
-    const int chunk = std::min(P->separable ? 2 : (P->mg ? 4 : 32), maxit - done_it);
+    // (multigrid CG: as many iterations as the last solve took before the
+    // first host check, then two at a time; converged ones return at once)
+    const int mg_chunk = first ? std::max(4, std::min(P->last_iters, 32)) : 2;
+    const int chunk = std::min(P->separable ? 2 : (P->mg ? mg_chunk : 32), maxit - done_it);
     if (first) {
       rc = queue_prologue(c, rtol, c->graph_dt, none, false);
       if (rc) return rc;
