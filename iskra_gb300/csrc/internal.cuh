@@ -346,6 +346,52 @@ struct CircuitDev {            // device-resident circuit state (FP64)
   int pad;
 };
 
+struct CircuitArgs {
+  CircuitDev *cd;
+  const double *phi;
+  const float2 *phid;          // ϕ as double-float pairs (separable solver), else nullptr
+  double *sigma;
+  int pos_ref, neg_ref;
+  int wall;                    // discard wall feeding the floating electrode, -1 none
+  int ns;
+  SpeciesState *st[kMaxSpecies];
+  double qw[kMaxSpecies];      // q * w0 per species
+};
+
+// advance!(circuit, ϕ, Δt, config) (circuit_coupling.jl:35-43) with
+// advance_circuit! (Circuit.jl:117-136); V_ext = ϕ(positive) - ϕ(negative)
+// of the PlasmaDevice (circuit_coupling.jl:18-29); wall-absorbed charge enters
+// σ as hit! does (circuit_coupling.jl:45-55).
+__device__ __forceinline__ void circuit_advance(const CircuitArgs &A, double dt, unsigned long long *seen) {
+  CircuitDev &c = *A.cd;
+  auto phi_at = [&](int k) { return A.phid ? (double)A.phid[k].x + (double)A.phid[k].y : A.phi[k]; };
+  const double vext = phi_at(A.pos_ref) - phi_at(A.neg_ref);
+  const double i = c.i, q = c.q, t = c.t;
+  const double vsrc = c.amp * sin(2.0 * M_PI * c.freq * t) + c.dc;
+  double in = (c.L / dt - c.R / 2) * i + vext - vsrc;
+  if (c.C > 0.0) {
+    in -= q / c.C;
+    in /= (c.L / dt + c.R / 2);
+    c.q = q + dt * i;
+  } else {
+    in /= (c.L / dt + c.R / 2);
+  }
+  c.i = in;
+  c.t = t + dt;
+  c.vext = vext;
+  double ds = -dt * in / c.area * c.scale;
+  if (A.wall >= 0) {
+    for (int s = 0; s < A.ns; s++) {
+      const unsigned long long now = A.st[s]->absorbed[A.wall];
+      const unsigned long long d = now - seen[s];
+      seen[s] = now;
+      ds += A.qw[s] * (double)d / c.area;
+    }
+  }
+  A.sigma[c.sigma_dof] += ds;
+}
+int circuit_args(struct Ctx *c, CircuitArgs &A);
+
 // Surface tracker (pic/surfaces/*.jl): per cell (numbered like nodes,
 // i0 + nx j0) the surface behind each of its four edges, in the order of
 // kSurfDir, and whether track! records particles of the cell.
@@ -793,7 +839,58 @@ __device__ __forceinline__ void finalize_df_node(const FinalizeDfArgs &A, const 
   }
   rho[k] = r;
 }
+// The FP64 form.
+struct FinalizeArgs {
+  int ns;
+  unsigned long long *acc[kMaxSpecies];
+  unsigned *cnt[kMaxSpecies];
+  double *n[kMaxSpecies];
+  double scale[kMaxSpecies];  // w0 * 2^-48
+  double q[kMaxSpecies];
+  int consume[kMaxSpecies];
+};
+__device__ __forceinline__ void finalize_node(const FinalizeArgs &A, const double *__restrict__ vol_inv,
+                                              const double *__restrict__ bg, double *__restrict__ rho, int k,
+                                              int &flags) {
+  // all loads of the node first (independent, in flight together), then the
+  // arithmetic and the stores
+  const double vi = vol_inv[k];
+  const double b = bg ? bg[k] : 0.0;
+  unsigned long long a[kMaxSpecies];
+  unsigned cn[kMaxSpecies];
+  double nold[kMaxSpecies];
+#pragma unroll
+  for (int s = 0; s < kMaxSpecies; s++) {
+    if (s >= A.ns) break;
+    if (A.consume[s]) {
+      a[s] = A.acc[s][k];
+      cn[s] = A.cnt[s][k];
+    } else {
+      nold[s] = A.n[s][k];
+    }
+  }
+  double r = 0.0;
+#pragma unroll
+  for (int s = 0; s < kMaxSpecies; s++) {
+    if (s >= A.ns) break;
+    double n;
+    if (A.consume[s]) {
+      if (cn[s] > kMaxCell) flags |= DERR_OVERFLOW;
+      n = (double)a[s] * A.scale[s] * vi;
+      A.n[s][k] = n;
+      A.acc[s][k] = 0ull;
+      A.cnt[s][k] = 0u;
+    } else {
+      n = nold[s];
+    }
+    r += n * A.q[s];
+  }
+  if (rho) rho[k] = r + b;
+}
 int launch_step_density(Ctx *c);  // ρ of a graph step (with the fused warm start)
+int step_density_args(Ctx *c, bool df, FinalizeArgs &A, FinalizeDfArgs &D);
+bool poisson_one_block(Ctx *c);               // a step's field part runs as one block
+int launch_field_block(Ctx *c, double rtol);  // circuit, density, ρ, solve and E of a step
 void poisson_destroy(Poisson *p);
 void mcc_destroy(Mcc *m);
 

@@ -181,58 +181,12 @@ int launch_deposit(Ctx *c, int sid) {
 // ---------------------------------------------------------------------------
 // density + charge density
 // ---------------------------------------------------------------------------
-struct FinalizeArgs {
-  int ns;
-  unsigned long long *acc[kMaxSpecies];
-  unsigned *cnt[kMaxSpecies];
-  double *n[kMaxSpecies];
-  double scale[kMaxSpecies];  // w0 * 2^-48
-  double q[kMaxSpecies];
-  int consume[kMaxSpecies];
-};
-
-
-
 __global__ void k_finalize(FinalizeArgs A, const double *__restrict__ vol_inv, const double *__restrict__ bg,
                            double *__restrict__ rho, int nn, int *err) {
   pdl_wait();
   int flags = 0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x) {
-    // all loads of the node first (independent, in flight together), then the
-    // arithmetic and the stores
-    const double vi = vol_inv[k];
-    const double b = bg ? bg[k] : 0.0;
-    unsigned long long a[kMaxSpecies];
-    unsigned cn[kMaxSpecies];
-    double nold[kMaxSpecies];
-#pragma unroll
-    for (int s = 0; s < kMaxSpecies; s++) {
-      if (s >= A.ns) break;
-      if (A.consume[s]) {
-        a[s] = A.acc[s][k];
-        cn[s] = A.cnt[s][k];
-      } else {
-        nold[s] = A.n[s][k];
-      }
-    }
-    double r = 0.0;
-#pragma unroll
-    for (int s = 0; s < kMaxSpecies; s++) {
-      if (s >= A.ns) break;
-      double n;
-      if (A.consume[s]) {
-        if (cn[s] > kMaxCell) flags |= DERR_OVERFLOW;
-        n = (double)a[s] * A.scale[s] * vi;
-        A.n[s][k] = n;
-        A.acc[s][k] = 0ull;
-        A.cnt[s][k] = 0u;
-      } else {
-        n = nold[s];
-      }
-      r += n * A.q[s];
-    }
-    if (rho) rho[k] = r + b;
-  }
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x)
+    finalize_node(A, vol_inv, bg, rho, k, flags);
   if (flags) atomicOr(err, flags);
 }
 
@@ -297,17 +251,11 @@ static int sync_n64(Ctx *c, Species &sp) {
   return ISKRA_OK;
 }
 
-// Brings every species' density up to date (depositing species whose
-// positions changed without a deposit, consuming unconsumed accumulators) and,
-// when with_rho, forms ρ -- in double-float when the next solve takes it so
-// (separable operator with a double-float state), else in FP64.
-static int finalize(Ctx *c, bool with_rho, bool step = false) {
-  const bool df = with_rho && poisson_df_rho(c);
-  c->warm_fused = false;
-  FinalizeArgs A{};
-  FinalizeDfArgs D{};
+// Arguments of a density pass over every species (depositing species whose
+// positions changed without a deposit); *any: some accumulator is unconsumed.
+static int finalize_args(Ctx *c, bool df, FinalizeArgs &A, FinalizeDfArgs &D, bool *any) {
   A.ns = D.ns = (int)c->species.size();
-  bool any = false;
+  *any = false;
   for (int s = 0; s < A.ns; s++) {
     Species &sp = c->species[s];
     if (!sp.acc_valid && !sp.n_valid) {
@@ -332,8 +280,40 @@ static int finalize(Ctx *c, bool with_rho, bool step = false) {
     A.q[s] = sp.q;
     D.q[s] = df_host(sp.q);
     A.consume[s] = D.consume[s] = sp.acc_valid ? 1 : 0;
-    any |= sp.acc_valid;
+    *any |= sp.acc_valid;
   }
+  return ISKRA_OK;
+}
+
+// which copies are current after a density pass
+static void finalize_done(Ctx *c, bool df, bool with_rho) {
+  if (with_rho) {
+    c->rho_df_valid = df;
+    c->rho64_valid = !df;
+  }
+  for (auto &sp : c->species) {
+    if (sp.acc_valid) {
+      sp.acc_valid = false;
+      sp.acc_zero = true;
+      sp.n64_valid = !df;
+      sp.n_df_valid = df;
+    }
+    sp.n_valid = true;
+  }
+}
+
+// Brings every species' density up to date (consuming unconsumed
+// accumulators) and, when with_rho, forms ρ -- in double-float when the next
+// solve takes it so (separable operator with a double-float state), else in
+// FP64.
+static int finalize(Ctx *c, bool with_rho, bool step = false) {
+  const bool df = with_rho && poisson_df_rho(c);
+  c->warm_fused = false;
+  FinalizeArgs A{};
+  FinalizeDfArgs D{};
+  bool any = false;
+  const int rc = finalize_args(c, df, A, D, &any);
+  if (rc) return rc;
   if (!any && !with_rho) return ISKRA_OK;
   if (df) {
     WarmArgs W{};
@@ -345,27 +325,23 @@ static int finalize(Ctx *c, bool with_rho, bool step = false) {
       ISKRA_CUDA(c, launch_pdl(k_finalize_df<false>, node_blocks(c), 256, 0, c->stream, D,
                                (const float2 *)c->vol_inv_df, (const float2 *)c->bg_df, c->rho_df, c->nn, c->d_err, W));
     }
-    c->rho_df_valid = true;
-    c->rho64_valid = false;
   } else {
     ISKRA_CUDA(c, launch_pdl(k_finalize, node_blocks(c), 256, 0, c->stream, A, (const double *)c->vol_inv,
                              (const double *)c->rho_bg, with_rho ? c->rho : nullptr, c->nn, c->d_err));
-    if (with_rho) {
-      c->rho64_valid = true;
-      c->rho_df_valid = false;
-    }
   }
   ISKRA_CUDA(c, cudaGetLastError());
-  for (int s = 0; s < A.ns; s++) {
-    Species &sp = c->species[s];
-    if (sp.acc_valid) {
-      sp.acc_valid = false;
-      sp.acc_zero = true;
-      sp.n64_valid = !df;
-      sp.n_df_valid = df;
-    }
-    sp.n_valid = true;
-  }
+  finalize_done(c, df, with_rho);
+  return ISKRA_OK;
+}
+
+// The same for a step whose density pass runs inside the one-block field
+// kernel (poisson.cu): its arguments instead of a launch.
+int step_density_args(Ctx *c, bool df, FinalizeArgs &A, FinalizeDfArgs &D) {
+  bool any = false;
+  const int rc = finalize_args(c, df, A, D, &any);
+  if (rc) return rc;
+  c->warm_fused = false;
+  finalize_done(c, df, true);
   return ISKRA_OK;
 }
 

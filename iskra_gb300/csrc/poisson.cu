@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(64) k_tridiag(float *__restrict__ spec, int nx
 // contiguously (fwd: nf (α, γ) pairs, back: nb (a/b, c/b) pairs, backb: nb
 // 1/b, then 1/b of the last row), and the block stages them in shared memory
 // with the data in one pass, so the 2L dependent levels run on shared memory
-// only.  Work item `item` takes modes G item ...; ends with a block barrier.
+// only.  A block takes modes G blockIdx.x ...
 struct CrArgs {
   float *spec;
   int nx, K, G, L, nf, nb;
@@ -903,35 +903,45 @@ struct CrArgs {
   int cyclic, pin0;
 };
 
-__device__ __forceinline__ void cr_item(int item, const CrArgs &A, float *fsh) {
-  const int nx = A.nx, K = A.K, G = A.G, L = A.L, nf = A.nf, nb = A.nb;
-  float *__restrict__ spec = A.spec;
-  const int k0 = item * G;
-  const int g = min(G, K - k0), ncol = 2 * g;
-  float2 *cf = reinterpret_cast<float2 *>(fsh + 2 * G * nx);  // [g][nf]
-  float2 *cb = cf + (size_t)G * nf;                            // [g][nb]
-  float *cbb = reinterpret_cast<float *>(cb + (size_t)G * nb);  // [g][nb]
-  for (int t = threadIdx.x; t < g * nf; t += blockDim.x) cf[t] = __ldg(A.fwd + (size_t)k0 * nf + t);
+// shared-memory layout of a block's modes: data of 2G columns, then per mode the
+// coefficients
+struct CrShared {
+  float *d;            // [col][nx]
+  float2 *cf, *cb;     // [g][nf], [g][nb]
+  float *cbb;          // [g][nb]
+};
+__device__ __forceinline__ CrShared cr_shared(const CrArgs &A, float *fsh) {
+  CrShared q;
+  q.d = fsh;
+  q.cf = reinterpret_cast<float2 *>(fsh + 2 * A.G * A.nx);
+  q.cb = q.cf + (size_t)A.G * A.nf;
+  q.cbb = reinterpret_cast<float *>(q.cb + (size_t)A.G * A.nb);
+  return q;
+}
+// coefficients of modes k0 .. k0 + g - 1 (no barrier)
+__device__ __forceinline__ void cr_stage(const CrArgs &A, const CrShared &q, int k0, int g) {
+  const int nf = A.nf, nb = A.nb;
+  for (int t = threadIdx.x; t < g * nf; t += blockDim.x) q.cf[t] = __ldg(A.fwd + (size_t)k0 * nf + t);
   for (int t = threadIdx.x; t < g * nb; t += blockDim.x) {
-    cb[t] = __ldg(A.back + (size_t)k0 * nb + t);
-    cbb[t] = __ldg(A.backb + (size_t)k0 * nb + t);
+    q.cb[t] = __ldg(A.back + (size_t)k0 * nb + t);
+    q.cbb[t] = __ldg(A.backb + (size_t)k0 * nb + t);
   }
-  for (int t = threadIdx.x; t < nx * ncol; t += blockDim.x) {
-    const int i = t / ncol, col = t - i * ncol;
-    const int k = k0 + (col >> 1);
-    float v = spec[((size_t)i * K + k) * 2 + (col & 1)];
-    if (A.pin0 >= 0 && k == 0 && i == A.pin0) v = 0.f;  // pinned row of the singular mode
-    fsh[col * nx + i] = v;
-  }
-  __syncthreads();
+}
+// The 2L levels on the staged columns; REAL: one real column per mode (ny = 2),
+// else its real and imaginary parts.  Ends with a block barrier.
+template <bool REAL>
+__device__ __forceinline__ void cr_levels(const CrArgs &A, const CrShared &q, int k0, int ncol) {
+  const int nx = A.nx, L = A.L, nf = A.nf, nb = A.nb;
+  constexpr int sh = REAL ? 0 : 1;  // column -> mode
+  if (REAL) ncol = 2;
   int F = 0, B = 0;
   for (int l = 0; l < L; l++) {
     const int s = 1 << l, cnt = nx >> (l + 1);
     for (int t = threadIdx.x; t < cnt * ncol; t += blockDim.x) {
       const int m = t / ncol, col = t - m * ncol;
       const int i = (m + 1) * 2 * s - 1;
-      const float2 ag = cf[(col >> 1) * nf + F + m];
-      float *dc = fsh + col * nx;
+      const float2 ag = q.cf[(col >> sh) * nf + F + m];
+      float *dc = q.d + col * nx;
       float v = dc[i] - ag.x * dc[i - s];
       if (i + s < nx) v -= ag.y * dc[i + s];
       dc[i] = v;
@@ -941,7 +951,7 @@ __device__ __forceinline__ void cr_item(int item, const CrArgs &A, float *fsh) {
     __syncthreads();
   }
   const int topr = (1 << L) - 1;
-  for (int col = threadIdx.x; col < ncol; col += blockDim.x) fsh[col * nx + topr] *= __ldg(A.top + k0 + (col >> 1));
+  for (int col = threadIdx.x; col < ncol; col += blockDim.x) q.d[col * nx + topr] *= __ldg(A.top + k0 + (col >> sh));
   __syncthreads();
   for (int l = L - 1; l >= 0; l--) {
     const int s = 1 << l, ecnt = ((nx >> l) + 1) >> 1;
@@ -949,32 +959,55 @@ __device__ __forceinline__ void cr_item(int item, const CrArgs &A, float *fsh) {
     for (int t = threadIdx.x; t < ecnt * ncol; t += blockDim.x) {
       const int m = t / ncol, col = t - m * ncol;
       const int j = (2 * m + 1) * s - 1;
-      const int o = (col >> 1) * nb + B + m;
-      const float2 r = cb[o];
-      float *dc = fsh + col * nx;
-      float x = cbb[o] * dc[j];
+      const int o = (col >> sh) * nb + B + m;
+      const float2 r = q.cb[o];
+      float *dc = q.d + col * nx;
+      float x = q.cbb[o] * dc[j];
       if (j - s >= 0) x -= r.x * dc[j - s];
       if (j + s < nx) x -= r.y * dc[j + s];
       dc[j] = x;
     }
     __syncthreads();
   }
+}
+// solution of mode k at row i from its solved column (Sherman-Morrison for
+// x-periodic operators)
+__device__ __forceinline__ float cr_value(const CrArgs &A, const float *dc, int k, int i) {
+  float v = dc[i];
+  if (A.cyclic && !(k == 0 && A.pin0 >= 0))
+    v -= (dc[0] + A.gk[A.K + k] * dc[A.nx - 1]) * A.gk[k] * A.q[(size_t)i * A.K + k];
+  return v;
+}
+
+// spec -> spec for the modes of work item `item` (staged coefficients, data in
+// q.d).  Ends with a block barrier.
+__device__ __forceinline__ void cr_solve(const CrArgs &A, const CrShared &q, float *__restrict__ spec, int k0, int g) {
+  const int nx = A.nx, K = A.K, ncol = 2 * g;
   for (int t = threadIdx.x; t < nx * ncol; t += blockDim.x) {
     const int i = t / ncol, col = t - i * ncol;
     const int k = k0 + (col >> 1);
-    const float *dc = fsh + col * nx;
-    float v = dc[i];
-    if (A.cyclic && !(k == 0 && A.pin0 >= 0)) v -= (dc[0] + A.gk[K + k] * dc[nx - 1]) * A.gk[k] * A.q[(size_t)i * K + k];
-    spec[((size_t)i * K + k) * 2 + (col & 1)] = v;
+    float v = spec[((size_t)i * K + k) * 2 + (col & 1)];
+    if (A.pin0 >= 0 && k == 0 && i == A.pin0) v = 0.f;  // pinned row of the singular mode
+    q.d[col * nx + i] = v;
+  }
+  __syncthreads();
+  cr_levels<false>(A, q, k0, ncol);
+  for (int t = threadIdx.x; t < nx * ncol; t += blockDim.x) {
+    const int i = t / ncol, col = t - i * ncol;
+    const int k = k0 + (col >> 1);
+    spec[((size_t)i * K + k) * 2 + (col & 1)] = cr_value(A, q.d + col * nx, k, i);
   }
   __syncthreads();
 }
 
 __global__ void __launch_bounds__(256) k_tridiag_cr(CrArgs A, const PoissonScal *__restrict__ sc) {
   pdl_wait();
-  extern __shared__ float fsh[];  // data [col][nx] (col = 2 (k - k0) + part), then per mode fwd, back, backb
+  extern __shared__ float fsh[];  // CrShared (column = 2 (k - k0) + part)
   if (sc->done) return;
-  cr_item(blockIdx.x, A, fsh);
+  const int k0 = blockIdx.x * A.G, g = min(A.G, A.K - k0);
+  const CrShared q = cr_shared(A, fsh);
+  cr_stage(A, q, k0, g);
+  cr_solve(A, q, A.spec, k0, g);
 }
 
 // spec -> δ (nx, ny) by the inverse of k_fft_fwd for work item `item`; x +=
@@ -2333,6 +2366,302 @@ int poisson_solve_graph(Ctx *c, double rtol) {
   rc = queue_sweeps(c, rtol, n, false, last);
   if (rc) return rc;
   return finish_solve(c);
+}
+
+// ---- a step's field part in one block ------------------------------------------
+// On grids of up to kFieldBlockNodes nodes the circuit, the density pass, the warm
+// start, the driven rows, the residuals and corrections, and E run as phases of
+// one 512-thread block with ϕ, the right-hand side, the residual and the spectrum
+// in shared memory: at these sizes each of the 9 (double-float) to 18 (FP64,
+// singular) launches they took costs 3-10 us of launch and memory latency for
+// well under a microsecond of work.  The phases are the multi-launch path's own
+// node and line functions, so ϕ, ρ and E are the same bits; only the norms'
+// summation order differs.  At ny = 2 (the quasi-1D grids) the transform is a sum
+// and a difference, taken while the lines are loaded and stored.  Whole steps:
+// 257 x 2 discharge 103 -> 85 us, 128 x 2 periodic beams 94 -> 68 us with their
+// record (the block itself 17 and 25 us with warm caches).  A cluster of eight
+// such blocks did not pay: its barriers cost 2-3 us each (128 x 2: no gain over
+// the launches, 128 x 64: 56 against 50 us).
+struct FieldBlock {
+  FinalizeArgs A;
+  FinalizeDfArgs D;
+  CircuitArgs cir;             // cir.cd == nullptr: none
+  unsigned long long *cir_seen;
+  const double *vol_inv, *bg;
+  const float2 *vol_inv_df, *bg_df;
+  double *rho;
+  float2 *rho_df;
+  int warm;                    // ϕ <- 2 ϕ_n - ϕ_(n-1) once the history is valid
+  OpView op;
+  double *x;
+  float2 *xd;
+  void *xh;
+  PoissonScal *sc;
+  const int *dnode, *dgroup;
+  const double *dpar;
+  int ndn;
+  const unsigned long long *step;
+  double dt, nie, rtol2, dsum;
+  float2 nie_df;
+  double *bfix;
+  int singular, rho_fixed, sweeps, nn;
+  FftPlan F;
+  CrArgs C;
+  EOut eo;
+  int *err, *notconv;
+};
+constexpr int kFieldThreads = 512;
+// MODE: 0 ny = 2, 1 ny another power of two, 2 any other ny
+template <bool DF, int MODE>
+__global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
+  extern __shared__ __align__(16) unsigned char field_smem[];
+  __shared__ double red[2 * kFieldThreads];
+  __shared__ RowClass cls_sh[kSmemClasses];
+  const int tid = threadIdx.x, T = kFieldThreads, nn = P.nn, nx = P.op.nx, ny = P.op.ny;
+  constexpr bool TWO = MODE == 0, ODD = MODE == 2;
+  // shared memory: ϕ, b or ρ (8 B a node), residual, spectrum, then the
+  // transform's columns or the lines of the cyclic reduction
+  float2 *xd = reinterpret_cast<float2 *>(field_smem), *bd = xd + nn;
+  double *x64 = reinterpret_cast<double *>(field_smem), *rho64 = x64 + nn;
+  float *r32 = reinterpret_cast<float *>(bd + nn);
+  float2 *spec = reinterpret_cast<float2 *>(r32 + (nn + (nn & 1)));
+  float2 *fbuf = spec + (TWO ? 0 : (size_t)nx * P.C.K);
+  // coefficients of the lines: written by the operator build, read before the wait
+  const size_t fft_n = TWO ? 0 : (ODD ? 2 : 1) * (size_t)((nx + 1) / 2) * (P.F.N + 1) + P.F.N / 2 + (ODD ? P.F.odd : 0);
+  const CrShared cr = cr_shared(P.C, reinterpret_cast<float *>(fbuf + fft_n));
+  cr_stage(P.C, cr, 0, P.C.K);
+  const RowClass *CT = stage_classes(P.op, cls_sh);
+  PoissonScal *sc = P.sc;
+  pdl_wait();
+  const bool rho_df = DF && !P.singular && !P.rho_fixed;  // ρ formed in double-float
+  const bool hist = P.warm && sc->hist != 0;
+  // The last warp: circuit (it reads ϕ of the last step in global memory, which
+  // is rewritten at the end) and driven values (a sine each in FP64) beside the
+  // density pass.
+  if (P.cir.cd && tid == T - 1) circuit_advance(P.cir, P.dt, P.cir_seen);
+  // driven rows (the solve of step n uses V((n-2)Δt), n >= 2)
+  for (int t = tid - (T - 32); t >= 0 && t < P.ndn; t += 32) {
+    const unsigned long long n_step = *P.step;
+    if (n_step >= 2) P.bfix[P.dnode[t]] = drive_value(P.dpar + 4 * P.dgroup[t], (double)(n_step - 2) * P.dt);
+  }
+  {
+    int flags = 0;
+    for (int k = tid; k < nn; k += T) {
+      if (rho_df) {
+        finalize_df_node(P.D, P.vol_inv_df, P.bg_df, P.rho_df, k, flags);
+      } else {
+        finalize_node(P.A, P.vol_inv, P.bg, P.rho, k, flags);
+        if (!DF) rho64[k] = P.rho[k];
+      }
+      const bool upd = hist && !(P.op.cls[k] & kFixedBit);
+      if (DF) {
+        const float2 a = P.xd[k];
+        xd[k] = upd ? df_add(make_float2(2.f * a.x, 2.f * a.y), df_neg(((float2 *)P.xh)[k])) : a;
+        if (P.warm) ((float2 *)P.xh)[k] = a;
+      } else {
+        const double a = P.x[k];
+        x64[k] = upd ? 2.0 * a - ((double *)P.xh)[k] : a;
+        if (P.warm) ((double *)P.xh)[k] = a;
+      }
+    }
+    if (flags) atomicOr(P.err, flags);
+  }
+  __syncthreads();
+  if (P.warm && tid == 0) sc->hist = 1;
+  if (P.ndn) {
+    for (int t = tid; t < P.ndn; t += T) {
+      const int k = P.dnode[t];
+      if (DF) xd[k] = df_from(P.bfix[k]);
+      else x64[k] = P.bfix[k];
+    }
+    __syncthreads();
+  }
+  if (P.rho_fixed) {  // ρ-valued identity rows
+    for (int k = tid; k < nn; k += T) {
+      const unsigned ck = P.op.cls[k];
+      if (ck & kFixedBit) {
+        const double v = CT[ck & kClassMask].rho ? P.rho[k] * P.nie : P.op.bfix[k];
+        if (DF) xd[k] = df_from(v);
+        else x64[k] = v;
+      }
+    }
+    __syncthreads();
+  }
+  const double *rho = DF ? P.rho : rho64;
+  double lam = 0.0;
+  if (P.singular) {  // projection of the right-hand side onto the range
+    double v[1] = {0}, t[1];
+    for (int k = tid; k < nn; k += T) {
+      const RowClass &C = CT[P.op.cls[k] & kClassMask];
+      if (!C.fixed) {
+        double b = C.rho ? rho[k] * P.nie : P.op.bfix[k];
+        if (C.sig_dof >= 0) b -= C.sig_coef * P.op.sigma[C.sig_dof];
+        v[0] += C.d * b;
+      }
+    }
+    block_sums<1>(v, red, t);
+    lam = P.dsum > 0 ? t[0] / P.dsum : 0.0;
+    if (tid == 0) sc->lambda = lam;
+  }
+  double rhs2 = 0;
+  for (int s = 0;; s++) {
+    double a2 = 0, b2 = 0;
+    if (DF) {
+      if (s == 0)
+        residual_df_nodes<true, false>(P.op, CT, xd, rho, rho_df ? P.rho_df : nullptr, P.nie_df, P.nie, bd, r32, nn,
+                                       P.singular, lam, P.eo, tid, T, a2, b2);
+      else
+        residual_df_nodes<false, false>(P.op, CT, xd, nullptr, nullptr, P.nie_df, P.nie, bd, r32, nn, P.singular, lam,
+                                        P.eo, tid, T, a2, b2);
+    } else {
+      for (int k = tid; k < nn; k += T) {
+        const int j = k / nx, i = k - j * nx;
+        r32[k] = s == 0 ? residual_node<true>(P.op, CT, x64, rho, P.nie, lam, P.singular, k, i, j, nullptr, a2, b2)
+                        : residual_node<false>(P.op, CT, x64, rho, P.nie, lam, P.singular, k, i, j, nullptr, a2, b2);
+      }
+    }
+    const double v[2] = {a2, b2};
+    double t[2];
+    block_sums<2>(v, red, t);
+    if (s == 0) rhs2 = t[1];
+    const bool done = (rhs2 > 0 && t[0] <= P.rtol2 * rhs2) || t[0] == 0.0;
+    if (done || s == P.sweeps) {
+      if (tid == 0) {
+        sc->rhs2 = rhs2;
+        sc->res2 = t[0];
+        sc->relres = rhs2 > 0 ? sqrt(t[0] / rhs2) : sqrt(t[0]);
+        sc->iters = s;
+        sc->done = done;
+        sc->e_pending = 0;
+        if (!done) atomicOr(P.notconv, DERR_NOTCONV);
+      }
+      break;
+    }
+    // one FP32 correction
+    if (TWO) {
+      for (int i = tid; i < nx; i += T) {
+        const float a = r32[i], b = r32[i + nx];
+        cr.d[i] = P.C.pin0 == i ? 0.f : a + b;
+        cr.d[nx + i] = a - b;
+      }
+      __syncthreads();
+      cr_levels<true>(P.C, cr, 0, 2);
+      for (int i = tid; i < nx; i += T) {
+        const float a = cr_value(P.C, cr.d, 0, i), b = cr_value(P.C, cr.d + nx, 1, i);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const int k = i + nx * j;
+          if (P.op.cls[k] & kFixedBit) continue;
+          const float dz = (j ? a - b : a + b) * 0.5f;
+          if (DF) xd[k] = df_add_f(xd[k], dz);
+          else x64[k] += (double)dz;
+        }
+      }
+    } else {
+      const int TP = (nx + 1) / 2;
+      fft_fwd_item<ODD>(0, r32, nx, P.F, TP, spec, fbuf);
+      __syncthreads();
+      cr_solve(P.C, cr, reinterpret_cast<float *>(spec), 0, P.C.K);
+      fft_inv_item<DF, ODD>(0, spec, nx, P.F, TP, P.op.cls, xd, x64, fbuf);
+    }
+    __syncthreads();
+  }
+  // E, and ϕ to memory
+  for (int k = tid; k < nn; k += T) {
+    const int j = k / nx, i = k - j * nx;
+    if (DF) {
+      const int w = i > 0 ? k - 1 : k + nx - 1, e = i < nx - 1 ? k + 1 : k - nx + 1;
+      const int so = j > 0 ? k - nx : k + nx * (ny - 1), no = j < ny - 1 ? k + nx : k - nx * (ny - 1);
+      efield_df5(xd[k], xd[w], xd[e], xd[so], xd[no], k, i, j, nx, ny, P.eo);
+      if (!P.singular) P.xd[k] = xd[k];
+    } else {
+      efield_at(x64, k, i, j, nx, ny, P.eo);
+      if (!P.singular) P.x[k] = x64[k];
+    }
+  }
+  if (P.singular) {  // mean-zero ϕ
+    double v[1] = {0}, t[1];
+    for (int k = tid; k < nn; k += T) v[0] += DF ? df_value(xd[k]) : x64[k];
+    block_sums<1>(v, red, t);
+    const double m = t[0] / nn;
+    for (int k = tid; k < nn; k += T) {
+      if (DF) P.xd[k] = df_add(xd[k], df_neg(df_from(m)));
+      else P.x[k] = x64[k] - m;
+    }
+  }
+}
+
+// Largest grids whose field part runs as one block: the crossing with the
+// multi-launch path (whole steps: 33 x 32 36 against 43 us, 48 x 32 45 against 47,
+// 65 x 32 51 against 49; ny = 2: 1000 x 2 90 against 104, 2000 x 2 105 against
+// 109, 3000 x 2 equal).
+constexpr int kFieldBlockNodes = 1536, kFieldBlockNodes1D = 4096;
+constexpr size_t kFieldSmem = 192 * 1024;  // beside 28 KB of static arrays
+
+static size_t field_block_bytes(const Poisson *P) {
+  const size_t nn = P->nn;
+  size_t b = 20 * (nn + 1) + cr_smem(P, P->K);
+  if (P->N > 2) b += (size_t)P->nx * P->K * sizeof(float2) + fft_smem(P->N, P->odd, (P->nx + 1) / 2);
+  return b;
+}
+
+bool poisson_one_block(Ctx *c) {
+  const Poisson *P = c->ps;
+  return P && !P->dirty && P->separable && P->nn <= (P->N == 2 ? kFieldBlockNodes1D : kFieldBlockNodes) &&
+         field_block_bytes(P) <= kFieldSmem;
+}
+
+int launch_field_block(Ctx *c, double rtol) {
+  Poisson *P = c->ps;
+  const bool df = P->df_mode, rho_df = poisson_df_rho(c);
+  FieldBlock B{};
+  int rc = ISKRA_OK;
+  if (c->cir_d) {
+    rc = circuit_args(c, B.cir);
+    B.cir_seen = c->cir_seen;
+  }
+  if (!rc) rc = step_density_args(c, rho_df, B.A, B.D);
+  if (rc) return rc;
+  B.vol_inv = c->vol_inv;
+  B.bg = c->rho_bg;
+  B.vol_inv_df = c->vol_inv_df;
+  B.bg_df = c->bg_df;
+  B.rho = c->rho;
+  B.rho_df = c->rho_df;
+  B.warm = P->warm_mode == 1;
+  B.op = opview(P);
+  B.x = P->x;
+  B.xd = P->xd;
+  B.xh = P->xh;
+  B.sc = P->scal;
+  B.dnode = P->drive_node;
+  B.dgroup = P->drive_group;
+  B.dpar = P->drive_par;
+  B.ndn = P->ndrive_nodes;
+  B.step = c->d_step;
+  B.dt = c->graph_dt;
+  B.nie = -1.0 / P->eps0;
+  B.nie_df = df_host(B.nie);
+  B.rtol2 = rtol * rtol;
+  B.dsum = P->dsum;
+  B.bfix = P->bfix_d;
+  B.singular = P->singular;
+  B.rho_fixed = P->rho_fixed;
+  B.sweeps = std::min(8, graph_sweeps(P, rtol) + 2);  // (sweeps not needed cost nothing here)
+  B.nn = P->nn;
+  B.F = FftPlan{P->N, P->log2p, P->odd, P->tw, P->tw + P->N / 2};
+  B.C = cr_args(P, P->K);
+  B.eo = eout(c, true);
+  B.err = c->d_err;
+  B.notconv = c->d_err;
+  const int mode = P->N == 2 ? 0 : P->odd > 1 ? 2 : 1;
+  auto kern = df ? (mode == 0 ? k_field_block<true, 0> : mode == 1 ? k_field_block<true, 1> : k_field_block<true, 2>)
+                 : (mode == 0 ? k_field_block<false, 0> : mode == 1 ? k_field_block<false, 1> : k_field_block<false, 2>);
+  ISKRA_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFieldSmem));
+  ISKRA_CUDA(c, launch_pdl(kern, 1, kFieldThreads, field_block_bytes(P), c->stream, B));
+  c->e_from_phi = true;
+  if (df) P->x_stale = true;
+  return ISKRA_OK;
 }
 
 // Learned warm start of a CG solve: δ = scale y on the free rows (the

@@ -20,58 +20,17 @@ bool poisson_separable(Ctx *c);
 int poisson_solve_blocking(Ctx *c, double rtol, int maxit);
 int poisson_solve_graph(Ctx *c, double rtol);
 
-struct CircuitArgs {
-  CircuitDev *cd;
-  const double *phi;
-  const float2 *phid;          // ϕ as double-float pairs (separable solver), else nullptr
-  double *sigma;
-  int pos_ref, neg_ref;
-  int wall;                    // discard wall feeding the floating electrode, -1 none
-  int ns;
-  SpeciesState *st[kMaxSpecies];
-  double qw[kMaxSpecies];      // q * w0 per species
-};
-
-// advance!(circuit, ϕ, Δt, config) (circuit_coupling.jl:35-43) with
-// advance_circuit! (Circuit.jl:117-136); V_ext = ϕ(positive) - ϕ(negative)
-// of the PlasmaDevice (circuit_coupling.jl:18-29); wall-absorbed charge enters
-// σ as hit! does (circuit_coupling.jl:45-55).  One thread, FP64.
+// One thread, FP64.
 __global__ void k_circuit(CircuitArgs A, double dt, unsigned long long *seen) {
   pdl_wait();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  CircuitDev &c = *A.cd;
-  auto phi_at = [&](int k) { return A.phid ? (double)A.phid[k].x + (double)A.phid[k].y : A.phi[k]; };
-  const double vext = phi_at(A.pos_ref) - phi_at(A.neg_ref);
-  const double i = c.i, q = c.q, t = c.t;
-  const double vsrc = c.amp * sin(2.0 * M_PI * c.freq * t) + c.dc;
-  double in = (c.L / dt - c.R / 2) * i + vext - vsrc;
-  if (c.C > 0.0) {
-    in -= q / c.C;
-    in /= (c.L / dt + c.R / 2);
-    c.q = q + dt * i;
-  } else {
-    in /= (c.L / dt + c.R / 2);
-  }
-  c.i = in;
-  c.t = t + dt;
-  c.vext = vext;
-  double ds = -dt * in / c.area * c.scale;
-  if (A.wall >= 0) {
-    for (int s = 0; s < A.ns; s++) {
-      const unsigned long long now = A.st[s]->absorbed[A.wall];
-      const unsigned long long d = now - seen[s];
-      seen[s] = now;
-      ds += A.qw[s] * (double)d / c.area;
-    }
-  }
-  A.sigma[c.sigma_dof] += ds;
+  if (threadIdx.x == 0 && blockIdx.x == 0) circuit_advance(A, dt, seen);
 }
 
 __global__ void k_step_begin(unsigned long long *d_step) { pdl_wait(); *d_step += 1ull; }
 
-int launch_circuit(Ctx *c, double dt) {
+int circuit_args(Ctx *c, CircuitArgs &A) {
   if (!c->cir_d) return set_err(c, ISKRA_EINVAL, "no circuit");
-  CircuitArgs A{};
+  A = CircuitArgs{};
   A.cd = c->cir_d;
   A.phi = poisson_x_ptr(c);
   A.phid = poisson_xd_ptr(c);
@@ -84,6 +43,13 @@ int launch_circuit(Ctx *c, double dt) {
     A.st[s] = c->species[s].dev.st;
     A.qw[s] = c->species[s].q * c->species[s].w0;
   }
+  return ISKRA_OK;
+}
+
+int launch_circuit(Ctx *c, double dt) {
+  CircuitArgs A;
+  const int rc = circuit_args(c, A);
+  if (rc) return rc;
   ISKRA_CUDA(c, launch_pdl(k_circuit, 1, 32, 0, c->stream, A, dt, c->cir_seen));
   ISKRA_CUDA(c, cudaGetLastError());
   return ISKRA_OK;
@@ -115,6 +81,8 @@ static int queue_step(Ctx *c, double dt, uint64_t seed, double rtol, bool blocki
       ISKRA_CUDA(c, cudaGetLastError());
     }
   }
+  // small grids: circuit, density, ρ, solve and E in one block
+  if (!blocking_solve && poisson_one_block(c)) return launch_field_block(c, rtol);
   if (c->cir_d) {
     rc = launch_circuit(c, dt);
     if (rc) return rc;
