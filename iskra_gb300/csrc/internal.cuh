@@ -143,6 +143,22 @@ __device__ __forceinline__ MccWork mcc_entry(float4 a, float2 b, uint32_t pid, u
   return e;
 }
 
+// Appends a warp's n <= 32 buffered work-list entries to its run's list
+// (counter cnt, segment seg of cap entries).
+__device__ __forceinline__ void flush_entries(const MccWork *buf, int n, unsigned long long *cnt,
+                                              MccWork *__restrict__ seg, unsigned long long cap, int &flags) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();  // the entries are in buf
+  unsigned long long at = 0;
+  if (lane == 0) at = atomicAdd(cnt, (unsigned long long)n);
+  at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)lane;
+  if (lane < n) {
+    if (at < cap) seg[at] = buf[lane];
+    else flags |= DERR_CAPACITY;
+  }
+  __syncwarp();  // buf may be written again
+}
+
 // uniform in [0,1) with 24 random bits
 __device__ __forceinline__ float u01(uint32_t v) { return (float)(v >> 8) * 5.9604644775390625e-08f; }
 
@@ -764,7 +780,8 @@ int launch_efield_from(Ctx *c, const double *phi);
 int launch_efield64(Ctx *c, const double *phi);
 int launch_sort(Ctx *c, int sid);
 int species_speed2(Ctx *c, int sid, double *mean_v2);  // <vx² + vy²> of the live particles (synchronises)
-int launch_mcc(Ctx *c, int mid, double dt, uint64_t seed, const unsigned long long *d_step, uint64_t step_host);
+int launch_mcc_begin(Ctx *c, unsigned long long *step_ctr);  // before the MCC sets of a step
+int launch_mcc(Ctx *c, int mid, double dt, uint64_t seed, const unsigned long long *d_step);
 int launch_circuit(Ctx *c, double dt);
 int launch_surface_charge(Ctx *c);  // σ credit of floating-electrode hits (after a push)
 void tracker_destroy(Ctx *c);

@@ -168,6 +168,10 @@ __device__ __forceinline__ long long warp_reserve(bool want, long long *np, unsi
 // warp of phase 2 holds 32 colliding particles instead of the ~3 a single
 // pass over all particles would, and it reads them as one contiguous
 // 32-byte entry each instead of three scattered records.
+// Resident blocks per SM asked for k_mcc_find (4: the same, 6: 6 % slower).
+#ifndef ISKRA_MCC_FIND_PER_SM
+#define ISKRA_MCC_FIND_PER_SM 5
+#endif
 constexpr int kSelChunk = 1024;  // particles per block pass of k_mcc_select
 // words of hit bits per run (one bit per work-list entry), after the entries
 __host__ __device__ __forceinline__ size_t hit_words(size_t cap) { return (cap + 31) / 32; }
@@ -348,6 +352,114 @@ __global__ void __launch_bounds__(256) k_mcc_test(MccDev M, const uint2 *__restr
   }
 }
 
+// Phases 1 and 2a of a single context in one kernel: each warp draws the
+// selection counts of 32 U particles (their cell words and identifiers all loaded
+// at once), lists the selected ones in its shared memory, tests those 32 at a time
+// -- each lane one selected particle: its record, its node's gas density and
+// field, the cross section -- and appends the entries that collide to the work
+// list, 32 with one reservation.  The selected entries (a tenth of the particles)
+// never go through memory, and k_mcc_collide finds a list of collisions alone.
+// Warps never wait for one another: with block-wide lists and barriers the pass
+// took 237 us a set at 32 M particles on 1024 x 1024 nodes (mean of electrons and
+// ions), this one 131 (175 and 87), the two launches it replaced (k_mcc_select
+// with one cell word and identifier in flight per thread, k_mcc_test) 423 us.
+// The ions' 87 us stand against 57 us for reading 12 B a particle; the rest is the
+// issue of the selection hash (two 64-bit multiplications) and of the tests.
+// U = 8 (4: 5 % slower) where every SM's warps get several rounds, else U = 2.
+template <int U>
+__global__ void __launch_bounds__(256, ISKRA_MCC_FIND_PER_SM) k_mcc_find(
+    SpeciesDev s, MccDev M, const float2 *__restrict__ E, int nx, const unsigned long long *__restrict__ d_step,
+    MccWork *__restrict__ work, unsigned long long *__restrict__ nwork, unsigned long long cap_work, int *err) {
+  extern __shared__ float tab[];
+  __shared__ uint32_t sel_sh[8][32 * U + 32];  // selected slots: at most 31 left over and 32 U new
+  __shared__ MccWork hit_sh[8][64];   // colliding entries, likewise
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const float *te = M.eps, *ts = M.sig;
+  if (M.staged) {  // (written by the set's creation, read before the wait)
+    const int ntab = M.off[M.N];
+    for (int t = threadIdx.x; t < ntab; t += 256) {
+      tab[t] = M.eps[t];
+      tab[ntab + t] = M.sig[t];
+    }
+    te = tab;
+    ts = tab + ntab;
+    __syncthreads();
+  }
+  pdl_wait();
+  const long long np = s.st->np;
+  const int cur = s.st->cur;
+  const float4 *__restrict__ xv = pick(s.xv[0], s.xv[1], cur);
+  const float2 *__restrict__ zc = pick(s.zc[0], s.zc[1], cur);
+  const uint32_t *__restrict__ ids = pick(s.id[0], s.id[1], cur);
+  const unsigned long long step = *d_step;
+  const uint2 key = make_uint2(M.key0, M.key1);
+  const float expl = __expf(-M.lam);
+  int flags = 0, nsel = 0, nhit = 0;  // listed entries (warp-uniform)
+  uint32_t *sel = sel_sh[wib];
+  MccWork *hb = hit_sh[wib];
+  auto test = [&](int n) {  // the last n <= 32 selected slots
+    bool hit = false;
+    MccWork e{};
+    nsel -= n;
+    if (lane < n) {
+      const uint32_t p = sel[nsel + lane];
+      e = mcc_entry(xv[p], zc[p], ids[p], p);
+      hit = mcc_entry_hits(e, M, te, ts, E, nx, step, key, expl);
+    }
+    const unsigned m = __ballot_sync(FULL, hit);
+    if (hit) hb[nhit + __popc(m & ((1u << lane) - 1u))] = e;
+    nhit += __popc(m);
+    if (nhit >= 32) {
+      nhit -= 32;
+      flush_entries(hb + nhit, 32, nwork, work, cap_work, flags);
+    }
+  };
+  const long long warp = ((long long)blockIdx.x * 256 + threadIdx.x) >> 5, nwarps = (long long)gridDim.x * 8;
+  for (long long base = warp * (32 * U); base < np; base += nwarps * (32 * U)) {
+    int cell[U];
+    uint32_t pid[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long p = base + 32 * u + lane;
+      cell[u] = -1;
+      pid[u] = 0;
+      if (p < np) {
+        cell[u] = __float_as_int(zc[p].y);
+        pid[u] = ids[p];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const bool on = cell[u] >= 0 && draw_selections(selection_uniform(pid[u], step, key), M.lam, expl) > 0;
+      const unsigned m = __ballot_sync(FULL, on);
+      if (on) sel[nsel + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(base + 32 * u + lane);
+      nsel += __popc(m);
+    }
+    __syncwarp();
+#pragma unroll 1
+    while (nsel >= 32) test(32);
+    __syncwarp();
+  }
+  __syncwarp();
+  if (nsel) test(nsel);
+  if (nhit) flush_entries(hb, nhit, nwork, work, cap_work, flags);
+  const int f = __reduce_or_sync(FULL, flags);
+  if (lane == 0 && f) atomicOr(err, f);
+}
+
+// What the last block of a single context's collision pass does: the appended
+// particles become part of the species, and the work list and the append cursors
+// are ready for the next set (ticket == nullptr: none of it, ensembles).
+struct MccEnd {
+  unsigned long long *nwork, *ticket;
+  SpeciesState *src, *prod;    // prod: nullptr without a product species
+  long long cap_src, cap_prod;
+};
+
+// ALL: every entry of the list collides (k_mcc_find); else the ones whose bit
+// k_mcc_test set.
+template <bool ALL>
 __global__ void __launch_bounds__(256, ISKRA_MCC_COLLIDE_MIN_BLOCKS) k_mcc_collide(const SpeciesDev *__restrict__ src,
                                                      const SpeciesDev *__restrict__ prod, int has_prod, MccDev M,
                                                      const uint2 *__restrict__ keys, unsigned long long *counts_runs,
@@ -356,14 +468,17 @@ __global__ void __launch_bounds__(256, ISKRA_MCC_COLLIDE_MIN_BLOCKS) k_mcc_colli
                                                      const MccWork *__restrict__ work,
                                                      const unsigned long long *__restrict__ nwork,
                                                      unsigned long long cap_run,
-                                                     const unsigned *__restrict__ hits, int *err) {
+                                                     const unsigned *__restrict__ hits, int *err, MccEnd end) {
   pdl_wait();
   extern __shared__ float tab[];
   const unsigned FULL = 0xffffffffu;
   // log-uniform tables take O(1) lookups, read through the caches; others
   // (binary search) are staged in shared memory
   const float *te = M.eps, *ts = M.sig;
-  if (M.staged) {
+  const int r = blockIdx.y;
+  const long long nw = (long long)min(nwork[(size_t)r * kNworkStride], cap_run);
+  const bool idle = ALL && (long long)blockIdx.x * blockDim.x >= nw;  // no entries for this block
+  if (M.staged && !idle) {
     const int ntab = M.off[M.N];
     for (int t = threadIdx.x; t < ntab; t += blockDim.x) {
       tab[t] = M.eps[t];
@@ -374,8 +489,6 @@ __global__ void __launch_bounds__(256, ISKRA_MCC_COLLIDE_MIN_BLOCKS) k_mcc_colli
     ts = tab + ntab;
   }
   const unsigned long long step = *d_step;
-  const int r = blockIdx.y;
-  const long long nw = (long long)min(nwork[(size_t)r * kNworkStride], cap_run);
   const MccWork *__restrict__ seg = work + (size_t)r * cap_run;
   const float expl = __expf(-M.lam);
   int flags = 0;
@@ -401,28 +514,7 @@ __global__ void __launch_bounds__(256, ISKRA_MCC_COLLIDE_MIN_BLOCKS) k_mcc_colli
   unsigned *q = wq[threadIdx.x >> 5];
   int qn = 0;  // queued entries (warp-uniform)
   const unsigned *__restrict__ hw = hits + (size_t)r * hit_words(cap_run);
-  for (long long base = warp * 32;; base += nwarps * 32) {
-    const bool more = base < nw;  // warp-uniform
-    if (more) {
-      const long long wt = base + lane;
-      const unsigned hm = hw[base >> 5];  // bits past nw are zero
-      const bool hit = (hm >> lane) & 1u;
-      if (hit) q[qn + __popc(hm & ((1u << lane) - 1u))] = (unsigned)wt;
-      qn += __popc(hm);
-      __syncwarp();
-    }
-    if (qn < 32 && (more || qn == 0)) {
-      if (more) continue;
-      break;
-    }
-    const int take = qn < 32 ? qn : 32;
-    const bool act = lane < take;
-    const long long w = act ? (long long)q[lane] : 0;
-    __syncwarp();
-    if (lane < qn - take) q[lane] = q[take + lane];  // the rest moves to the front (at most 31)
-    __syncwarp();
-    qn -= take;
-    {
+  auto collide = [&](bool act, long long w) {  // one entry per lane
     int nsel = 0;
     long long p = 0;
     MccWork e{};
@@ -557,9 +649,35 @@ __global__ void __launch_bounds__(256, ISKRA_MCC_COLLIDE_MIN_BLOCKS) k_mcc_colli
         }
       }
     }
+  };
+  if (ALL) {
+    for (long long base = warp * 32; base < nw; base += nwarps * 32) collide(base + lane < nw, base + lane);
+  } else {
+    for (long long base = warp * 32;; base += nwarps * 32) {
+      const bool more = base < nw;  // warp-uniform
+      if (more) {
+        const long long wt = base + lane;
+        const unsigned hm = hw[base >> 5];  // bits past nw are zero
+        const bool hit = (hm >> lane) & 1u;
+        if (hit) q[qn + __popc(hm & ((1u << lane) - 1u))] = (unsigned)wt;
+        qn += __popc(hm);
+        __syncwarp();
+      }
+      if (qn < 32 && (more || qn == 0)) {
+        if (more) continue;
+        break;
+      }
+      const int take = qn < 32 ? qn : 32;
+      const bool act = lane < take;
+      const long long w = act ? (long long)q[lane] : 0;
+      __syncwarp();
+      if (lane < qn - take) q[lane] = q[take + lane];  // the rest moves to the front (at most 31)
+      __syncwarp();
+      qn -= take;
+      collide(act, w);
+      if (!more && qn == 0) break;
+      if (!more) base -= nwarps * 32;  // more queued entries: another group without new tests
     }
-    if (!more && qn == 0) break;
-    if (!more) base -= nwarps * 32;  // more queued entries: another group without new tests
   }
 #pragma unroll
   for (int k = 0; k < kMaxProc; k++) {
@@ -569,6 +687,25 @@ __global__ void __launch_bounds__(256, ISKRA_MCC_COLLIDE_MIN_BLOCKS) k_mcc_colli
   }
   const int f = __reduce_or_sync(FULL, flags);
   if (lane == 0 && f) atomicOr(err, f);
+  if (ALL) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(end.ticket, 1ull) == (unsigned long long)gridDim.x - 1) {
+        __threadfence();
+        *end.ticket = 0ull;
+        *end.nwork = 0ull;
+        const long long ns = min((long long)__ldcg(&end.src->np_new), end.cap_src);
+        end.src->np = ns;
+        end.src->np_new = ns;
+        if (end.prod) {
+          const long long nq = min((long long)__ldcg(&end.prod->np_new), end.cap_prod);
+          end.prod->np = nq;
+          end.prod->np_new = nq;
+        }
+      }
+    }
+  }
 }
 
 __global__ void k_zero_u64(unsigned long long *p, int n, int stride) {
@@ -577,16 +714,22 @@ __global__ void k_zero_u64(unsigned long long *p, int n, int stride) {
 }
 
 // Appends reserve slots from np_new so that np (the loop bound of the running
-// kernel) stays fixed during the launch; np takes the new extent afterwards,
-// clamped to the capacity (failed appends already raised DERR_CAPACITY).
-__global__ void k_append_begin(SpeciesState *a, SpeciesState *b) {
+// kernels) stays fixed while a set runs; np takes the new extent when its
+// collision pass ends (MccEnd), clamped to the capacity (failed appends already
+// raised DERR_CAPACITY).  This opens a step's sets: cursors at np, an empty work
+// list and, when given, the step counter advanced.
+struct MccStates {
+  int ns;
+  SpeciesState *st[kMaxSpecies];
+};
+__global__ void k_mcc_begin(MccStates S, unsigned long long *nwork, unsigned long long *step) {
   pdl_wait();
-  a->np_new = a->np;
-  if (b) b->np_new = b->np;
-}
-__global__ void k_append_end(SpeciesState *st, long long cap) {
-  pdl_wait();
-  st->np = st->np_new > cap ? cap : st->np_new;
+  const int t = threadIdx.x;
+  if (t < S.ns) S.st[t]->np_new = S.st[t]->np;
+  if (t == 0) {
+    *nwork = 0ull;
+    if (step) *step += 1ull;
+  }
 }
 
 // Philox key of (seed, set)
@@ -637,8 +780,8 @@ static int mcc_params(Ctx *c, int mid, double dt, uint64_t seed, MccDev &M) {
   return ISKRA_OK;
 }
 
-// Both phases for R runs: src/prod device views (R each), keys (R, or
-// nullptr with key1 for a single context), per-run counters, node fields E
+// Both phases for R runs: src/prod device views (R each), keys (R), per-run
+// counters, node fields E
 // (R x nn), work list of cap_work entries with its counter.
 static int queue_mcc_phases(Ctx *c, int mid, const MccDev &M, int R, const SpeciesDev *src, const SpeciesDev *prod,
                             const uint2 *keys, unsigned long long *counts, const float2 *E, int nn, int select_blocks,
@@ -649,7 +792,7 @@ static int queue_mcc_phases(Ctx *c, int mid, const MccDev &M, int R, const Speci
   const size_t smem = M.staged ? (size_t)2 * ntab * sizeof(float) : 0;
   if (smem > 48 * 1024) {  // tables of up to kMaxTable nodes
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_test, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_collide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_collide<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
   const uint2 key1 = make_uint2(M.key0, M.key1);
   if (phases != kMccCollideOnly) {
@@ -659,36 +802,62 @@ static int queue_mcc_phases(Ctx *c, int mid, const MccDev &M, int R, const Speci
   }
   if (phases == kMccSelectAhead) return ISKRA_OK;
   unsigned *hits = reinterpret_cast<unsigned *>(work + (size_t)R * cap_work);
-  ISKRA_CUDA(c, launch_pdl(k_mcc_test, dim3(R == 1 ? c->num_sms * 8 : std::max(1, select_blocks * ISKRA_MCC_TEST_SCALE8 / 8), R), 256, smem, st, M, keys,
-                           E, nn, c->nx, d_step, (const MccWork *)work, (const unsigned long long *)nwork, cap_work,
+  ISKRA_CUDA(c, launch_pdl(k_mcc_test, dim3(std::max(1, select_blocks * ISKRA_MCC_TEST_SCALE8 / 8), R), 256, smem, st,
+                           M, keys, E, nn, c->nx, d_step, (const MccWork *)work, (const unsigned long long *)nwork, cap_work,
                            hits));
-  const int collide_blocks = R == 1 ? c->num_sms * 8 : std::max(1, select_blocks / ISKRA_MCC_COLLIDE_SPLIT);
-  ISKRA_CUDA(c, launch_pdl(k_mcc_collide, dim3(collide_blocks, R), 256, smem, st, src, prod, (int)(m->prod >= 0), M,
+  const int collide_blocks = std::max(1, select_blocks / ISKRA_MCC_COLLIDE_SPLIT);
+  ISKRA_CUDA(c, launch_pdl(k_mcc_collide<false>, dim3(collide_blocks, R), 256, smem, st, src, prod, (int)(m->prod >= 0), M,
                            keys, counts, E, nn, c->nx, d_step, (const MccWork *)work, (const unsigned long long *)nwork,
-                           cap_work, (const unsigned *)hits, err));
+                           cap_work, (const unsigned *)hits, err, MccEnd{}));
   return ISKRA_OK;
 }
 
-int launch_mcc(Ctx *c, int mid, double dt, uint64_t seed, const unsigned long long *d_step, uint64_t step_host) {
-  (void)step_host;
+// Before the sets of a step (or one set): k_mcc_begin.
+int launch_mcc_begin(Ctx *c, unsigned long long *step_ctr) {
+  if (!c->mcc_work) return set_err(c, ISKRA_EINVAL, "MCC work list missing");
+  MccStates S{};
+  S.ns = (int)c->species.size();
+  for (int i = 0; i < S.ns; i++) S.st[i] = c->species[i].dev.st;
+  ISKRA_CUDA(c, launch_pdl(k_mcc_begin, 1, 32, 0, c->stream, S, c->mcc_nwork, step_ctr));
+  return ISKRA_OK;
+}
+
+int launch_mcc(Ctx *c, int mid, double dt, uint64_t seed, const unsigned long long *d_step) {
   Mcc *m = c->mccs[mid];
   Species &s = c->species[m->src];
   MccDev M;
   int rc = mcc_params(c, mid, dt, seed, M);
   if (rc) return rc;
-  if (!c->mcc_work) return set_err(c, ISKRA_EINVAL, "MCC work list missing");
-  long long want = (s.cap + kSelChunk - 1) / kSelChunk;
-  long long maxb = (long long)c->num_sms * 4;
-  int blocks = (int)(want < maxb ? (want < 1 ? 1 : want) : maxb);
+  const size_t smem = M.staged ? (size_t)2 * m->off[m->N] * sizeof(float) : 0;
+  if (smem > 16 * 1024) {  // beside the kernels' static arrays
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_find<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_find<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_collide<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  }
+  const bool small = s.cap < (long long)c->num_sms * 4 * 2048;
+  const int chunk = small ? 512 : 2048;
+  const long long want = (s.cap + chunk - 1) / chunk, most = (long long)c->num_sms * ISKRA_MCC_FIND_PER_SM;
+  const int blocks = (int)std::max(1LL, std::min(want, most));
+  MccWork *work = (MccWork *)c->mcc_work;
+  ISKRA_CUDA(c, launch_pdl(small ? k_mcc_find<2> : k_mcc_find<8>, blocks, 256, smem, c->stream, s.dev, M,
+                           (const float2 *)c->E32, c->nx, d_step, work, c->mcc_nwork, c->mcc_work_cap, c->d_err));
+  MccEnd end{};
+  end.nwork = c->mcc_nwork;
+  end.ticket = c->mcc_nwork + 1;
+  end.src = s.dev.st;
+  end.cap_src = s.cap;
+  if (m->prod >= 0 && m->prod != m->src) {
+    end.prod = c->species[m->prod].dev.st;
+    end.cap_prod = c->species[m->prod].cap;
+  }
   const SpeciesDev *pd = m->prod >= 0 ? c->species[m->prod].dview : s.dview;
-  SpeciesState *pst = m->prod >= 0 ? c->species[m->prod].dev.st : nullptr;
-  ISKRA_CUDA(c, launch_pdl(k_append_begin, 1, 1, 0, c->stream, s.dev.st, pst));
-  rc = queue_mcc_phases(c, mid, M, 1, s.dview, pd, nullptr, nullptr, c->E32, c->nn, blocks, (MccWork *)c->mcc_work,
-                        c->mcc_nwork, c->mcc_work_cap, d_step, c->d_err, c->stream);
-  if (rc) return rc;
-  ISKRA_CUDA(c, launch_pdl(k_append_end, 1, 1, 0, c->stream, s.dev.st, s.cap));
-  if (m->prod >= 0)
-    ISKRA_CUDA(c, launch_pdl(k_append_end, 1, 1, 0, c->stream, c->species[m->prod].dev.st, c->species[m->prod].cap));
+  // a block takes 256 collisions a round; most of these blocks find none
+  const int cblocks = (int)std::max(1LL, std::min<long long>((s.cap + 2047) / 2048, c->num_sms * 3));
+  ISKRA_CUDA(c, launch_pdl(k_mcc_collide<true>, dim3(cblocks, 1), 256, smem, c->stream, (const SpeciesDev *)s.dview, pd,
+                           (int)(m->prod >= 0), M, (const uint2 *)nullptr, (unsigned long long *)nullptr,
+                           (const float2 *)c->E32, c->nn, c->nx, d_step, (const MccWork *)work,
+                           (const unsigned long long *)c->mcc_nwork, c->mcc_work_cap, (const unsigned *)nullptr,
+                           c->d_err, end));
   ISKRA_CUDA(c, cudaGetLastError());
   // appended particles are not in the deposit accumulators
   for (int sid : {m->src, m->prod}) {
@@ -739,7 +908,10 @@ int ensure_mcc_work(Ctx *c) {
   c->mcc_work = nullptr;
   c->mcc_work_cap = 0;
   ISKRA_CUDA(c, cudaMalloc(&c->mcc_work, mcc_work_bytes(1, (size_t)cap)));
-  if (!c->mcc_nwork) ISKRA_CUDA(c, cudaMalloc(&c->mcc_nwork, sizeof(unsigned long long)));
+  if (!c->mcc_nwork) {  // the list's counter, the collision pass's finished blocks
+    ISKRA_CUDA(c, cudaMalloc(&c->mcc_nwork, 2 * sizeof(unsigned long long)));
+    ISKRA_CUDA(c, cudaMemsetAsync(c->mcc_nwork, 0, 2 * sizeof(unsigned long long), c->stream));
+  }
   c->mcc_work_cap = (unsigned long long)cap;
   return ISKRA_OK;
 }
@@ -888,7 +1060,9 @@ int iskra_mcc_perform(iskra_ctx *h, int mid, double dt, uint64_t seed, uint64_t 
   ISKRA_CUDA(c, cudaMemcpyAsync(c->d_step, &st, sizeof(st), cudaMemcpyHostToDevice, c->stream));
   ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
   c->d_step_known = ~0ull;
-  return launch_mcc(c, mid, dt, seed, c->d_step, step);
+  int rc = launch_mcc_begin(c, nullptr);
+  if (rc) return rc;
+  return launch_mcc(c, mid, dt, seed, c->d_step);
 }
 
 int iskra_mcc_counts(iskra_ctx *h, int mid, int64_t *counts) {

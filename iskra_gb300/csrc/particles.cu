@@ -585,22 +585,6 @@ int launch_sort(Ctx *c, int sid) {
   return ISKRA_OK;
 }
 
-// Appends a warp's n <= 32 buffered work-list entries to its run's list
-// (counter cnt, segment seg of cap entries).
-__device__ __forceinline__ void flush_entries(const MccWork *buf, int n, unsigned long long *cnt,
-                                              MccWork *__restrict__ seg, unsigned long long cap, int &flags) {
-  const int lane = threadIdx.x & 31;
-  __syncwarp();  // the entries are in buf
-  unsigned long long at = 0;
-  if (lane == 0) at = atomicAdd(cnt, (unsigned long long)n);
-  at = __shfl_sync(0xffffffffu, at, 0) + (unsigned)lane;
-  if (lane < n) {
-    if (at < cap) seg[at] = buf[lane];
-    else flags |= DERR_CAPACITY;
-  }
-  __syncwarp();  // buf may be written again
-}
-
 // ---------------------------------------------------------------------------
 // ensemble push: run r = blockIdx.y; every block of a run stages the run's
 // whole E grid (cx*cy <= kEnsWinCells cells), pushes a grid-stride share of the

@@ -60,10 +60,10 @@ static int queue_step(Ctx *c, double dt, uint64_t seed, double rtol, bool blocki
   int rc = launch_step_sources(c, dt, seed);  // sample! of every source (ParticleInCell.jl:104-106)
   if (rc) return rc;
   if (!c->mccs.empty()) {  // MCC keys read the step counter first
-    ISKRA_CUDA(c, launch_pdl(k_step_begin, 1, 1, 0, c->stream, c->d_step));
-    ISKRA_CUDA(c, cudaGetLastError());
+    rc = launch_mcc_begin(c, c->d_step);
+    if (rc) return rc;
     for (int m = 0; m < (int)c->mccs.size(); m++) {
-      rc = launch_mcc(c, m, dt, seed, c->d_step, 0);
+      rc = launch_mcc(c, m, dt, seed, c->d_step);
       if (rc) return rc;
     }
     rc = launch_step_dsmc(c, dt, seed);  // the DSMC sets, after the MCC sets (interactions)
