@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "multigrid.cuh"
 
 namespace iskra {
 
@@ -2370,8 +2371,8 @@ int poisson_solve_graph(Ctx *c, double rtol) {
 
 // ---- a step's field part in one block ------------------------------------------
 // On grids of up to kFieldBlockNodes nodes the circuit, the density pass, the warm
-// start, the driven rows, the residuals and corrections, and E run as phases of
-// one 512-thread block with ϕ, the right-hand side, the residual and the spectrum
+// start, the driven rows, the residuals and corrections (or the whole multigrid
+// CG, up to ~1200 nodes), and E run as phases of one 512-thread block with ϕ, the right-hand side, the residual and the spectrum
 // in shared memory: at these sizes each of the 9 (double-float) to 18 (FP64,
 // singular) launches they took costs 3-10 us of launch and memory latency for
 // well under a microsecond of work.  The phases are the multi-launch path's own
@@ -2408,17 +2409,20 @@ struct FieldBlock {
   FftPlan F;
   CrArgs C;
   EOut eo;
+  MgBlock mg;
+  double idx2, idx1, idy2, idy1;  // 1/(2Δx), ... of the CG path's FP64 field
   int *err, *notconv;
 };
-constexpr int kFieldThreads = 512;
-// MODE: 0 ny = 2, 1 ny another power of two, 2 any other ny
+constexpr int kFieldThreads = 512, kFieldMgIterations = 10000;
+// MODE: 0 ny = 2, 1 ny another power of two, 2 any other ny (direct solves); 3
+// multigrid CG (FP64 state)
 template <bool DF, int MODE>
 __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
   extern __shared__ __align__(16) unsigned char field_smem[];
   __shared__ double red[2 * kFieldThreads];
   __shared__ RowClass cls_sh[kSmemClasses];
   const int tid = threadIdx.x, T = kFieldThreads, nn = P.nn, nx = P.op.nx, ny = P.op.ny;
-  constexpr bool TWO = MODE == 0, ODD = MODE == 2;
+  constexpr bool TWO = MODE == 0, ODD = MODE == 2, MG = MODE == 3;
   // shared memory: ϕ, b or ρ (8 B a node), residual, spectrum, then the
   // transform's columns or the lines of the cyclic reduction
   float2 *xd = reinterpret_cast<float2 *>(field_smem), *bd = xd + nn;
@@ -2428,8 +2432,18 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
   float2 *fbuf = spec + (TWO ? 0 : (size_t)nx * P.C.K);
   // coefficients of the lines: written by the operator build, read before the wait
   const size_t fft_n = TWO ? 0 : (ODD ? 2 : 1) * (size_t)((nx + 1) / 2) * (P.F.N + 1) + P.F.N / 2 + (ODD ? P.F.odd : 0);
-  const CrShared cr = cr_shared(P.C, reinterpret_cast<float *>(fbuf + fft_n));
-  cr_stage(P.C, cr, 0, P.C.K);
+  CrShared cr{};
+  // multigrid CG: r, p, S p after ϕ and ρ, then the levels
+  double *r64 = rho64 + nn, *p64 = r64 + nn, *ap64 = p64 + nn;
+  float *lev = reinterpret_cast<float *>(ap64 + nn);
+  const float *ci = P.mg.cinv;
+  if (MG) {
+    const float *staged = mg_bottom_stage(lev, P.mg.lv, 0, P.mg.L, P.mg.cinv, P.mg.cinv_shared);
+    if (P.mg.cinv_shared) ci = staged;
+  } else {
+    cr = cr_shared(P.C, reinterpret_cast<float *>(fbuf + fft_n));
+    cr_stage(P.C, cr, 0, P.C.K);
+  }
   const RowClass *CT = stage_classes(P.op, cls_sh);
   PoissonScal *sc = P.sc;
   pdl_wait();
@@ -2504,7 +2518,79 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
     if (tid == 0) sc->lambda = lam;
   }
   double rhs2 = 0;
-  for (int s = 0;; s++) {
+  if (MG) {
+    // flexible PCG as in k_pcg_ap, k_pcg_update and the cycle, the whole solve
+    // without a launch or a host check
+    double v2[2] = {0, 0}, t2[2];
+    for (int k = tid; k < nn; k += T)
+      residual_node<true>(P.op, CT, x64, rho, P.nie, 0.0, 0, k, k % nx, k / nx, r64, v2[0], v2[1]);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // the staged levels (a barrier follows)
+    block_sums<2>(v2, red, t2);
+    rhs2 = t2[1];
+    double res2 = t2[0], rz = 0, alpha = 0;
+    int it = 0;
+    bool done = (rhs2 > 0 && res2 <= P.rtol2 * rhs2) || res2 == 0.0;
+    const MgSh q = mg_sh(lev, P.mg.lv[0]);
+    while (!done && it < kFieldMgIterations) {
+      for (int k = tid; k < nn; k += T) q.b[k] = (float)r64[k];
+      __syncthreads();
+      mg_bottom_cycle(lev, P.mg.lv, 0, P.mg.L, ci);
+      v2[0] = v2[1] = 0;
+      for (int k = tid; k < nn; k += T) {
+        const double z = (double)q.x[k];
+        v2[0] = fma(z, r64[k], v2[0]);
+        if (it) v2[1] = fma(z, ap64[k], v2[1]);
+      }
+      block_sums<2>(v2, red, t2);
+      const double beta = it && rz != 0 ? -alpha * t2[1] / rz : 0.0;
+      rz = t2[0];
+      for (int k = tid; k < nn; k += T) {
+        double p = (double)q.x[k];
+        if (beta != 0) p = fma(beta, p64[k], p);
+        p64[k] = p;
+      }
+      __syncthreads();
+      double v1[1] = {0}, t1[1];
+      for (int k = tid; k < nn; k += T) {
+        const RowClass &C = CT[P.op.cls[k] & kClassMask];
+        int w, e, so, no;
+        nbr(k, nx, ny, w, e, so, no);
+        double a = C.s0 * p64[k];
+        a = fma(C.sW, p64[w], a);
+        a = fma(C.sE, p64[e], a);
+        a = fma(C.sS, p64[so], a);
+        a = fma(C.sN, p64[no], a);
+        ap64[k] = a;
+        v1[0] = fma(p64[k], a, v1[0]);
+      }
+      block_sums<1>(v1, red, t1);
+      alpha = t1[0] != 0 ? rz / t1[0] : 0.0;
+      v1[0] = 0;
+      for (int k = tid; k < nn; k += T) {
+        const unsigned ck = P.op.cls[k];
+        if (ck & kFixedBit) continue;
+        x64[k] = fma(alpha, p64[k], x64[k]);
+        const double rr = fma(-alpha, ap64[k], r64[k]);
+        r64[k] = rr;
+        const double res = rr * CT[ck & kClassMask].inv_d;
+        v1[0] = fma(res, res, v1[0]);
+      }
+      block_sums<1>(v1, red, t1);
+      res2 = t1[0];
+      it++;
+      done = (rhs2 > 0 && res2 <= P.rtol2 * rhs2) || res2 == 0.0;
+    }
+    if (tid == 0) {
+      sc->rhs2 = rhs2;
+      sc->res2 = res2;
+      sc->relres = rhs2 > 0 ? sqrt(res2 / rhs2) : sqrt(res2);
+      sc->iters = it;
+      sc->done = done;
+      sc->e_pending = 0;
+      if (!done) atomicOr(P.notconv, DERR_NOTCONV);
+    }
+  }
+  for (int s = 0; !MG; s++) {
     double a2 = 0, b2 = 0;
     if (DF) {
       if (s == 0)
@@ -2569,7 +2655,14 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
   // E, and ϕ to memory
   for (int k = tid; k < nn; k += T) {
     const int j = k / nx, i = k - j * nx;
-    if (DF) {
+    if (MG) {  // in FP64 as k_efield
+      const double ex = i == 0 ? (x64[k] - x64[k + 1]) * P.idx1
+                               : i == nx - 1 ? (x64[k - 1] - x64[k]) * P.idx1 : (x64[k - 1] - x64[k + 1]) * P.idx2;
+      const double ey = j == 0 ? (x64[k] - x64[k + nx]) * P.idy1
+                               : j == ny - 1 ? (x64[k - nx] - x64[k]) * P.idy1 : (x64[k - nx] - x64[k + nx]) * P.idy2;
+      P.eo.E32[k] = make_float2((float)ex, (float)ey);
+      P.x[k] = x64[k];
+    } else if (DF) {
       const int w = i > 0 ? k - 1 : k + nx - 1, e = i < nx - 1 ? k + 1 : k - nx + 1;
       const int so = j > 0 ? k - nx : k + nx * (ny - 1), no = j < ny - 1 ? k + nx : k - nx * (ny - 1);
       efield_df5(xd[k], xd[w], xd[e], xd[so], xd[no], k, i, j, nx, ny, P.eo);
@@ -2607,7 +2700,12 @@ static size_t field_block_bytes(const Poisson *P) {
 
 bool poisson_one_block(Ctx *c) {
   const Poisson *P = c->ps;
-  return P && !P->dirty && P->separable && P->nn <= (P->N == 2 ? kFieldBlockNodes1D : kFieldBlockNodes) &&
+  if (!P || P->dirty) return false;
+  if (!P->separable) {  // multigrid CG without a learned warm start, levels and vectors in shared memory
+    MgBlock v;
+    return mg_block_view(P->mg, &v) && !lws_active(c) && 40 * (size_t)P->nn + v.bytes <= kFieldSmem;
+  }
+  return P->separable && P->nn <= (P->N == 2 ? kFieldBlockNodes1D : kFieldBlockNodes) &&
          field_block_bytes(P) <= kFieldSmem;
 }
 
@@ -2649,11 +2747,23 @@ int launch_field_block(Ctx *c, double rtol) {
   B.rho_fixed = P->rho_fixed;
   B.sweeps = std::min(8, graph_sweeps(P, rtol) + 2);  // (sweeps not needed cost nothing here)
   B.nn = P->nn;
-  B.F = FftPlan{P->N, P->log2p, P->odd, P->tw, P->tw + P->N / 2};
-  B.C = cr_args(P, P->K);
   B.eo = eout(c, true);
   B.err = c->d_err;
   B.notconv = c->d_err;
+  if (!P->separable) {
+    mg_block_view(P->mg, &B.mg);
+    B.idx2 = 1.0 / (2 * c->g.dx);
+    B.idx1 = 1.0 / c->g.dx;
+    B.idy2 = 1.0 / (2 * c->g.dy);
+    B.idy1 = 1.0 / c->g.dy;
+    ISKRA_CUDA(c, cudaFuncSetAttribute(k_field_block<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kFieldSmem));
+    ISKRA_CUDA(c, launch_pdl(k_field_block<false, 3>, 1, kFieldThreads, 40 * (size_t)P->nn + B.mg.bytes, c->stream, B));
+    c->e_from_phi = true;
+    return ISKRA_OK;
+  }
+  B.F = FftPlan{P->N, P->log2p, P->odd, P->tw, P->tw + P->N / 2};
+  B.C = cr_args(P, P->K);
   const int mode = P->N == 2 ? 0 : P->odd > 1 ? 2 : 1;
   auto kern = df ? (mode == 0 ? k_field_block<true, 0> : mode == 1 ? k_field_block<true, 1> : k_field_block<true, 2>)
                  : (mode == 0 ? k_field_block<false, 0> : mode == 1 ? k_field_block<false, 1> : k_field_block<false, 2>);

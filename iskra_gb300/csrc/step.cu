@@ -123,9 +123,10 @@ static int update_sort_periods(Ctx *c, double dt) {
 // costs ~0.1 ns more than a tile's (64 M sampled particles on 1024 x 1024
 // nodes: 6.8 ms per step until the first periodic sort, up to 64 steps
 // later, against 0.9 ms sorted) and a sort costs ~0.045 ns per particle of
-// the species and its launches (~20 us), so a tail of at least an eighth of
-// the capacity pays within four steps; a smaller one waits for the period.
-static bool tail_wants_sort(const Species &s) { return s.tail >= 65536 && 8 * s.tail >= s.cap; }
+// the species and its launches (~20 us; the tail push of 20 k particles on 10 x
+// 10 nodes takes 13 us longer than the tiles'), so a tail of at least an eighth
+// of the capacity pays within a few steps; a smaller one waits for the period.
+static bool tail_wants_sort(const Species &s) { return s.tail >= 4096 && 8 * s.tail >= s.cap; }
 
 // Captures the work queued by fn() on the context stream into an executable
 // graph and counts its kernel nodes.
@@ -289,7 +290,8 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
       rc = launch_sort(c, s);
       if (rc) return rc;
     }
-  if (!poisson_separable(c)) {
+  const bool direct = poisson_separable(c);
+  if (!direct && !poisson_one_block(c)) {
     // eager path: CG needs host-side convergence checks
     for (int n = 0; n < nsteps; n++) {
       rc = queue_step(c, dt, seed, rtol, true);
@@ -349,7 +351,8 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
       }
     }
   }
-  return ISKRA_OK;
+  // (steps of CG operators report their errors before they return)
+  return direct ? ISKRA_OK : collect_device_errors(c);
 }
 
 // Sort-cadence autotuner: runs `trial` steps of the caller's own simulation

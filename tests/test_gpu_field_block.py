@@ -18,7 +18,10 @@ pytestmark = pytest.mark.gpu
                                              ("slab", 33, 7, 1e-9), ("slab", 64, 24, 1e-9), ("slab", 257, 2, 1e-10),
                                              ("slab", 40, 16, 1e-10), ("periodic", 128, 2, 1e-9),
                                              ("periodic", 32, 32, 1e-10), ("periodic", 21, 9, 1e-9),
-                                             ("neumann_gauss", 201, 2, 1e-9), ("driven", 129, 2, 1e-9)])
+                                             ("neumann_gauss", 201, 2, 1e-9), ("driven", 129, 2, 1e-9),
+                                             ("open_box", 10, 10, 1e-9), ("open_box", 20, 20, 1e-10),
+                                             ("open_box", 21, 20, 1e-9), ("open_box", 34, 34, 1e-10),
+                                             ("open_box", 300, 3, 1e-9)])
 def test_step_field_matches_the_single_stages(lib, kind, nx, ny, rtol):
     dx, n = 1e-4, 4000
     rng = np.random.default_rng(nx + 7 * ny)

@@ -45,10 +45,11 @@ def test_split_tiles_match_the_oracle(orc, lib, nx, ny, n):
     ctx.close()
 
 
-@pytest.mark.parametrize("n,cap", [(65535, 70000), (65536, 70000), (65536, 8 * 65536), (65536, 8 * 65536 + 1)])
+@pytest.mark.parametrize("n,cap", [(4095, 5000), (4096, 5000), (65536, 70000), (65536, 8 * 65536),
+                                   (65536, 8 * 65536 + 1)])
 def test_steps_after_a_source_fill_do_not_depend_on_its_sort(lib, n, cap):
     """A species filled by a source is sorted once before its first step when
-    the fill is large (at least 65536 particles and an eighth of the
+    the fill is large (at least 4096 particles and an eighth of the
     capacity): same fields, bit for bit, as with an explicit sort or none."""
     out = []
     for how in ("auto", "sorted", "never"):
