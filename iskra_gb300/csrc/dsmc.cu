@@ -42,6 +42,7 @@ struct DsmcArgs {
   const float *tab;
   int ntab;
   double sgmax, dt, inv_area;   // 1 / (Δx Δy)
+  double denom;                 // Pab + (Wb/Wa) Pba of the weights
   int nn;
   bool same;                    // source and target are one species
   double *remaining;
@@ -103,6 +104,80 @@ __global__ void k_dsmc_scatter(SpeciesDev s, int nx, const int *__restrict__ sta
   }
 }
 
+// The same three passes for small sets, one block per species with the counts in
+// shared memory: count, scan, scatter.  On the 20 x 20-cell problem of 2 x 5000
+// particles the two memsets and six launches took 20 us of the 53 us a perform!,
+// this one 6.
+constexpr int kBucketCells = 8192;        // counts of one block (32 KB)
+constexpr long long kBucketSlots = 32768;  // slots one block walks twice
+struct DsmcBuckets {
+  SpeciesDev s[2];
+  int *cnt[2];
+  unsigned *idx[2];
+};
+__global__ void __launch_bounds__(1024) k_dsmc_bucket(DsmcBuckets B, int nx, int n) {
+  extern __shared__ int bucket[];  // n counts, then cursors
+  __shared__ int part[32];
+  const int q = blockIdx.x, t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  for (int k = t; k < n; k += 1024) bucket[k] = 0;
+  pdl_wait();
+  const SpeciesDev &s = B.s[q];
+  const int np = (int)s.st->np;
+  const float2 *zc = pick(s.zc[0], s.zc[1], s.st->cur);
+  __syncthreads();
+  constexpr int U = 8;  // slots per thread with their loads in flight together
+  for (int p0 = 0; p0 < np; p0 += 1024 * U) {
+    int cell[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int p = p0 + 1024 * u + t;
+      cell[u] = p < np ? __float_as_int(zc[p].y) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (cell[u] >= 0) atomicAdd(&bucket[(cell[u] & 0xffff) + nx * (cell[u] >> 16)], 1);
+  }
+  __syncthreads();
+  // exclusive scan: a run of cells per thread, then over the threads
+  const int per = (n + 1023) / 1024, lo = min(n, t * per), hi = min(n, lo + per);
+  int sum = 0;
+  for (int k = lo; k < hi; k++) sum += bucket[k];
+  int x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) part[wid] = x;
+  __syncthreads();
+  int before = 0, total = 0;
+  for (int w = 0; w < 32; w++) {
+    if (w < wid) before += part[w];
+    total += part[w];
+  }
+  int run = before + x - sum;
+  for (int k = lo; k < hi; k++) {
+    const int c = bucket[k];
+    bucket[k] = run;
+    B.cnt[q][k] = run;
+    run += c;
+  }
+  if (t == 0) B.cnt[q][n] = total;
+  __syncthreads();
+  for (int p0 = 0; p0 < np; p0 += 1024 * U) {
+    int cell[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int p = p0 + 1024 * u + t;
+      cell[u] = p < np ? __float_as_int(zc[p].y) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (cell[u] >= 0)
+        B.idx[q][atomicAdd(&bucket[(cell[u] & 0xffff) + nx * (cell[u] >> 16)], 1)] = (unsigned)(p0 + 1024 * u + t);
+  }
+}
+
 // a cell's slots ordered by particle identifier (insertion sort: cells hold
 // few particles), so the picks depend neither on the order the scatter wrote
 // them in nor on where the sort left the particles in memory
@@ -121,75 +196,103 @@ __device__ __forceinline__ void set_vel(const SpeciesDev &s, unsigned p, float3 
   zc[p] = make_float2(v.z, zc[p].y);
 }
 
-// The pairs of one cell in order (dsmc.jl:108-133), by the whole warp:
+// The pairs of one cell in order (dsmc.jl:108-133), by a block of T threads:
 // ncol pairs from the id-ordered lists (positions ra < Na, rb < Nb), pair c
 // drawing its own random numbers (Philox keyed by (seed, set, step, cell,
 // c)), accepted with probability σ(g) g / σgmax and scattered by
 // perform!(::ElasticCollision) (dsmc.jl:31-84, vss_inv = 1: an isotropic
-// direction for the relative velocity in the CM frame).  The 32 lanes test
-// 32 consecutive pairs against the current velocities; the first accepted
-// one collides (its lane writes the velocities) and the test resumes after
+// direction for the relative velocity in the CM frame).  The threads test U T
+// consecutive pairs against the current velocities; the first accepted
+// one collides (its thread writes the velocities) and the test resumes after
 // it, so the outcome is that of testing the pairs one by one (acceptance is
 // rare: the 05_dsmc problem accepts ~1 pair in 1500).  A pair of one species
 // draws its second particle among the other Nb - 1 (the reference redraws
 // until they differ, :112-114: the same distribution).  get/set reach the
-// velocities of the r-th particle of each list (shared or global memory).
-// Returns the accepted collisions (on every lane).
-template <class GA, class SA, class GB, class SB>
-__device__ unsigned dsmc_pairs(const DsmcArgs &A, int cell, unsigned long long step, long long ncol, int Na, int Nb,
-                               int lane, GA get_a, SA set_a, GB get_b, SB set_b) {
+// velocities of the r-th particle of each list (shared or global memory).  gt,
+// st: the cross-section table (shared memory when it fits).  first: shared
+// memory.  Returns the accepted collisions (in every thread).
+// A round is one chain of dependent latencies and the cell with the most pairs
+// (Na Nb, several times the mean) sets the pass's length: with one warp and one
+// pair a lane the 20 x 20-cell problem took 26 us, with four pairs a lane still
+// 26; 128 threads of two pairs each 17.
+template <int T, class GA, class SA, class GB, class SB>
+__device__ __forceinline__ unsigned dsmc_pairs(const DsmcArgs &A, const float *gt, const float *st, int cell,
+                                               unsigned long long step, long long ncol, int Na, int Nb, int *first,
+                                               GA get_a, SA set_a, GB get_b, SB set_b) {
+  constexpr int U = 2, kNone = 0x7fffffff;
   const unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31;
   const double Wa = A.w[0], Wb = A.w[1];
   const float ma = (float)A.m[0], mb = (float)A.m[1];
   const float mr1 = ma / (ma + mb), mr2 = mb / (ma + mb);
   const float sgmax = (float)A.sgmax;
-  const float *gt = A.tab, *st = A.tab + A.ntab;
   const uint32_t k1 = A.k1 ^ (uint32_t)(step >> 32);
   unsigned accepted = 0;
   long long c = 0;
   while (c < ncol) {
-    const long long my = c + lane;
-    bool acc = false;
-    int ra = 0, rb = 0;
-    U4 r0{0, 0, 0, 0}, r1{0, 0, 0, 0};
-    float3 va{0, 0, 0}, vb{0, 0, 0};
-    float g = 0.f;
-    if (my < ncol) {
-      r0 = philox4x32_10(U4{(uint32_t)my, (uint32_t)cell, (uint32_t)step, A.set}, A.k0, k1);
-      r1 = philox4x32_10(U4{(uint32_t)my, (uint32_t)cell, (uint32_t)step, A.set | 0x80000000u}, A.k0, k1);
-      ra = min(Na - 1, (int)(u01(r0.x) * Na));
-      if (A.same) rb = (ra + 1 + min(Nb - 2, (int)(u01(r0.y) * (Nb - 1)))) % Nb;
-      else rb = min(Nb - 1, (int)(u01(r0.y) * Nb));
-      va = get_a(ra);
-      vb = get_b(rb);
-      const float gx = va.x - vb.x, gy = va.y - vb.y, gz = va.z - vb.z;
-      g = sqrtf(gx * gx + gy * gy + gz * gz);
-      const float P = sigma_at(gt, st, A.ntab, g, 0, 0.f, 0.f) * g / sgmax;
-      acc = !(P < u01(r0.z));
+    bool acc[U];
+    int ra[U], rb[U];
+    float uz[U], uw[U];
+    float3 va[U], vb[U];
+    float g[U];
+    if (tid == 0) *first = kNone;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long my = c + T * u + tid;
+      acc[u] = false;
+      ra[u] = rb[u] = 0;
+      uz[u] = uw[u] = g[u] = 0.f;
+      va[u] = vb[u] = float3{0, 0, 0};
+      if (my < ncol) {
+        const U4 r0 = philox4x32_10(U4{(uint32_t)my, (uint32_t)cell, (uint32_t)step, A.set}, A.k0, k1);
+        ra[u] = min(Na - 1, (int)(u01(r0.x) * Na));
+        if (A.same) rb[u] = (ra[u] + 1 + min(Nb - 2, (int)(u01(r0.y) * (Nb - 1)))) % Nb;
+        else rb[u] = min(Nb - 1, (int)(u01(r0.y) * Nb));
+        uz[u] = u01(r0.z);
+        uw[u] = u01(r0.w);
+        va[u] = get_a(ra[u]);
+        vb[u] = get_b(rb[u]);
+        const float gx = va[u].x - vb[u].x, gy = va[u].y - vb[u].y, gz = va[u].z - vb[u].z;
+        g[u] = sqrtf(gx * gx + gy * gy + gz * gz);
+        const float P = sigma_at(gt, st, A.ntab, g[u], 0, 0.f, 0.f) * g[u] / sgmax;
+        acc[u] = !(P < uz[u]);
+      }
     }
-    const unsigned m = __ballot_sync(FULL, acc);
-    if (m == 0u) {
-      c += 32;
+    __syncthreads();  // *first is set; every velocity of the round has been read
+#pragma unroll
+    for (int u = U - 1; u >= 0; u--) {
+      const unsigned m = __ballot_sync(FULL, acc[u]);
+      if (m && lane == __ffs(m) - 1) atomicMin(first, T * u + tid);
+    }
+    __syncthreads();
+    const int f = *first;
+    if (f == kNone) {
+      c += T * U;
+      __syncthreads();  // (read before the next round sets it)
       continue;
     }
-    const int f = __ffs(m) - 1;
-    if (lane == f) {
-      const float vcx = mr1 * va.x + mr2 * vb.x, vcy = mr1 * va.y + mr2 * vb.y, vcz = mr1 * va.z + mr2 * vb.z;
-      const float B = 2.0f * u01(r0.w) - 1.0f;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (T * u + tid != f) continue;
+      const long long my = c + f;
+      const U4 r1 = philox4x32_10(U4{(uint32_t)my, (uint32_t)cell, (uint32_t)step, A.set | 0x80000000u}, A.k0, k1);
+      const float3 a = va[u], b = vb[u];
+      const float vcx = mr1 * a.x + mr2 * b.x, vcy = mr1 * a.y + mr2 * b.y, vcz = mr1 * a.z + mr2 * b.z;
+      const float B = 2.0f * uw[u] - 1.0f;
       const float Aa = sqrtf(fmaxf(1.0f - B * B, 0.0f));
       float sC, cC;
       sincospif(2.0f * u01(r1.x), &sC, &cC);
-      const float rx = g * B, ry = g * Aa * cC, rz = g * Aa * sC;
+      const float rx = g[u] * B, ry = g[u] * Aa * cC, rz = g[u] * Aa * sC;
       if (A.w[0] == A.w[1]) {
-        set_a(ra, make_float3(vcx + mr2 * rx, vcy + mr2 * ry, vcz + mr2 * rz));
-        set_b(rb, make_float3(vcx - mr1 * rx, vcy - mr1 * ry, vcz - mr1 * rz));
+        set_a(ra[u], make_float3(vcx + mr2 * rx, vcy + mr2 * ry, vcz + mr2 * rz));
+        set_b(rb[u], make_float3(vcx - mr1 * rx, vcy - mr1 * ry, vcz - mr1 * rz));
       } else {  // unequal weights (dsmc.jl:72-83)
-        const float u = u01(r1.y);
-        if ((float)(Wb / Wa) > u) set_a(ra, make_float3(vcx + mr2 * rx, vcy + mr2 * ry, vcz + mr2 * rz));
-        if ((float)(Wa / Wb) > u) set_b(rb, make_float3(vcx - mr2 * rx, vcy - mr2 * ry, vcz - mr2 * rz));
+        const float w = u01(r1.y);
+        if ((float)(Wb / Wa) > w) set_a(ra[u], make_float3(vcx + mr2 * rx, vcy + mr2 * ry, vcz + mr2 * rz));
+        if ((float)(Wa / Wb) > w) set_b(rb[u], make_float3(vcx - mr2 * rx, vcy - mr2 * ry, vcz - mr2 * rz));
       }
     }
-    __syncwarp();
+    __syncthreads();
     accepted++;
     c += f + 1;
   }
@@ -198,48 +301,51 @@ __device__ unsigned dsmc_pairs(const DsmcArgs &A, int cell, unsigned long long s
 
 // cells whose lists fit are staged in shared memory: the pair loop then
 // waits on shared-memory loads instead of dependent global ones
-constexpr int kDsmcStage = 512;
+constexpr int kDsmcStage = 512, kDsmcTab = 64;
 struct __align__(16) DsmcShared {  // 16-byte aligned: tid is read as uint4
   float3 va[kDsmcStage], vb[kDsmcStage];      // velocities, id order
   unsigned sa[kDsmcStage], sb[kDsmcStage];    // slots, id order
   unsigned tslot[kDsmcStage];                 // a list as scattered
   uint32_t tid[kDsmcStage];                   // its identifiers
+  float tab[2 * kDsmcTab];                    // a small cross-section table
 };
 
 // the list l[0..n) ordered by identifier into out (ids are unique: each
-// element's rank is the number of smaller ids); the warp's lanes share it
-__device__ __forceinline__ void warp_rank_sort(const unsigned *__restrict__ l, int n, const uint32_t *__restrict__ id,
-                                               DsmcShared &sh, unsigned *out, int lane) {
-  for (int e = lane; e < n; e += 32) {
+// element's rank is the number of smaller ids); the block's T threads share it
+template <int T>
+__device__ __forceinline__ void rank_sort(const unsigned *__restrict__ l, int n, const uint32_t *__restrict__ id,
+                                               DsmcShared &sh, unsigned *out) {
+  for (int e = threadIdx.x; e < n; e += T) {
     sh.tslot[e] = l[e];
     sh.tid[e] = id[l[e]];
   }
-  __syncwarp();
-  for (int e = lane; e < n; e += 32) {
+  __syncthreads();
+  for (int e = threadIdx.x; e < n; e += T) {
     const uint32_t key = sh.tid[e];
     int r = 0;
     for (int q = 0; q < n; q++) r += sh.tid[q] < key;
     out[r] = sh.tslot[e];
   }
-  __syncwarp();
+  __syncthreads();
 }
 
-// The same order for a list of any length, into global memory: each lane
-// ranks one element of every 32 against all ids, staged through shared
-// memory kDsmcStage at a time (n²/32 shared-memory compares per lane, no
+// The same order for a list of any length, into global memory: each thread
+// ranks one element of every T against all ids, staged through shared
+// memory kDsmcStage at a time (n²/T shared-memory compares per thread, no
 // dependent global loads).
-__device__ void warp_rank_sort_long(const unsigned *__restrict__ l, int n, const uint32_t *__restrict__ id,
-                                    DsmcShared &sh, unsigned *__restrict__ out, int lane) {
-  for (int g = 0; g < n; g += 32) {
-    const int e = g + lane;
+template <int T>
+__device__ void rank_sort_long(const unsigned *__restrict__ l, int n, const uint32_t *__restrict__ id,
+                               DsmcShared &sh, unsigned *__restrict__ out) {
+  for (int g = 0; g < n; g += T) {
+    const int e = g + threadIdx.x;
     const unsigned slot = e < n ? l[e] : 0u;
     const uint32_t key = e < n ? id[slot] : 0u;
     int r = 0;
     for (int c0 = 0; c0 < n; c0 += kDsmcStage) {
       const int m = min(kDsmcStage, n - c0);
-      __syncwarp();
-      for (int q = lane; q < m; q += 32) sh.tid[q] = id[l[c0 + q]];
-      __syncwarp();
+      __syncthreads();
+      for (int q = threadIdx.x; q < m; q += T) sh.tid[q] = id[l[c0 + q]];
+      __syncthreads();
       int q = 0;
       for (; q + 4 <= m; q += 4) {
         const uint4 t = *reinterpret_cast<const uint4 *>(sh.tid + q);
@@ -249,15 +355,26 @@ __device__ void warp_rank_sort_long(const unsigned *__restrict__ l, int n, const
     }
     if (e < n) out[r] = slot;
   }
-  __syncwarp();
+  __syncthreads();
 }
 
-// PIC.perform!(dsmc, ...) for one cell (dsmc.jl:103-134), a warp per cell.
+// PIC.perform!(dsmc, ...) for one cell (dsmc.jl:103-134), a block of T threads
+// per cell: 128 where the cells are fewer than the chip's resident blocks (the
+// longest cell sets the time), 32 on larger grids (their number does).
 // Cells are numbered like nodes (i0 + nx j0; the reference's (i0+1, j0+1)).
-__global__ void __launch_bounds__(32) k_dsmc_cells(DsmcArgs A) {
-  pdl_wait();
+template <int T>
+__global__ void __launch_bounds__(T) k_dsmc_cells(DsmcArgs A) {
   __shared__ DsmcShared sh;
+  __shared__ int first;
   const int k = blockIdx.x, lane = threadIdx.x;
+  const float *gt = A.tab, *st = A.tab + A.ntab;
+  if (A.ntab <= kDsmcTab) {  // (written by the set's creation, read before the wait)
+    for (int t = lane; t < 2 * A.ntab; t += T) sh.tab[t] = A.tab[t];
+    __syncthreads();
+    gt = sh.tab;
+    st = sh.tab + A.ntab;
+  }
+  pdl_wait();
   const int sa0 = A.cnt[0][k], Na = A.cnt[0][k + 1] - sa0;
   const int sb0 = A.cnt[1][k], Nb = A.cnt[1][k + 1] - sb0;
   if (Na < 2 || Nb < 2) {
@@ -266,13 +383,9 @@ __global__ void __launch_bounds__(32) k_dsmc_cells(DsmcArgs A) {
   }
   // Nc = na Nb Δt σgmax / (Pab + (Wb/Wa) Pba), doubled for two species,
   // plus the remainder of the last step (dsmc.jl:94-117)
-  const double Wa = A.w[0], Wb = A.w[1];
-  double Pab = 1.0, Pba = 1.0;
-  if (Wa > Wb) Pab = Wb / Wa;
-  else Pba = Wa / Wb;
-  const double na = Na * Wa * A.inv_area;
+  const double na = Na * A.w[0] * A.inv_area;
   double Nc = na * Nb * A.dt * A.sgmax;
-  Nc /= Pab + (Wb / Wa) * Pba;
+  Nc /= A.denom;
   if (!A.same) Nc *= 2.0;
   Nc += A.remaining[k];
   const double fl = floor(Nc);
@@ -283,37 +396,37 @@ __global__ void __launch_bounds__(32) k_dsmc_cells(DsmcArgs A) {
   const uint32_t *id1 = pick(S1.id[0], S1.id[1], S1.st->cur);
   unsigned *la = A.idx[0] + sa0, *lb = A.idx[1] + sb0;
   if (Na <= kDsmcStage && Nb <= kDsmcStage) {
-    warp_rank_sort(la, Na, id0, sh, sh.sa, lane);
-    if (!A.same) warp_rank_sort(lb, Nb, id1, sh, sh.sb, lane);
-    for (int r = lane; r < Na; r += 32) sh.va[r] = vel_of(S0, sh.sa[r]);
+    rank_sort<T>(la, Na, id0, sh, sh.sa);
+    if (!A.same) rank_sort<T>(lb, Nb, id1, sh, sh.sb);
+    for (int r = lane; r < Na; r += T) sh.va[r] = vel_of(S0, sh.sa[r]);
     if (!A.same)
-      for (int r = lane; r < Nb; r += 32) sh.vb[r] = vel_of(S1, sh.sb[r]);
-    __syncwarp();
+      for (int r = lane; r < Nb; r += T) sh.vb[r] = vel_of(S1, sh.sb[r]);
+    __syncthreads();
     float3 *vb = A.same ? sh.va : sh.vb;
     auto ga = [&](int r) { return sh.va[r]; };
     auto sa = [&](int r, float3 v) { sh.va[r] = v; };
     auto gb = [&](int r) { return vb[r]; };
     auto sb = [&](int r, float3 v) { vb[r] = v; };
-    const unsigned nacc = dsmc_pairs(A, k, step, ncol, Na, Nb, lane, ga, sa, gb, sb);
+    const unsigned nacc = dsmc_pairs<T>(A, gt, st, k, step, ncol, Na, Nb, &first, ga, sa, gb, sb);
     if (lane == 0) {
       A.nu[k] = nacc;
       A.remaining[k] = Nc - fl;
     }
-    __syncwarp();
-    for (int r = lane; r < Na; r += 32) set_vel(S0, sh.sa[r], sh.va[r]);
+    __syncthreads();
+    for (int r = lane; r < Na; r += T) set_vel(S0, sh.sa[r], sh.va[r]);
     if (!A.same)
-      for (int r = lane; r < Nb; r += 32) set_vel(S1, sh.sb[r], sh.vb[r]);
+      for (int r = lane; r < Nb; r += T) set_vel(S1, sh.sb[r], sh.vb[r]);
     return;
   }
   // a crowded cell: lists ranked into identifier order in global memory,
   // velocities in global memory
   {
     unsigned *oa = A.ord[0] + sa0;
-    warp_rank_sort_long(la, Na, id0, sh, oa, lane);
+    rank_sort_long<T>(la, Na, id0, sh, oa);
     la = oa;
     if (!A.same) {
       unsigned *ob = A.ord[1] + sb0;
-      warp_rank_sort_long(lb, Nb, id1, sh, ob, lane);
+      rank_sort_long<T>(lb, Nb, id1, sh, ob);
       lb = ob;
     } else {
       lb = oa;
@@ -323,7 +436,7 @@ __global__ void __launch_bounds__(32) k_dsmc_cells(DsmcArgs A) {
   auto sa = [&](int r, float3 v) { set_vel(S0, la[r], v); };
   auto gb = [&](int r) { return vel_of(S1, lb[r]); };
   auto sb = [&](int r, float3 v) { set_vel(S1, lb[r], v); };
-  const unsigned nacc = dsmc_pairs(A, k, step, ncol, Na, Nb, lane, ga, sa, gb, sb);
+  const unsigned nacc = dsmc_pairs<T>(A, gt, st, k, step, ncol, Na, Nb, &first, ga, sa, gb, sb);
   if (lane == 0) {
     A.nu[k] = nacc;
     A.remaining[k] = Nc - fl;
@@ -356,16 +469,27 @@ int launch_dsmc(Ctx *c, int k, double dt, uint64_t seed, const unsigned long lon
                 unsigned long long step_value) {
   Dsmc *d = dsmc_of(c)[k];
   const int nn = c->nn;
-  ISKRA_CUDA(c, cudaMemsetAsync(d->cnt, 0, 2 * (size_t)(nn + 1) * sizeof(int), c->stream));
-  ISKRA_CUDA(c, cudaMemsetAsync(d->fill, 0, 2 * (size_t)nn * sizeof(int), c->stream));
-  const int blocks = c->num_sms * 4;
   const int nsp = d->a == d->b ? 1 : 2;
-  for (int q = 0; q < nsp; q++) {
-    const Species &sp = c->species[q == 0 ? d->a : d->b];
-    k_dsmc_count<<<blocks, 256, 0, c->stream>>>(sp.dev, c->nx, d->cnt + (size_t)q * (nn + 1));
-    k_dsmc_scan<<<1, 1024, 0, c->stream>>>(d->cnt + (size_t)q * (nn + 1), nn);
-    k_dsmc_scatter<<<blocks, 256, 0, c->stream>>>(sp.dev, c->nx, d->cnt + (size_t)q * (nn + 1),
-                                                   d->fill + (size_t)q * nn, d->idx[q]);
+  const long long slots = std::max(c->species[d->a].cap, c->species[d->b].cap);
+  if (nn <= kBucketCells && slots <= kBucketSlots) {
+    DsmcBuckets B{};
+    for (int q = 0; q < nsp; q++) {
+      B.s[q] = c->species[q == 0 ? d->a : d->b].dev;
+      B.cnt[q] = d->cnt + (size_t)q * (nn + 1);
+      B.idx[q] = d->idx[q];
+    }
+    ISKRA_CUDA(c, launch_pdl(k_dsmc_bucket, nsp, 1024, (size_t)nn * sizeof(int), c->stream, B, c->nx, nn));
+  } else {
+    ISKRA_CUDA(c, cudaMemsetAsync(d->cnt, 0, 2 * (size_t)(nn + 1) * sizeof(int), c->stream));
+    ISKRA_CUDA(c, cudaMemsetAsync(d->fill, 0, 2 * (size_t)nn * sizeof(int), c->stream));
+    const int blocks = c->num_sms * 4;
+    for (int q = 0; q < nsp; q++) {
+      const Species &sp = c->species[q == 0 ? d->a : d->b];
+      k_dsmc_count<<<blocks, 256, 0, c->stream>>>(sp.dev, c->nx, d->cnt + (size_t)q * (nn + 1));
+      k_dsmc_scan<<<1, 1024, 0, c->stream>>>(d->cnt + (size_t)q * (nn + 1), nn);
+      k_dsmc_scatter<<<blocks, 256, 0, c->stream>>>(sp.dev, c->nx, d->cnt + (size_t)q * (nn + 1),
+                                                     d->fill + (size_t)q * nn, d->idx[q]);
+    }
   }
   ISKRA_CUDA(c, cudaGetLastError());
   DsmcArgs A{};
@@ -380,6 +504,8 @@ int launch_dsmc(Ctx *c, int k, double dt, uint64_t seed, const unsigned long lon
   A.sgmax = d->sgmax;
   A.dt = dt;
   A.inv_area = 1.0 / (c->g.dx * c->g.dy);
+  const double Wa = A.w[0], Wb = A.w[1];
+  A.denom = (Wa > Wb ? Wb / Wa : 1.0) + (Wb / Wa) * (Wa > Wb ? 1.0 : Wa / Wb);  // Pab + (Wb/Wa) Pba
   A.nn = nn;
   A.same = d->a == d->b;
   A.remaining = d->remaining;
@@ -397,7 +523,8 @@ int launch_dsmc(Ctx *c, int k, double dt, uint64_t seed, const unsigned long lon
   A.set = (uint32_t)k;
   A.step = step;
   A.step_value = step_value;
-  ISKRA_CUDA(c, launch_pdl(k_dsmc_cells, nn, 32, 0, c->stream, A));
+  if (nn <= c->num_sms * 8) ISKRA_CUDA(c, launch_pdl(k_dsmc_cells<128>, nn, 128, 0, c->stream, A));
+  else ISKRA_CUDA(c, launch_pdl(k_dsmc_cells<32>, nn, 32, 0, c->stream, A));
   ISKRA_CUDA(c, cudaGetLastError());
   return ISKRA_OK;
 }
