@@ -257,6 +257,7 @@ __device__ __forceinline__ void cp_async16(unsigned dst, const void *src, unsign
 template <bool RELU>
 __global__ void __launch_bounds__(128) k_conv32_tc(const bf16 *__restrict__ in, const bf16 *__restrict__ w,
                                                    bf16 *__restrict__ out, int H, int W, int *err) {
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char tc_smem[];
   __shared__ __align__(8) unsigned long long bar[2];
   __shared__ unsigned tmem_base;
@@ -389,6 +390,7 @@ template <bool RELU>
 __global__ void __launch_bounds__(128) k_conv32_tma(const __grid_constant__ CUtensorMap map,
                                                     const bf16 *__restrict__ w, bf16 *__restrict__ out, int H, int W,
                                                     int *err) {
+  pdl_wait();
   extern __shared__ __align__(128) unsigned char tc_smem[];
   __shared__ __align__(8) unsigned long long ld_bar[2], mma_bar[2];
   __shared__ unsigned tmem_base;
@@ -530,6 +532,7 @@ __global__ void __launch_bounds__(128) k_conv32_tma(const __grid_constant__ CUte
 // and add their sums to dw once.
 __global__ void __launch_bounds__(288) k_conv32_dw(const bf16 *__restrict__ in, const bf16 *__restrict__ dz,
                                                    float *__restrict__ dw, int H, int W) {
+  pdl_wait();
   __shared__ __align__(16) bf16 patch[kPatch][kPs];
   __shared__ __align__(16) bf16 dzs[kTy * kTx][kPs];
   const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5;
@@ -595,6 +598,7 @@ __global__ void __launch_bounds__(288) k_conv32_dw(const bf16 *__restrict__ in, 
 // weights in registers; the quad's x loads coincide (one transaction).
 __global__ void __launch_bounds__(256) k_enc0(const float *__restrict__ x, const bf16 *__restrict__ w0,
                                               bf16 *__restrict__ a0, int H, int W) {
+  pdl_wait();
   const int o = threadIdx.x & 3;
   float wr[9][8];
 #pragma unroll
@@ -629,17 +633,30 @@ __global__ void __launch_bounds__(256) k_enc0(const float *__restrict__ x, const
   }
 }
 
+constexpr int kDwIlp = 8;
 // dw0[tap][c] += Σ_p x[p + off(tap)] dz[p][c]: thread (tap, c) of 288
 __global__ void __launch_bounds__(288) k_enc0_dw(const float *__restrict__ x, const bf16 *__restrict__ dz,
                                                  float *__restrict__ dw, int H, int W) {
+  pdl_wait();
   const int tap = threadIdx.x / kCh, c = threadIdx.x % kCh;
   const int oy = tap / 3 - 1, ox = tap % 3 - 1;
   const int P = H * W;
   float s = 0.f;
-  for (int p = blockIdx.x; p < P; p += gridDim.x) {
-    const int y = p / W + oy, xx = p % W + ox;
-    if (y < 0 || y >= H || xx < 0 || xx >= W) continue;
-    s = fmaf(x[y * W + xx], bf(dz[(size_t)p * kCh + c]), s);
+  // kDwIlp pixels' loads in flight together: one at a time the pass was the length
+  // of its ~80 dependent loads (256 x 192: 30 us)
+  for (int p0 = blockIdx.x; p0 < P; p0 += kDwIlp * gridDim.x) {
+    float a[kDwIlp];
+    bf16 g[kDwIlp];
+#pragma unroll
+    for (int u = 0; u < kDwIlp; u++) {
+      const int p = p0 + u * gridDim.x;
+      const int y = p / W + oy, xx = p % W + ox;
+      const bool in = p < P && y >= 0 && y < H && xx >= 0 && xx < W;
+      a[u] = in ? x[y * W + xx] : 0.f;
+      g[u] = in ? dz[(size_t)p * kCh + c] : __float2bfloat16(0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < kDwIlp; u++) s = fmaf(a[u], bf(g[u]), s);
   }
   atomicAdd(dw + tap * kCh + c, s);
 }
@@ -650,6 +667,7 @@ __global__ void __launch_bounds__(288) k_enc0_dw(const float *__restrict__ x, co
 // block's pixel range advances uniformly so every lane reaches the shuffles.
 __global__ void __launch_bounds__(256) k_head(const bf16 *__restrict__ a, const bf16 *__restrict__ w7,
                                               float *__restrict__ y, int H, int W) {
+  pdl_wait();
   const int o = threadIdx.x & 3;
   float wr[9][8];
 #pragma unroll
@@ -689,6 +707,7 @@ __global__ void __launch_bounds__(256) k_head(const bf16 *__restrict__ a, const 
 // dz6[p][c] = (Σ_tap dy[p - off(tap)] w7[tap][c]) (a6[p][c] > 0)
 __global__ void k_head_dx(const float *__restrict__ dy, const bf16 *__restrict__ w7, const bf16 *__restrict__ a,
                           bf16 *__restrict__ dz, int H, int W) {
+  pdl_wait();
   __shared__ float ws[kW1];
   for (int t = threadIdx.x; t < kW1; t += blockDim.x) ws[t] = bf(w7[t]);
   __syncthreads();
@@ -726,14 +745,24 @@ __global__ void k_head_dx(const float *__restrict__ dy, const bf16 *__restrict__
 // dw7[tap][c] += Σ_p a[p + off(tap)][c] dy[p]: thread (tap, c) of 288
 __global__ void __launch_bounds__(288) k_head_dw(const bf16 *__restrict__ a, const float *__restrict__ dy,
                                                  float *__restrict__ dw, int H, int W) {
+  pdl_wait();
   const int tap = threadIdx.x / kCh, c = threadIdx.x % kCh;
   const int oy = tap / 3 - 1, ox = tap % 3 - 1;
   const int P = H * W;
   float s = 0.f;
-  for (int p = blockIdx.x; p < P; p += gridDim.x) {
-    const int y = p / W + oy, xx = p % W + ox;
-    if (y < 0 || y >= H || xx < 0 || xx >= W) continue;
-    s = fmaf(bf(a[((size_t)y * W + xx) * kCh + c]), dy[p], s);
+  for (int p0 = blockIdx.x; p0 < P; p0 += kDwIlp * gridDim.x) {  // (as k_enc0_dw)
+    bf16 v[kDwIlp];
+    float g[kDwIlp];
+#pragma unroll
+    for (int u = 0; u < kDwIlp; u++) {
+      const int p = p0 + u * gridDim.x;
+      const int y = p / W + oy, xx = p % W + ox;
+      const bool in = p < P && y >= 0 && y < H && xx >= 0 && xx < W;
+      v[u] = in ? a[((size_t)y * W + xx) * kCh + c] : __float2bfloat16(0.f);
+      g[u] = in ? dy[p] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kDwIlp; u++) s = fmaf(bf(v[u]), g[u], s);
   }
   atomicAdd(dw + tap * kCh + c, s);
 }
@@ -756,6 +785,7 @@ __device__ __forceinline__ uint4 ld8(const bf16 *base, size_t pix, int q) {
 
 // out (H/2 x W/2) = 2x2 average of in (H x W)
 __global__ void k_pool(const bf16 *__restrict__ in, bf16 *__restrict__ out, int H, int W) {
+  pdl_wait();
   const int h = H / 2, w = W / 2, n = h * w * 4;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = t & 3, p = t >> 2, y = p / w, x = p - y * w;
@@ -775,6 +805,7 @@ __global__ void k_pool(const bf16 *__restrict__ in, bf16 *__restrict__ out, int 
 // u (H x W) = up(a) + skip, a at H/2 x W/2
 __global__ void k_up_add(const bf16 *__restrict__ a, const bf16 *__restrict__ skip, bf16 *__restrict__ u, int H,
                          int W) {
+  pdl_wait();
   const int n = H * W * 4, w = W / 2;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = t & 3, p = t >> 2, y = p / W, x = p - y * W;
@@ -790,6 +821,7 @@ __global__ void k_up_add(const bf16 *__restrict__ a, const bf16 *__restrict__ sk
 // dz (h x w) = (Σ over the 2x2 children of du (2h x 2w)) (a > 0)
 __global__ void k_up_bwd_mask(const bf16 *__restrict__ du, const bf16 *__restrict__ a, bf16 *__restrict__ dz, int h,
                               int w) {
+  pdl_wait();
   const int n = h * w * 4, W = 2 * w;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = t & 3, p = t >> 2, y = p / w, x = p - y * w;
@@ -810,6 +842,7 @@ __global__ void k_up_bwd_mask(const bf16 *__restrict__ du, const bf16 *__restric
 // dz (H x W) = (dp(y/2, x/2) / 4 + ds) (a > 0), dp at H/2 x W/2
 __global__ void k_pool_bwd_mask(const bf16 *__restrict__ dp, const bf16 *__restrict__ ds, const bf16 *__restrict__ a,
                                 bf16 *__restrict__ dz, int H, int W) {
+  pdl_wait();
   const int n = H * W * 4, w = W / 2;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = t & 3, p = t >> 2, y = p / W, x = p - y * W;
@@ -995,6 +1028,9 @@ struct Lws {
   LwsScal *scal = nullptr;                     // device: s of the running solve, warm-start statistics
   std::vector<std::pair<const void *, CUtensorMap>> maps;  // TMA maps of the 32 -> 32 convolutions' inputs
   std::vector<void *> allocs;
+  cudaGraphExec_t fwd = nullptr, bwd = nullptr;  // the passes' launches (lws_replay)
+  cudaStream_t side = nullptr;                 // weight gradients beside the chain of activation gradients
+  cudaEvent_t fork[7] = {}, join = nullptr;
 };
 
 namespace {
@@ -1007,6 +1043,12 @@ int lws_alloc(Ctx *c, Lws *L, void **p, size_t bytes) {
 }
 
 void lws_free(Lws *L) {
+  if (L->fwd) cudaGraphExecDestroy(L->fwd);
+  if (L->bwd) cudaGraphExecDestroy(L->bwd);
+  if (L->side) cudaStreamDestroy(L->side);
+  for (cudaEvent_t e : L->fork)
+    if (e) cudaEventDestroy(e);
+  if (L->join) cudaEventDestroy(L->join);
   for (void *p : L->allocs) cudaFree(p);
   delete L;
 }
@@ -1025,11 +1067,12 @@ dim3 conv_grid(int H, int W) { return dim3((W + kTx - 1) / kTx, (H + kTy - 1) / 
     if (rc_) return rc_;     \
   } while (0)
 
+#define LWS_LAUNCH(kern, grid, block, smem, ...) ISKRA_CUDA(c, launch_pdl(kern, grid, block, smem, st, __VA_ARGS__))
+
 // out = act(conv(in, w)) for one 32 -> 32 layer: tcgen05 kernel, or the
 // mma.sync kernel when the context selected it (ISKRA_CONV_MMA_SYNC=1, kept
 // for measurement)
-int conv32(Ctx *c, bool relu, const bf16 *in, const bf16 *w, bf16 *out, int H, int W) {
-  cudaStream_t st = c->stream;
+int conv32(Ctx *c, cudaStream_t st, bool relu, const bf16 *in, const bf16 *w, bf16 *out, int H, int W) {
   static const bool legacy = [] {
     const char *e = std::getenv("ISKRA_CONV_MMA_SYNC");
     return e && e[0] == '1';
@@ -1054,12 +1097,9 @@ int conv32(Ctx *c, bool relu, const bf16 *in, const bf16 *w, bf16 *out, int H, i
   for (const auto &m : c->lws->maps)
     if (m.first == in) map = &m.second;
   if (map) {
-    if (relu) k_conv32_tma<true><<<grid, 128, kTmaSmem, st>>>(*map, w, out, H, W, c->d_err);
-    else k_conv32_tma<false><<<grid, 128, kTmaSmem, st>>>(*map, w, out, H, W, c->d_err);
-  } else if (relu) {
-    k_conv32_tc<true><<<grid, 128, kTcSmem, st>>>(in, w, out, H, W, c->d_err);
+    LWS_LAUNCH(relu ? k_conv32_tma<true> : k_conv32_tma<false>, grid, 128, kTmaSmem, *map, w, out, H, W, c->d_err);
   } else {
-    k_conv32_tc<false><<<grid, 128, kTcSmem, st>>>(in, w, out, H, W, c->d_err);
+    LWS_LAUNCH(relu ? k_conv32_tc<true> : k_conv32_tc<false>, grid, 128, kTcSmem, in, w, out, H, W, c->d_err);
   }
   ISKRA_CUDA(c, cudaGetLastError());
   return ISKRA_OK;
@@ -1109,68 +1149,123 @@ static void make_maps(Lws *L) {
   for (int l = 1; l <= 3; l++) add(L->dz[l], l);
 }
 
-int lws_forward(Ctx *c, Lws *L) {
+// Replays a fixed sequence of launches as a graph (captured when it is first
+// needed; *exec belongs to the network): a pass is 14 to 33 launches of a few
+// microseconds each, which the host could not queue as fast as they run (256 x
+// 192: forward, then forward and backward with the copies around them 496 -> 332 us,
+// with the weight gradients beside the chain and their loads in flight).
+// Inside another capture the launches are queued as they are.
+template <class F>
+int lws_replay(Ctx *c, cudaGraphExec_t *exec, F queue) {
+  cudaStreamCaptureStatus cs;
+  ISKRA_CUDA(c, cudaStreamIsCapturing(c->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return queue();
+  if (!*exec) {
+    cudaGraph_t g;
+    ISKRA_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = queue();
+    const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    if (rc) {
+      if (e == cudaSuccess) cudaGraphDestroy(g);
+      return rc;
+    }
+    ISKRA_CUDA(c, e);
+    const cudaError_t ei = cudaGraphInstantiate(exec, g, 0);
+    cudaGraphDestroy(g);
+    ISKRA_CUDA(c, ei);
+  }
+  ISKRA_CUDA(c, cudaGraphLaunch(*exec, c->stream));
+  return ISKRA_OK;
+}
+
+int lws_queue_forward(Ctx *c, Lws *L) {
   cudaStream_t st = c->stream;
   const int T = 256;
   const bf16 *wb = L->wb;
   const int *h = L->h, *w = L->w;
-  k_enc0<<<blocks_for(c, (long long)h[0] * w[0], T), T, 0, st>>>(L->x, wb + layer_off(0), L->a[0], h[0], w[0]);
+  LWS_LAUNCH(k_enc0, blocks_for(c, (long long)h[0] * w[0], T), T, 0, L->x, wb + layer_off(0), L->a[0], h[0], w[0]);
   for (int l = 1; l <= 3; l++) {
-    k_pool<<<blocks_for(c, (long long)h[l] * w[l] * 4, T), T, 0, st>>>(L->a[l - 1], L->p[l], h[l - 1], w[l - 1]);
-    LWS_TRY(conv32(c, true, L->p[l], wb + layer_off(l), L->a[l], h[l], w[l]));
+    LWS_LAUNCH(k_pool, blocks_for(c, (long long)h[l] * w[l] * 4, T), T, 0, L->a[l - 1], L->p[l], h[l - 1], w[l - 1]);
+    LWS_TRY(conv32(c, st, true, L->p[l], wb + layer_off(l), L->a[l], h[l], w[l]));
   }
   // decoder: a4 at level 2, a5 at level 1, a6 at level 0
   for (int l = 2; l >= 0; l--) {
     const int li = 6 - l;  // layer 4, 5, 6
-    k_up_add<<<blocks_for(c, (long long)h[l] * w[l] * 4, T), T, 0, st>>>(L->a[li - 1], L->a[l], L->u[l], h[l], w[l]);
-    LWS_TRY(conv32(c, true, L->u[l], wb + layer_off(li), L->a[li], h[l], w[l]));
+    LWS_LAUNCH(k_up_add, blocks_for(c, (long long)h[l] * w[l] * 4, T), T, 0, L->a[li - 1], L->a[l], L->u[l], h[l],
+               w[l]);
+    LWS_TRY(conv32(c, st, true, L->u[l], wb + layer_off(li), L->a[li], h[l], w[l]));
   }
-  k_head<<<blocks_for(c, (long long)h[0] * w[0], T), T, 0, st>>>(L->a[6], wb + layer_off(7), L->y, h[0], w[0]);
-  ISKRA_CUDA(c, cudaGetLastError());
+  LWS_LAUNCH(k_head, blocks_for(c, (long long)h[0] * w[0], T), T, 0, L->a[6], wb + layer_off(7), L->y, h[0], w[0]);
   return ISKRA_OK;
 }
+int lws_forward(Ctx *c, Lws *L) {
+  return lws_replay(c, &L->fwd, [&] { return lws_queue_forward(c, L); });
+}
 
-// loss and gradients (into g32, zeroed here) for target tscale t: the mean
-// squared error of the output (energy = false) or the energy norm of the
-// error under the 5-point stencil, the norm CG minimises (energy = true)
-int lws_backward(Ctx *c, Lws *L, const float *t, float tscale, bool energy = false) {
-  cudaStream_t st = c->stream;
+// Gradients (into g32, zeroed here) from the output gradient dy.  The weight
+// gradients hang off the chain of activation gradients: they run beside it on a
+// second stream, which joins at the end.
+int lws_queue_backward(Ctx *c, Lws *L) {
   const int T = 256;
   const int *h = L->h, *w = L->w;
   const int P0 = h[0] * w[0];
+  cudaStream_t main = c->stream, side = L->side;
   // weight-gradient blocks: at most two per SM, at most one per tile of the level
   auto dwb = [&](int l) {
     return std::max(1, std::min(2 * c->num_sms, ((w[l] + kTx - 1) / kTx) * ((h[l] + kTy - 1) / kTy)));
   };
+  int ev = 0;
+  auto fork = [&]() -> int {  // the side stream goes on from here
+    ISKRA_CUDA(c, cudaEventRecord(L->fork[ev], main));
+    ISKRA_CUDA(c, cudaStreamWaitEvent(side, L->fork[ev], 0));
+    ev++;
+    return ISKRA_OK;
+  };
+  cudaStream_t st = main;
   ISKRA_CUDA(c, cudaMemsetAsync(L->g32, 0, kParams * sizeof(float), st));
-  if (energy) {
-    k_err<<<blocks_for(c, P0, T), T, 0, st>>>(L->y, t, tscale, L->te, P0);
-    k_energy<<<blocks_for(c, P0, T), T, 0, st>>>(L->te, L->dy, h[0], w[0], L->loss);
-  } else {
-    k_mse<<<blocks_for(c, P0, T), T, 0, st>>>(L->y, t, tscale, L->dy, P0, L->loss);
-  }
-  k_head_dx<<<blocks_for(c, P0, T), T, 0, st>>>(L->dy, L->wb + layer_off(7), L->a[6], L->dz[6], h[0], w[0]);
-  k_head_dw<<<std::min(P0, 4 * c->num_sms), 288, 0, st>>>(L->a[6], L->dy, L->g32 + layer_off(7), h[0], w[0]);
+  LWS_TRY(fork());
+  k_head_dw<<<std::min(P0, 4 * c->num_sms), 288, 0, side>>>(L->a[6], L->dy, L->g32 + layer_off(7), h[0], w[0]);
+  LWS_LAUNCH(k_head_dx, blocks_for(c, P0, T), T, 0, L->dy, L->wb + layer_off(7), L->a[6], L->dz[6], h[0], w[0]);
   // decoder layers 6, 5, 4 (levels 0, 1, 2): input u[l], output gradient dz[li]
   for (int l = 0; l <= 2; l++) {
     const int li = 6 - l;
-    LWS_TRY(conv32(c, false, L->dz[li], L->wt + layer_off(li), L->du[l], h[l], w[l]));
-    k_conv32_dw<<<dwb(l), 288, 0, st>>>(L->u[l], L->dz[li], L->g32 + layer_off(li), h[l], w[l]);
+    LWS_TRY(fork());
+    k_conv32_dw<<<dwb(l), 288, 0, side>>>(L->u[l], L->dz[li], L->g32 + layer_off(li), h[l], w[l]);
+    LWS_TRY(conv32(c, st, false, L->dz[li], L->wt + layer_off(li), L->du[l], h[l], w[l]));
     // the upsampled input came from layer li - 1 one level down
-    k_up_bwd_mask<<<blocks_for(c, (long long)h[l + 1] * w[l + 1] * 4, T), T, 0, st>>>(
-        L->du[l], L->a[li - 1], L->dz[li - 1], h[l + 1], w[l + 1]);
+    LWS_LAUNCH(k_up_bwd_mask, blocks_for(c, (long long)h[l + 1] * w[l + 1] * 4, T), T, 0, L->du[l], L->a[li - 1],
+               L->dz[li - 1], h[l + 1], w[l + 1]);
   }
   // encoder layers 3, 2, 1: input p[l], then the pooled layer l - 1 gets its
   // pooling gradient plus the skip gradient du[l - 1]
   for (int l = 3; l >= 1; l--) {
-    LWS_TRY(conv32(c, false, L->dz[l], L->wt + layer_off(l), L->dp[l], h[l], w[l]));
-    k_conv32_dw<<<dwb(l), 288, 0, st>>>(L->p[l], L->dz[l], L->g32 + layer_off(l), h[l], w[l]);
-    k_pool_bwd_mask<<<blocks_for(c, (long long)h[l - 1] * w[l - 1] * 4, T), T, 0, st>>>(
-        L->dp[l], L->du[l - 1], L->a[l - 1], L->dz[l - 1], h[l - 1], w[l - 1]);
+    LWS_TRY(fork());
+    k_conv32_dw<<<dwb(l), 288, 0, side>>>(L->p[l], L->dz[l], L->g32 + layer_off(l), h[l], w[l]);
+    LWS_TRY(conv32(c, st, false, L->dz[l], L->wt + layer_off(l), L->dp[l], h[l], w[l]));
+    LWS_LAUNCH(k_pool_bwd_mask, blocks_for(c, (long long)h[l - 1] * w[l - 1] * 4, T), T, 0, L->dp[l], L->du[l - 1],
+               L->a[l - 1], L->dz[l - 1], h[l - 1], w[l - 1]);
   }
-  k_enc0_dw<<<std::min(P0, 4 * c->num_sms), 288, 0, st>>>(L->x, L->dz[0], L->g32 + layer_off(0), h[0], w[0]);
+  LWS_LAUNCH(k_enc0_dw, std::min(P0, 4 * c->num_sms), 288, 0, L->x, L->dz[0], L->g32 + layer_off(0), h[0], w[0]);
+  ISKRA_CUDA(c, cudaEventRecord(L->join, side));
+  ISKRA_CUDA(c, cudaStreamWaitEvent(main, L->join, 0));
   ISKRA_CUDA(c, cudaGetLastError());
   return ISKRA_OK;
+}
+
+// loss and gradients for target tscale t: the mean squared error of the output
+// (energy = false) or the energy norm of the error under the 5-point stencil, the
+// norm CG minimises (energy = true)
+int lws_backward(Ctx *c, Lws *L, const float *t, float tscale, bool energy = false) {
+  cudaStream_t st = c->stream;
+  const int T = 256, P0 = L->h[0] * L->w[0];
+  if (energy) {
+    k_err<<<blocks_for(c, P0, T), T, 0, st>>>(L->y, t, tscale, L->te, P0);
+    k_energy<<<blocks_for(c, P0, T), T, 0, st>>>(L->te, L->dy, L->h[0], L->w[0], L->loss);
+  } else {
+    k_mse<<<blocks_for(c, P0, T), T, 0, st>>>(L->y, t, tscale, L->dy, P0, L->loss);
+  }
+  ISKRA_CUDA(c, cudaGetLastError());
+  return lws_replay(c, &L->bwd, [&] { return lws_queue_backward(c, L); });
 }
 
 int lws_sync_weights(Ctx *c, Lws *L) {
@@ -1349,6 +1444,13 @@ int iskra_lws_create(iskra_ctx *h, int capacity, uint64_t seed) {
     LWS_ALLOC(L->dout, (size_t)capacity * P0 * sizeof(float));
   }
 #undef LWS_ALLOC
+  bool ok = cudaStreamCreateWithFlags(&L->side, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaEventCreateWithFlags(&L->join, cudaEventDisableTiming) == cudaSuccess;
+  for (cudaEvent_t &e : L->fork) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    lws_free(L);
+    return set_err(c, ISKRA_ECUDA, "network streams");
+  }
   make_maps(L);
   // He initialisation (std sqrt(2 / fan_in)); the output layer starts small
   std::vector<float> w0(kParams);
