@@ -16,7 +16,8 @@
 // assembled operator has them; identity rows removed: the correction is zero
 // there).  Coarser levels halve each axis that has at least 3 nodes (6 when
 // periodic): coarse node I sits on fine node 2I, odd fine nodes interpolate
-// linearly from their two coarse neighbours (one at an open far end), so
+// linearly from their two coarse neighbours (one at an open far end; the seam of
+// an odd periodic axis is at axis_parents), so
 // P = Px (x) Py is bilinear; the coarse operator is the Galerkin product
 // P^T S P (9-point), formed on the host in FP64.  Smoother: damped Jacobi
 // (omega = 0.7), 2 sweeps before and after the coarse correction; the
@@ -63,35 +64,43 @@ void mg_destroy(Mg *m) {
 }
 
 // ---- interpolation weights along one axis ----------------------------------
-// fine index i -> up to two coarse parents with weights (coarsened axis of n
-// fine / nc coarse nodes, periodic when per): even i -> i/2 (1); odd i ->
-// (i-1)/2 and (i+1)/2 (1/2 each; (i+1)/2 wraps to 0 when periodic, and at an
-// open far end the single parent takes 1).  Not coarsened: i -> i (1).
-__host__ __device__ __forceinline__ int axis_parents(int i, int n, int nc, int coarsened, int per, int *c, float *w) {
-  if (!coarsened) {
-    c[0] = i;
-    w[0] = 1.f;
-    return 1;
-  }
-  if ((i & 1) == 0) {
-    c[0] = i >> 1;
-    w[0] = 1.f;
-    return 1;
-  }
+// The seam of a coarsened axis (MgXfer::seam_x, seam_y):
+//   kSeamOpen    no coupling, or an odd periodic axis of 2m + 1 nodes, m odd: fine
+//                nodes 2m and 0 are coarse nodes both, m + 1 in all
+//   kSeamEven    an even periodic axis: the last odd node lies between coarse
+//                nodes nc - 1 and 0
+//   kSeamJump    an odd periodic axis of 2m + 1 nodes, m even: m coarse nodes, fine
+//                node 2m - 1 takes the value of coarse node m - 1, fine node 2m that
+//                of coarse node 0
+// Both odd forms leave an even number of coarse nodes, so that the next coarsening
+// closes the uneven interval at the seam again: the spacings of a level stay within
+// a factor of 4, and point Jacobi goes on smoothing.  (Stopping at the odd axis and
+// coarsening the other alone, as the hierarchy first did, makes the operator
+// anisotropic: 257 x 257 nodes, y-periodic, took 48 iterations.)
+static int coarse_nodes(int n, int per) {
+  if (!per || n % 2 == 0) return (n + 1) / 2;
+  const int m = n / 2;
+  return m % 2 ? m + 1 : m;
+}
+static int seam(int n, int per) { return !per ? kSeamOpen : n % 2 == 0 ? kSeamEven : n / 2 % 2 ? kSeamOpen : kSeamJump; }
+
+// fine index i -> up to two coarse parents with weights (n fine / nc coarse nodes):
+// even i -> i/2 (1); odd i -> (i-1)/2 and (i+1)/2 (1/2 each), past the last coarse
+// node as the seam has it.  Not coarsened: i -> i (1).
+static int axis_parents(int i, int n, int nc, int coarsened, int per, int *c, float *w) {
+  const int sm = seam(n, per);
+  w[0] = 1.f;
+  c[0] = coarsened ? i >> 1 : i;
+  if (!coarsened) return 1;
+  if (c[0] >= nc) c[0] = 0;  // kSeamJump's last node
+  if ((i & 1) == 0) return 1;
   int hi = (i + 1) >> 1;
   if (hi >= nc) {
-    if (per) {
-      hi = 0;
-    } else {
-      c[0] = (i - 1) >> 1;
-      w[0] = 1.f;
-      return 1;
-    }
+    if (sm != kSeamEven) return 1;
+    hi = 0;
   }
-  c[0] = (i - 1) >> 1;
-  w[0] = 0.5f;
+  w[0] = w[1] = 0.5f;
   c[1] = hi;
-  w[1] = 0.5f;
   return 2;
 }
 
@@ -256,13 +265,13 @@ struct HostLevel {
   std::vector<char> active;  // node takes part in the correction
 };
 
-static bool can_coarsen(int n, int per) { return per ? (n >= 6 && n % 2 == 0) : n >= 3; }
+static bool can_coarsen(int n, int per) { return n >= (per ? 6 : 3); }
 
 // Galerkin P^T A P of a level onto its coarsening
 static HostLevel galerkin(const HostLevel &F, int cx, int cy) {
   HostLevel C;
-  C.nx = cx ? (F.per_x ? F.nx / 2 : (F.nx + 1) / 2) : F.nx;
-  C.ny = cy ? (F.per_y ? F.ny / 2 : (F.ny + 1) / 2) : F.ny;
+  C.nx = cx ? coarse_nodes(F.nx, F.per_x) : F.nx;
+  C.ny = cy ? coarse_nodes(F.ny, F.per_y) : F.ny;
   C.per_x = F.per_x;
   C.per_y = F.per_y;
   const int nf = F.nx * F.ny, nc = C.nx * C.ny;
@@ -280,7 +289,7 @@ static HostLevel galerkin(const HostLevel &F, int cx, int cy) {
     const int j = k / F.nx, i = k - j * F.nx;
     int fci[2], fcj[2];
     float fwi[2], fwj[2];
-    const int fpi = axis_parents(i, F.nx, C.nx, cx, C.per_x, fci, fwi);
+    const int fpi = axis_parents(i, F.nx, C.nx, cx, F.per_x, fci, fwi);
     const int fpj = axis_parents(j, F.ny, C.ny, cy, C.per_y, fcj, fwj);
     for (int dy = -1; dy <= 1; dy++)
       for (int dx = -1; dx <= 1; dx++) {
@@ -418,8 +427,8 @@ int mg_build(Ctx *c, int nx, int ny, const std::vector<double> &s0, const std::v
     D.nx = S.nx;
     D.ny = S.ny;
     D.n = S.nx * S.ny;
-    D.per_x = S.per_x;
-    D.per_y = S.per_y;
+    D.seam_x = seam(S.nx, S.per_x);
+    D.seam_y = seam(S.ny, S.per_y);
     D.cx = l + 1 < H.size() ? cxs[l] : 0;
     D.cy = l + 1 < H.size() ? cys[l] : 0;
     D.five = 1;
@@ -501,12 +510,14 @@ int mg_queue_cycle(Ctx *c, Mg *m, const double *r, double *z, const int *skip, c
   *dots_done = L > 1;
   auto xfer = [&](int l) {
     const MgLevel &F = m->lv[l], &C = m->lv[l + 1];
-    return MgXfer{F.nx, F.ny, C.nx, C.ny, F.cx, F.cy, F.per_x, F.per_y};
+    return MgXfer{F.nx, F.ny, C.nx, C.ny, F.cx, F.cy, F.seam_x, F.seam_y};
   };
   const int lb = m->bottom ? m->bottom : L - 1;  // first level not run by per-level kernels
   for (int l = 0; l < lb; l++) {
     MgLevel &F = m->lv[l], &C = m->lv[l + 1];
-    const dim3 g((C.nx + kDownCx - 1) / kDownCx, (C.ny + kDownCy - 1) / kDownCy);
+    // tiles over the fine nodes (kSeamJump has one beyond the last coarse node's two)
+    const int ox = F.cx ? 2 * kDownCx : kDownCx, oy = F.cy ? 2 * kDownCy : kDownCy;
+    const dim3 g((F.nx + ox - 1) / ox, (F.ny + oy - 1) / oy);
     ISKRA_CUDA(c, launch_pdl(F.five ? k_mg_down<true> : k_mg_down<false>, g, kDownThreads, 0, st,
                              (const float *)F.coef, (const float *)F.dinv, F.x, (const float *)F.b, C.b, xfer(l), skip,
                              l == 0 ? r : nullptr));

@@ -14,7 +14,7 @@ constexpr int kMgCoarsest = 128, kMgSingle = 400;
 
 struct MgLevel {
   int nx = 0, ny = 0, n = 0;
-  int per_x = 0, per_y = 0;   // couplings across the seam exist on this axis
+  int seam_x = 0, seam_y = 0;  // kSeam* of the axis
   int cx = 0, cy = 0;          // x / y coarsened towards the next level
   int five = 0;                // no corner couplings (5-point stencil)
   float *coef = nullptr;       // 9 x n: offset o = (dy + 1) 3 + (dx + 1), node-major
@@ -65,17 +65,20 @@ __device__ __forceinline__ float apply9t(const MgStencil<FIVE> &S, const float *
   return a;
 }
 
+enum { kSeamOpen = 0, kSeamEven = 1, kSeamJump = 2 };  // (multigrid.cu, interpolation weights)
 struct MgXfer {
-  int nx, ny, ncx, ncy, cx, cy, per_x, per_y;
+  int nx, ny, ncx, ncy, cx, cy, seam_x, seam_y;
 };
 
 // Weight along one axis of fine index f = 2I + d in coarse index I's restriction
-// (axis_parents transposed): 1 at d = 0, 1/2 beside it, 1 on an open far end's
-// last odd node, 0 outside the axis.
-__device__ __forceinline__ float restrict_weight(int f, int d, int n, int nc, int per) {
+// (axis_parents transposed): 1 at d = 0, 1/2 beside it, 1 on the last odd node
+// when it has one parent and on kSeamJump's last node (f = -1), 0 outside the axis.
+__device__ __forceinline__ float restrict_weight(int f, int d, int n, int nc, int seam) {
   if (d == 0) return 1.f;
-  if (!per && (f < 0 || f >= n)) return 0.f;
-  return !per && d > 0 && (f + 1) >> 1 >= nc ? 1.f : 0.5f;
+  if (seam == kSeamEven) return 0.5f;
+  if (f < 0) return seam == kSeamJump ? 1.f : 0.f;
+  if (f >= n) return 0.f;
+  return d > 0 && (f + 1) >> 1 >= nc ? 1.f : 0.5f;
 }
 
 // coarse b = P^T r at coarse node (I, J), gathered from its fine candidates
@@ -88,13 +91,13 @@ __device__ __forceinline__ float restrict_at(R r, const MgXfer &T, int I, int J)
   for (int dj = -1; dj <= 1; dj++) {
     if (!T.cy && dj) continue;
     const int fj = T.cy ? 2 * J + dj : J;
-    const float wy = restrict_weight(fj, dj, T.ny, T.ncy, T.per_y);
+    const float wy = restrict_weight(fj, dj, T.ny, T.ncy, T.seam_y);
     if (wy == 0.f) continue;
 #pragma unroll
     for (int di = -1; di <= 1; di++) {
       if (!T.cx && di) continue;
       const int fi = T.cx ? 2 * I + di : I;
-      const float wx = restrict_weight(fi, di, T.nx, T.ncx, T.per_x);
+      const float wx = restrict_weight(fi, di, T.nx, T.ncx, T.seam_x);
       if (wx != 0.f) s = fmaf(wx * wy, r(fi, fj), s);
     }
   }
@@ -103,20 +106,21 @@ __device__ __forceinline__ float restrict_at(R r, const MgXfer &T, int I, int J)
 
 // the parents of fine index i along one axis (axis_parents): c0, and c1 >= 0
 // when two share it equally
-__device__ __forceinline__ void prolong_parents(int i, int nc, int coarsened, int per, int &c0, int &c1) {
+__device__ __forceinline__ void prolong_parents(int i, int nc, int coarsened, int seam, int &c0, int &c1) {
   c0 = coarsened ? i >> 1 : i;
   c1 = -1;
+  if (coarsened && c0 >= nc) c0 = 0;  // kSeamJump's last node
   if (coarsened && (i & 1)) {
     const int hi = (i + 1) >> 1;
-    c1 = hi < nc ? hi : per ? 0 : -1;
+    c1 = hi < nc ? hi : seam == kSeamEven ? 0 : -1;
   }
 }
 
 // (P xc) at fine node (i, j)
 __device__ __forceinline__ float prolong_at(const float *xc, const MgXfer &T, int i, int j) {
   int i0, i1, j0, j1;
-  prolong_parents(i, T.ncx, T.cx, T.per_x, i0, i1);
-  prolong_parents(j, T.ncy, T.cy, T.per_y, j0, j1);
+  prolong_parents(i, T.ncx, T.cx, T.seam_x, i0, i1);
+  prolong_parents(j, T.ncy, T.cy, T.seam_y, j0, j1);
   const float w = (i1 >= 0 ? 0.5f : 1.f) * (j1 >= 0 ? 0.5f : 1.f);
   float v = w * xc[i0 + T.ncx * j0];
   if (i1 >= 0) v = fmaf(w, xc[i1 + T.ncx * j0], v);
@@ -187,7 +191,7 @@ __device__ __forceinline__ void mg_bottom_cycle(float *base, const MgLevel *__re
                                                 const float *cinv) {
   auto xfer = [&](int l) {
     const MgLevel &F = lv[l], &C = lv[l + 1];
-    return MgXfer{F.nx, F.ny, C.nx, C.ny, F.cx, F.cy, F.per_x, F.per_y};
+    return MgXfer{F.nx, F.ny, C.nx, C.ny, F.cx, F.cy, F.seam_x, F.seam_y};
   };
   float *at = base;
   for (int l = l0; l + 1 < L; l++) {
