@@ -229,13 +229,15 @@ __device__ __forceinline__ float selection_uniform(uint32_t pid, unsigned long l
   z ^= z >> 27;
   z *= 0x94D049BB133111EBull;
   z ^= z >> 31;
-  return (float)(z >> 40) * 5.9604644775390625e-08f;
+  // (24 bits, converted as a 32-bit integer: conversions from 64 bits run on the FP64 pipe)
+  return (float)(uint32_t)(z >> 40) * 5.9604644775390625e-08f;
 }
 
 // selections ~ Poisson(lam) by inversion (bounded) of the selection uniform u
 __device__ __forceinline__ int draw_selections(float u, float lam, float expl) {
-  float pk = expl, cdf = expl;
-  int nsel = 0;
+  if (!(u > expl)) return 0;
+  float pk = expl * lam, cdf = expl + pk;  // (lam / 1 is lam: the first selection takes no division)
+  int nsel = 1;
   while (u > cdf && nsel < 16) {
     nsel++;
     pk *= lam / nsel;

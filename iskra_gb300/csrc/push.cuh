@@ -80,8 +80,15 @@ __device__ __forceinline__ bool reduce_runs(int key, Moments &m, unsigned &n) {
   return tail;
 }
 
-// Move by d cells along one axis in FP32: offset h in [0,1) on the 2^-24 grid,
-// cell index i (int).  Returns the new offset; i is updated in place.
+// Whether at most kFewPairs lanes hold their neighbour's key: unsorted particles,
+// which deposit lane by lane for fewer instructions than the segmented sum takes.
+// Above that the same-address atomics of the pairs cost more than the sum.
+constexpr int kFewPairs = 6;
+__device__ __forceinline__ bool few_runs(int key) {
+  const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+  return __popc(__ballot_sync(0xffffffffu, prev == key) & ~1u) <= kFewPairs;
+}
+
 // Move by d cells along one axis in FP32: offset h in [0,1) on the 2^-24
 // grid, cell index i (int).  t0 = h + d (one rounding), its integer part k
 // moves the cell, the fraction t0 - k goes onto the 2^-24 grid (a fraction
@@ -171,8 +178,11 @@ template <int MODE>
 __device__ __forceinline__ int apply_boundary(int &i, int P) {
   if (i >= 0 && i < P) return 0;
   if (MODE == ISKRA_BND_WRAP) {
-    i %= P;
-    if (i < 0) i += P;
+    i += i < 0 ? P : -P;  // one period brings all but the fastest back
+    if ((unsigned)i >= (unsigned)P) {
+      i %= P;
+      if (i < 0) i += P;
+    }
     return 0;
   }
   if (MODE == ISKRA_BND_DISCARD) return i < 0 ? 1 : 2;
@@ -237,7 +247,7 @@ constexpr int kEnsWinCells = kEnsWin * kEnsWin;
 enum { kMomN, kMomU1, kMomU0, kMomV1, kMomV0, kMomQ2, kMomQ1, kMomQ0, kMoms };
 
 // Shared memory of an ensemble-run block: E records of the run's cells.
-// Dynamic shared memory of an ensemble push block (53 KB: 4 blocks per SM):
+// Dynamic shared memory of an ensemble push block (56 KB: 4 blocks per SM):
 // per warp a ring of kEnsStages record stages filled by cp.async (two warp
 // iterations in flight while the third is pushed), the selection buffer,
 // E at the window's nodes, the deposit moments.
@@ -245,8 +255,10 @@ constexpr int kEnsStages = 3;
 constexpr int kEnsWinNodes = 2 * kEnsWinCells + 2;  // most nodes of a window of at most kEnsWinCells cells
 struct PushShared {
   static constexpr int kWinCells = kEnsWinCells;
+  static constexpr bool kSorted = false;  // particles in any order
   float4 ra[8][kEnsStages][32];     // staged records {hx, hy, vx, vy}
   float2 rb[8][kEnsStages][32];     // staged records {vz, cell}
+  uint32_t ri[8][kEnsStages][32];   // staged identifiers (for the selection draw)
   MccWork wbuf[8][64];              // selected work-list entries, per warp
   float2 ne[kEnsWinNodes];          // E at the window's nodes (row stride: cells per row + 1)
   unsigned mom[kMoms][kWinCells];   // deposit moments of the window cells
@@ -284,6 +296,7 @@ constexpr int kPushBlock = ISKRA_PUSH_THREADS + (ISKRA_PUSH_BULK == 2 ? 32 : 0);
 template <int TS>
 struct TileShared {
   static constexpr int kTileC = 1 << TS;
+  static constexpr bool kSorted = true;            // cell-sorted particles but for the drift since the last sort
   static constexpr int kWin = kTileC + 2 * kHalo;  // window cells per axis
   static constexpr int kWinN = kWin + 1;           // window nodes per axis
   static constexpr int kWinCells = kWin * kWin;
@@ -307,6 +320,10 @@ __device__ __forceinline__ void cp_async_record(float4 *sa, float2 *sb, const fl
   const unsigned da = (unsigned)__cvta_generic_to_shared(sa), db = (unsigned)__cvta_generic_to_shared(sb);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(da), "l"(ga) : "memory");
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(db), "l"(gb) : "memory");
+}
+__device__ __forceinline__ void cp_async_id(uint32_t *si, const uint32_t *gi) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(si)), "l"(gi)
+               : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -430,8 +447,8 @@ __device__ __forceinline__ void window_cell(const SH &sh, int w, unsigned long l
 // cells (particles that drifted off the window, the unsorted tail) use the
 // global records and 64-bit atomics.  The deposit key is the window cell, or
 // SH::kWinCells + the global cell index, so runs never mix the two.
-template <bool PUSH, int MX, int MY, bool WIN, bool TRK = false, class SH>
-__device__ __forceinline__ int push_one(float4 *__restrict__ xv, float2 *__restrict__ zc, long long p, bool valid,
+template <bool PUSH, int MX, int MY, bool WIN, bool TRK = false, class SH, class I>
+__device__ __forceinline__ int push_one(float4 *__restrict__ xv, float2 *__restrict__ zc, I p, bool valid,
                                         float4 a, float2 b, const float2 *__restrict__ E2, const SH &sh,
                                         int ox, int oy, int ww, int wh, const PushParams &P, unsigned ab[4],
                                         int &flags, Moments &m, float4 *out_a = nullptr, float2 *out_b = nullptr) {
@@ -529,8 +546,8 @@ __device__ __forceinline__ int push_one(float4 *__restrict__ xv, float2 *__restr
 // Warp-collective deposit of one particle per lane (key from push_one).
 template <bool WIN, class SH>
 __device__ __forceinline__ void deposit_warp(const SpeciesDev &s, SH &sh, int key, Moments m, int nx) {
-  unsigned n;
-  if (reduce_runs(key, m, n) && key >= 0) {
+  unsigned n = 1;
+  if ((!SH::kSorted && few_runs(key)) ? key >= 0 : reduce_runs(key, m, n) && key >= 0) {
     if (WIN && key < SH::kWinCells) {
       window_add(sh, key, n, m);
     } else {
@@ -546,9 +563,9 @@ __device__ __forceinline__ void deposit_warp(const SpeciesDev &s, SH &sh, int ke
   }
 }
 
-template <bool PUSH, int MX, int MY, bool WIN, bool TRK = false, class SH>
+template <bool PUSH, int MX, int MY, bool WIN, bool TRK = false, class SH, class I>
 __device__ __forceinline__ void push_warp(const SpeciesDev &s, float4 *__restrict__ xv, float2 *__restrict__ zc,
-                                          long long p, bool valid, float4 a, float2 b,
+                                          I p, bool valid, float4 a, float2 b,
                                           const float2 *__restrict__ E2, SH &sh, int ox, int oy, int ww,
                                           int wh, const PushParams &P, unsigned ab[4], int &flags,
                                           float4 *out_a = nullptr, float2 *out_b = nullptr) {
