@@ -141,9 +141,11 @@ struct Poisson {
 };
 
 constexpr int kPartials = 1024;
-// blocks per SM of the node passes (residuals, conversions); tuned on GB300
+// blocks per SM of the node passes (residuals, conversions): they are latency bound;
+// 20 steps of a 512 x 512 slab took 3764 us at 2, 3748 at 3, 3727 at 4, 3757 at 5 and
+// 3872 at 6
 #ifndef ISKRA_RES_BLOCKS_PER_SM
-#define ISKRA_RES_BLOCKS_PER_SM 2
+#define ISKRA_RES_BLOCKS_PER_SM 4
 #endif
 
 void poisson_destroy(Poisson *p) {
@@ -416,23 +418,34 @@ __device__ __forceinline__ float residual_node(const OpView &op, const RowClass 
 
 // Block partials of the norms, then the last block to finish sums them in
 // block order (deterministic), updates relres/iters and sets sc->done when
-// ||res|| <= rtol ||rhs_eff||.  Ends the kernel for every other block.
+// ||res|| <= rtol ||rhs_eff||.  Ends the kernel for every other block.  (256
+// threads; block_sums instead of a shuffle tree in every warp.)
 template <bool FIRST>
 __device__ __forceinline__ void finish_norms(PoissonScal *sc, double *__restrict__ part, double a2, double b2,
-                                             double rtol2, SweepLoop loop, double *sh, int *last) {
-  const double ta = block_sum(a2, sh);
-  const double tb = FIRST ? block_sum(b2, sh) : 0.0;
+                                             double rtol2, SweepLoop loop) {
+  constexpr int K = FIRST ? 2 : 1;
+  __shared__ double buf[K * 256];
+  __shared__ int last;
+  double v[K], t[K];
+  v[0] = a2;
+  if (FIRST) v[K - 1] = b2;
+  block_sums<K>(v, buf, t);
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = ta;
-    if (FIRST) part[kPartials + blockIdx.x] = tb;
+#pragma unroll
+    for (int q = 0; q < K; q++) part[q * kPartials + blockIdx.x] = t[q];
     __threadfence();
-    *last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
+    last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!*last) return;
+  if (!last) return;
   __threadfence();
-  const double a = sum_partials(part, gridDim.x, sh);
-  const double bb = FIRST ? sum_partials(part + kPartials, gridDim.x, sh) : 0.0;
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    v[q] = 0;
+    for (int k = threadIdx.x; k < gridDim.x; k += 256) v[q] += __ldcg(part + q * kPartials + k);
+  }
+  block_sums<K>(v, buf, t);
+  const double a = t[0], bb = FIRST ? t[K - 1] : 0.0;
   if (threadIdx.x == 0) {
     sc->ticket = 0u;
     const double rhs2 = FIRST ? bb : sc->rhs2;
@@ -451,12 +464,17 @@ __device__ __forceinline__ void finish_norms(PoissonScal *sc, double *__restrict
   }
 }
 
+// The row classes in shared memory when they fit, copied 8 bytes a thread (a whole
+// class per thread is a chain of 16-byte copies: 1 us more in every residual pass).
+// They are written by the operator build: callable before pdl_wait.  The caller's
+// next block barrier makes them readable.
 __device__ __forceinline__ const RowClass *stage_classes(const OpView &op, RowClass *cls_sh) {
-  const bool sm = op.nclass <= kSmemClasses;
-  if (sm)
-    for (int t = threadIdx.x; t < op.nclass; t += blockDim.x) cls_sh[t] = op.classes[t];
-  __syncthreads();
-  return sm ? cls_sh : op.classes;
+  if (op.nclass > kSmemClasses) return op.classes;
+  static_assert(sizeof(RowClass) % 8 == 0, "copied in words of 8 bytes");
+  const double *__restrict__ src = reinterpret_cast<const double *>(op.classes);
+  double *dst = reinterpret_cast<double *>(cls_sh);
+  for (int t = threadIdx.x; t < op.nclass * (int)(sizeof(RowClass) / 8); t += blockDim.x) dst[t] = __ldg(src + t);
+  return cls_sh;
 }
 
 // Residual pass over all nodes (scaled residual to r32 or r64), optionally
@@ -468,12 +486,11 @@ __global__ void __launch_bounds__(256) k_residual(OpView op, const double *__res
                                                   PoissonScal *sc, double *__restrict__ r64, float *__restrict__ r32,
                                                   double *__restrict__ part, int nn, int singular, double rtol2,
                                                   EOut eo, SweepLoop loop) {
-  pdl_wait();
-  __shared__ double sh[40];
   __shared__ RowClass cls_sh[kSmemClasses];
-  __shared__ int last;
-  if (!FIRST && sc->done) return;
   const RowClass *__restrict__ CT = stage_classes(op, cls_sh);
+  pdl_wait();
+  if (!FIRST && sc->done) return;
+  __syncthreads();
   const double lam = singular ? sc->lambda : 0.0;
   const int nx = op.nx, ny = op.ny;
   double a2 = 0, b2 = 0;
@@ -483,7 +500,7 @@ __global__ void __launch_bounds__(256) k_residual(OpView op, const double *__res
     const float v = residual_node<FIRST>(op, CT, x, rho, neg_inv_eps0, lam, singular, k, i, j, r64, a2, b2);
     if (r32) r32[k] = v;
   }
-  finish_norms<FIRST>(sc, part, a2, b2, rtol2, loop, sh, &last);
+  finish_norms<FIRST>(sc, part, a2, b2, rtol2, loop);
 }
 
 // E = -∇ϕ at node k from ϕ at the node and its four stencil neighbours
@@ -618,21 +635,20 @@ __global__ void __launch_bounds__(256) k_residual_df(OpView op, const float2 *__
                                                      float2 *__restrict__ bd, PoissonScal *sc, float *__restrict__ r32,
                                                      double *__restrict__ part, int nn, int singular, double rtol2,
                                                      EOut eo, SweepLoop loop) {
-  pdl_wait();
-  __shared__ double sh[40];
   __shared__ RowClass cls_sh[kSmemClasses];
-  __shared__ int last;
+  const RowClass *__restrict__ CT = stage_classes(op, cls_sh);
+  pdl_wait();
   const int k0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   if (!FIRST && sc->done) {
     if (EOUT && sc->e_pending) efield_df_nodes(x, op.nx, op.ny, nn, eo, k0, stride);
     return;
   }
-  const RowClass *__restrict__ CT = stage_classes(op, cls_sh);
+  __syncthreads();
   const double lam = singular ? sc->lambda : 0.0;
   double a2 = 0, b2 = 0;
   residual_df_nodes<FIRST, EOUT>(op, CT, x, rho, rho_df, nie_df, neg_inv_eps0, bd, r32, nn, singular, lam, eo, k0,
                                  stride, a2, b2);
-  finish_norms<FIRST>(sc, part, a2, b2, rtol2, loop, sh, &last);
+  finish_norms<FIRST>(sc, part, a2, b2, rtol2, loop);
 }
 
 // mean-zero projection of the double-float ϕ (singular operators)
