@@ -396,6 +396,14 @@ int launch_efield64(Ctx *c, const double *phi) {
 // counting sort by cell (histogram -> exclusive scan -> scatter), dropping
 // discarded particles
 // ---------------------------------------------------------------------------
+// U particles per lane and round of the histogram and the scatter: their loads and
+// the atomics' round trips (a chain of three latencies) overlap.  U = 8 where every
+// warp has that much (launch_sort), else 1: 33.5e6 particles in random order
+// scattered in 1014 us (U = 1: 1250, 2: 1135, 4: 1115) and counted in 171 (199),
+// 4.2e6 nearly sorted ones in 90 and 35 us (104 and 34); at 2e5 particles, one per
+// thread, U = 8 only leaves threads idle (11 against 10 us).  The random scatter is
+// bound by its partly written sectors: 28 bytes of a particle in three of them.
+template <int U>
 __global__ void __launch_bounds__(256) k_hist(SpeciesDev s, int tiles_x, int ts, int *__restrict__ count) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -404,15 +412,19 @@ __global__ void __launch_bounds__(256) k_hist(SpeciesDev s, int tiles_x, int ts,
   const float2 *__restrict__ zc = pick(s.zc[0], s.zc[1], cur);
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long base = warp * 32; base < np; base += nwarps * 32) {
-    const long long p = base + lane;
-    int key = -1;
-    if (p < np) {
-      int cell = __float_as_int(zc[p].y);
-      if (cell >= 0) key = cell_key(cell & 0xffff, cell >> 16, tiles_x, ts);
+  for (long long base = warp * (32 * U); base < np; base += nwarps * (32 * U)) {
+    int cell[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long p = base + 32 * u + lane;
+      cell[u] = p < np ? __float_as_int(zc[p].y) : -1;
     }
-    unsigned peers = __match_any_sync(FULL, key);
-    if (key >= 0 && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(count + key, __popc(peers));
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int key = cell[u] >= 0 ? cell_key(cell[u] & 0xffff, cell[u] >> 16, tiles_x, ts) : -1;
+      const unsigned peers = __match_any_sync(FULL, key);
+      if (key >= 0 && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(count + key, __popc(peers));
+    }
   }
 }
 
@@ -502,6 +514,7 @@ __global__ void __launch_bounds__(1024) k_scan_down(const int *__restrict__ in, 
   }
 }
 
+template <int U>
 __global__ void __launch_bounds__(256) k_scatter(SpeciesDev s, int tiles_x, int ts, int *__restrict__ cursor) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -515,29 +528,38 @@ __global__ void __launch_bounds__(256) k_scatter(SpeciesDev s, int tiles_x, int 
   uint32_t *__restrict__ io = pick(s.id[0], s.id[1], cur ^ 1);
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long base = warp * 32; base < np; base += nwarps * 32) {
-    const long long p = base + lane;
-    int key = -1;
-    float4 a;
-    float2 b;
-    uint32_t pid = 0;
-    if (p < np) {
-      a = xv[p];
-      b = zc[p];
-      pid = id[p];
-      int cell = __float_as_int(b.y);
-      if (cell >= 0) key = cell_key(cell & 0xffff, cell >> 16, tiles_x, ts);
+  for (long long base = warp * (32 * U); base < np; base += nwarps * (32 * U)) {
+    float4 a[U];
+    float2 b[U];
+    uint32_t pid[U];
+    int pos[U];
+    unsigned peers[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long long p = base + 32 * u + lane;
+      b[u] = make_float2(0.f, __int_as_float(-1));
+      if (p < np) {
+        a[u] = xv[p];
+        b[u] = zc[p];
+        pid[u] = id[p];
+      }
     }
-    unsigned peers = __match_any_sync(FULL, key);
-    int leader = __ffs(peers) - 1;
-    int rank = __popc(peers & ((1u << lane) - 1u));
-    int pos = 0;
-    if (key >= 0 && lane == leader) pos = atomicAdd(cursor + key, __popc(peers));
-    pos = __shfl_sync(FULL, pos, leader) + rank;
-    if (key >= 0) {
-      xo[pos] = a;
-      zo[pos] = b;
-      io[pos] = pid;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int cell = __float_as_int(b[u].y);
+      const int key = cell >= 0 ? cell_key(cell & 0xffff, cell >> 16, tiles_x, ts) : -1;
+      peers[u] = __match_any_sync(FULL, key);
+      pos[u] = 0;
+      if (key >= 0 && lane == __ffs(peers[u]) - 1) pos[u] = atomicAdd(cursor + key, __popc(peers[u]));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int q = __shfl_sync(FULL, pos[u], __ffs(peers[u]) - 1) + __popc(peers[u] & ((1u << lane) - 1u));
+      if (__float_as_int(b[u].y) >= 0) {
+        xo[q] = a[u];
+        zo[q] = b[u];
+        io[q] = pid[u];
+      }
     }
   }
 }
@@ -567,7 +589,8 @@ int launch_sort(Ctx *c, int sid) {
   const int nk = c->nkeys;
   ISKRA_CUDA(c, cudaMemsetAsync(c->cell_count, 0, (size_t)(nk + 1) * sizeof(int), c->stream));
   int blocks = sort_blocks(c, s);
-  k_hist<<<blocks, 256, 0, c->stream>>>(s.dev, c->tiles_x, c->tile_shift, c->cell_count);
+  const bool wide = s.cap >= (long long)blocks * 256 * 8;
+  (wide ? k_hist<8> : k_hist<1>)<<<blocks, 256, 0, c->stream>>>(s.dev, c->tiles_x, c->tile_shift, c->cell_count);
   ISKRA_CUDA(c, cudaGetLastError());
   int nb = (nk + kScanItems - 1) / kScanItems;
   k_scan_reduce<<<nb, 1024, 0, c->stream>>>(c->cell_count, nk, c->scan_tmp);
@@ -578,7 +601,7 @@ int launch_sort(Ctx *c, int sid) {
   // cell_count is free again: keep the grand total there for k_sort_finish
   ISKRA_CUDA(c, cudaMemcpyAsync(c->cell_count + nk, c->cell_cursor + nk, sizeof(int), cudaMemcpyDeviceToDevice,
                                 c->stream));
-  k_scatter<<<blocks, 256, 0, c->stream>>>(s.dev, c->tiles_x, c->tile_shift, c->cell_cursor);
+  (wide ? k_scatter<8> : k_scatter<1>)<<<blocks, 256, 0, c->stream>>>(s.dev, c->tiles_x, c->tile_shift, c->cell_cursor);
   k_sort_finish<<<1, 1, 0, c->stream>>>(s.dev.st, c->cell_count + nk);
   ISKRA_CUDA(c, cudaGetLastError());
   s.tail = 0;
