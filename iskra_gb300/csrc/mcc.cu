@@ -176,12 +176,12 @@ constexpr int kSelChunk = 1024;  // particles per block pass of k_mcc_select
 // words of hit bits per run (one bit per work-list entry), after the entries
 __host__ __device__ __forceinline__ size_t hit_words(size_t cap) { return (cap + 31) / 32; }
 
-// Phase 1 over the particles of run blockIdx.y (R = 1 for a single context):
+// Phase 1 of an ensemble over the particles of run blockIdx.y:
 // a block collects the selected particles of a chunk in shared memory and
 // appends them to its run's segment [r cap_run, ...) of the work list with
 // one atomic on the run's counter nwork[r kNworkStride].  step_ahead = 1 draws for the
 // step after the device counter's (a list built before the step begins).
-__global__ void __launch_bounds__(256) k_mcc_select(const SpeciesDev *__restrict__ src, float lam, uint2 key1,
+__global__ void __launch_bounds__(256) k_mcc_select(const SpeciesDev *__restrict__ src, float lam,
                                                     const uint2 *__restrict__ keys,
                                                     const unsigned long long *__restrict__ d_step, int step_ahead,
                                                     MccWork *__restrict__ work, unsigned long long *__restrict__ nwork,
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) k_mcc_select(const SpeciesDev *__restrict
   const unsigned FULL = 0xffffffffu;
   const int r = blockIdx.y;
   const SpeciesDev s = src[r];
-  const uint2 key = keys ? keys[r] : key1;
+  const uint2 key = keys[r];
   const int lane = threadIdx.x & 31;
   const long long np = s.st->np;
   const int cur = s.st->cur;
@@ -274,9 +274,6 @@ __device__ __forceinline__ bool mcc_entry_hits(const MccWork &e, const MccDev &M
   return false;
 }
 
-// Phase 2 over the work list segment of run r = blockIdx.y: the run's stores
-// src[r] / prod[r], node field E + r nn, key keys[r] (or M's key for a single
-// context), counters counts_runs + r N (or M.counts).
 // Blocks of 256 threads per SM asked of the register allocator for the
 // collision kernel: 3 (80 registers) against 2 (102 registers) -- measured
 // when the kernel also tested every entry: 245 against 283 us per electron
@@ -331,7 +328,7 @@ __global__ void __launch_bounds__(256) k_mcc_test(MccDev M, const uint2 *__restr
   const MccWork *__restrict__ seg = work + (size_t)r * cap_run;
   unsigned *__restrict__ hw = hits + (size_t)r * hit_words(cap_run);
   const float2 *Er = E + (size_t)r * nn;
-  const uint2 key = keys ? keys[r] : make_uint2(M.key0, M.key1);
+  const uint2 key = keys[r];
   const float expl = __expf(-M.lam);
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -794,10 +791,9 @@ static int queue_mcc_phases(Ctx *c, int mid, const MccDev &M, int R, const Speci
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_test, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_mcc_collide<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
-  const uint2 key1 = make_uint2(M.key0, M.key1);
   if (phases != kMccCollideOnly) {
     ISKRA_CUDA(c, launch_pdl(k_zero_u64, (R + 255) / 256, 256, 0, st, nwork, R, kNworkStride));
-    ISKRA_CUDA(c, launch_pdl(k_mcc_select, dim3(select_blocks, R), 256, 0, st, src, M.lam, key1, keys, d_step,
+    ISKRA_CUDA(c, launch_pdl(k_mcc_select, dim3(select_blocks, R), 256, 0, st, src, M.lam, keys, d_step,
                              phases == kMccSelectAhead ? 1 : 0, work, nwork, cap_work, err));
   }
   if (phases == kMccSelectAhead) return ISKRA_OK;

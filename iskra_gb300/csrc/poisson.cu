@@ -17,8 +17,11 @@
 //     with column electrodes -- it is solved exactly by a real FFT along y, one
 //     tridiagonal (Thomas / Sherman-Morrison for x-periodic) solve per Fourier
 //     mode along x, and an inverse FFT; the residual is then re-evaluated in
-//     FP64 and the correction repeated until ||res|| <= rtol ||rhs||;
-//   * otherwise Jacobi-preconditioned CG iterates to the same tolerance.
+//     FP64 and the correction repeated until ||res|| <= rtol ||rhs||
+//     (every ny up to 4096; the odd factor of ny by dense DFTs);
+//   * otherwise CG iterates to the same tolerance, preconditioned by a multigrid
+//     V-cycle (multigrid.cu) or, for singular operators, by Jacobi scaling;
+//   * small grids run a step's whole field part as one block (k_field_block).
 // All-periodic / all-open operators are singular; the solve then uses the
 // mean-zero gauge with the right-hand side projected onto the range (the
 // reference's dense A\b has no defined answer there; E = -∇ϕ is unaffected).
