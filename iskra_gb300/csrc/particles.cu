@@ -33,20 +33,21 @@ namespace iskra {
 // in push_t8.cu and push_t32.cu
 ISKRA_PUSH_TILE_TU(4, t16)
 cudaError_t push_tile_one_t8(cudaStream_t, bool, bool, const SpeciesDev &, const float2 *, const PushParams &, int,
-                             int, int, int *);
+                             int, int, int *, unsigned long long *);
 cudaError_t push_tile_two_t8(cudaStream_t, bool, const SpeciesDev &, const SpeciesDev &, const float2 *,
                              const PushParams &, const PushParams &, int, int, int, int *, unsigned long long *);
 cudaError_t push_tile_one_t32(cudaStream_t, bool, bool, const SpeciesDev &, const float2 *, const PushParams &, int,
-                              int, int, int *);
+                              int, int, int *, unsigned long long *);
 cudaError_t push_tile_two_t32(cudaStream_t, bool, const SpeciesDev &, const SpeciesDev &, const float2 *,
                               const PushParams &, const PushParams &, int, int, int, int *, unsigned long long *);
 
 cudaError_t push_tile_one(int ts, cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2,
-                          const PushParams &P, int ntiles, int parts, int blocks, int *err) {
+                          const PushParams &P, int ntiles, int parts, int blocks, int *err,
+                          unsigned long long *step_ctr) {
   switch (ts) {
-    case 3: return push_tile_one_t8(st, push, trk, s, E2, P, ntiles, parts, blocks, err);
-    case 4: return push_tile_one_t16(st, push, trk, s, E2, P, ntiles, parts, blocks, err);
-    case 5: return push_tile_one_t32(st, push, trk, s, E2, P, ntiles, parts, blocks, err);
+    case 3: return push_tile_one_t8(st, push, trk, s, E2, P, ntiles, parts, blocks, err, step_ctr);
+    case 4: return push_tile_one_t16(st, push, trk, s, E2, P, ntiles, parts, blocks, err, step_ctr);
+    case 5: return push_tile_one_t32(st, push, trk, s, E2, P, ntiles, parts, blocks, err, step_ctr);
   }
   return cudaErrorInvalidValue;
 }
@@ -119,21 +120,23 @@ static void mark_pushed(Species &s) {
   s.n_valid = false;
 }
 
-int launch_advance(Ctx *c, int sid, float dt) {
+static int advance_one(Ctx *c, int sid, float dt, unsigned long long *step_ctr) {
   Species &s = c->species[sid];
   int rc = clear_acc(c, s);
   if (rc) return rc;
   const int parts = push_parts(c, 1);
   ISKRA_CUDA(c, push_tile_one(c->tile_shift, c->stream, true, c->trk != nullptr, s.dev, c->E32, push_params(c, s, dt),
-                              c->ntiles, parts, push_blocks(c, 1, parts), c->d_err));
+                              c->ntiles, parts, push_blocks(c, 1, parts), c->d_err, step_ctr));
   ISKRA_CUDA(c, cudaGetLastError());
   mark_pushed(s);
   return launch_surface_charge(c);  // hit! of floating electrodes, as part of advance!
 }
 
+int launch_advance(Ctx *c, int sid, float dt) { return advance_one(c, sid, dt, nullptr); }
+
 // Every species of a step: two species with the same boundary rules in one
-// launch (k_push2, which also advances step_ctr when given: *folded), otherwise
-// one launch each.
+// launch, otherwise one launch each; the (first) launch also advances step_ctr when
+// given (*folded).
 int launch_advance_all(Ctx *c, float dt, unsigned long long *step_ctr, bool *folded) {
   if (folded) *folded = false;
   const int ns = (int)c->species.size();
@@ -153,9 +156,10 @@ int launch_advance_all(Ctx *c, float dt, unsigned long long *step_ctr, bool *fol
     return launch_surface_charge(c);
   }
   for (int s = 0; s < ns; s++) {
-    int rc = launch_advance(c, s, dt);
+    int rc = advance_one(c, s, dt, s == 0 ? step_ctr : nullptr);
     if (rc) return rc;
   }
+  if (folded) *folded = step_ctr != nullptr && ns > 0;
   return ISKRA_OK;
 }
 
@@ -171,7 +175,7 @@ int launch_deposit(Ctx *c, int sid) {
   P.tiles_x = c->tiles_x;
   const int parts = push_parts(c, 1);
   ISKRA_CUDA(c, push_tile_one(c->tile_shift, c->stream, false, false, s.dev, c->E32, P, c->ntiles, parts,
-                              push_blocks(c, 1, parts), c->d_err));
+                              push_blocks(c, 1, parts), c->d_err, nullptr));
   ISKRA_CUDA(c, cudaGetLastError());
   s.acc_valid = true;
   s.acc_zero = false;

@@ -813,14 +813,16 @@ __device__ __forceinline__ void push_block(const SpeciesDev &s, const PushParams
 }
 
 // TRK: with the surface tracker (a separate instantiation keeps the walk's
-// registers out of the push without one)
+// registers out of the push without one).  step_ctr as in k_push2.
 template <bool PUSH, int MX, int MY, bool TRK, int TS>
 __global__ void __launch_bounds__(kPushBlock, TRK ? ISKRA_PUSH_TRK_MIN_BLOCKS : ISKRA_PUSH_MIN_BLOCKS)
-    k_push(SpeciesDev s, const float2 *__restrict__ E2, PushParams P, int ntiles, int parts, int *err) {
+    k_push(SpeciesDev s, const float2 *__restrict__ E2, PushParams P, int ntiles, int parts, int *err,
+           unsigned long long *step_ctr) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char push_smem[];
   TileShared<TS> &sh = *reinterpret_cast<TileShared<TS> *>(push_smem);
   const int b = blockIdx.x, nt = ntiles * parts;
+  if (step_ctr && b == 0 && threadIdx.x == 0) *step_ctr += 1ull;
   if (b < nt) push_block<PUSH, MX, MY, TRK, TS>(s, P, E2, sh, b / parts, b % parts, parts, err);
   else push_block<PUSH, MX, MY, TRK, TS>(s, P, E2, sh, -1, b - nt, gridDim.x - nt, err);
 }
@@ -867,17 +869,18 @@ struct PushTile {
   }
   // one species: push (push = true) or deposit only
   static cudaError_t one(cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2,
-                         const PushParams &P, int ntiles, int parts, int blocks, int *err) {
+                         const PushParams &P, int ntiles, int parts, int blocks, int *err,
+                         unsigned long long *step_ctr) {
     if (!push) {
       auto kern = k_push<false, 0, 0, false, TS>;
       prepare(kern);
-      return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, parts, err);
+      return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, parts, err, step_ctr);
     }
 #define ISKRA_PUSH_CASE(MX, MY)                                                                \
   if (P.mode_x == MX && P.mode_y == MY) {                                                      \
     auto kern = trk ? k_push<true, MX, MY, true, TS> : k_push<true, MX, MY, false, TS>;        \
     prepare(kern);                                                                             \
-    return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, parts, err);             \
+    return launch_pdl(kern, blocks, kPushBlock, kSmem, st, s, E2, P, ntiles, parts, err, step_ctr);   \
   }
     ISKRA_PUSH_CASE(0, 0) ISKRA_PUSH_CASE(0, 1) ISKRA_PUSH_CASE(0, 2)
     ISKRA_PUSH_CASE(1, 0) ISKRA_PUSH_CASE(1, 1) ISKRA_PUSH_CASE(1, 2)
@@ -905,14 +908,16 @@ struct PushTile {
 
 // entry points of the per-tile-size translation units
 cudaError_t push_tile_one(int ts, cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2,
-                          const PushParams &P, int ntiles, int parts, int blocks, int *err);
+                          const PushParams &P, int ntiles, int parts, int blocks, int *err,
+                          unsigned long long *step_ctr);
 cudaError_t push_tile_two(int ts, cudaStream_t st, bool trk, const SpeciesDev &a, const SpeciesDev &b,
                           const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles, int parts, int blocks,
                           int *err, unsigned long long *step_ctr);
 #define ISKRA_PUSH_TILE_TU(TS, NAME)                                                                          \
   cudaError_t push_tile_one_##NAME(cudaStream_t st, bool push, bool trk, const SpeciesDev &s, const float2 *E2, \
-                                   const PushParams &P, int ntiles, int parts, int blocks, int *err) {                    \
-    return PushTile<TS>::one(st, push, trk, s, E2, P, ntiles, parts, blocks, err);                                    \
+                                   const PushParams &P, int ntiles, int parts, int blocks, int *err,          \
+                                   unsigned long long *step_ctr) {                                            \
+    return PushTile<TS>::one(st, push, trk, s, E2, P, ntiles, parts, blocks, err, step_ctr);                  \
   }                                                                                                            \
   cudaError_t push_tile_two_##NAME(cudaStream_t st, bool trk, const SpeciesDev &a, const SpeciesDev &b,         \
                                    const float2 *E2, const PushParams &Pa, const PushParams &Pb, int ntiles,   \

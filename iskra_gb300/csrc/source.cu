@@ -15,10 +15,7 @@
 namespace iskra {
 
 struct SourceDev {        // device-resident per-source scratch
-  long long base;         // first slot of the current sample
-  long long n;            // particles in it
-  unsigned int id0;       // first identifier
-  unsigned int pad;
+  unsigned ticket;        // blocks of the running sample that have finished
 };
 
 struct Source {
@@ -44,27 +41,16 @@ struct SourceArgs {
   unsigned long long step_value;   //   then this value
 };
 
-// reserves the slots: n = min(cap - np, floor(rate Δt)) (sources.jl:30)
-__global__ void k_source_reserve(SourceArgs A) {
-  pdl_wait();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  SpeciesState &st = *A.s.st;
-  long long n = A.cap - st.np;
-  if (n > A.nmax) n = A.nmax;
-  if (n < 0) n = 0;
-  A.d->base = st.np;
-  A.d->n = n;
-  A.d->id0 = st.next_id;
-  st.np += n;
-  st.next_id += (unsigned)n;
-}
-
 // px = rand() wx + dx, pv = randn() wv + dv (sources.jl:31-32) for slot
-// base + k; U(0,1) with 24 random bits, N(0,1) by Box-Muller (both values of
-// a pair used)
+// np + k, k < n = min(cap - np, floor(rate Δt)) (sources.jl:30); U(0,1) with 24
+// random bits, N(0,1) by Box-Muller (both values of a pair used).  Every block
+// takes np and the next identifier from the species state, which the last block to
+// finish advances (a reservation launch of its own was 2.5 us of every step).
 __global__ void k_source_fill(SourceArgs A, int *err) {
   pdl_wait();
-  const long long n = A.d->n, base = A.d->base;
+  const long long base = A.s.st->np;
+  const long long n = max(0LL, min(A.cap - base, A.nmax));
+  const uint32_t id0 = A.s.st->next_id;
   const unsigned long long step = A.step ? *A.step : A.step_value;
   const int cur = A.s.st->cur;
   float4 *xv = pick(A.s.xv[0], A.s.xv[1], cur);
@@ -89,7 +75,16 @@ __global__ void k_source_fill(SourceArgs A, int *err) {
     const long long p = base + k;
     xv[p] = make_float4((float)ux * kOffInv, (float)uy * kOffInv, vx, vy);
     zc[p] = make_float2(vz, __int_as_float(cell));
-    id[p] = A.d->id0 + (uint32_t)k;
+    id[p] = id0 + (uint32_t)k;
+  }
+  __syncthreads();  // every thread of the block has read the state
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&A.d->ticket, 1u) == gridDim.x - 1) {
+      A.d->ticket = 0u;
+      A.s.st->np = base + n;
+      A.s.st->next_id = id0 + (uint32_t)n;
+    }
   }
 }
 
@@ -123,7 +118,6 @@ int launch_source(Ctx *c, int src, double dt, uint64_t seed, const unsigned long
   A.src = (uint32_t)src;
   A.step = step;
   A.step_value = step_value;
-  ISKRA_CUDA(c, launch_pdl(k_source_reserve, 1, 32, 0, c->stream, A));
   const long long blocks = std::min<long long>((A.nmax + 255) / 256, (long long)c->num_sms * 8);
   ISKRA_CUDA(c, launch_pdl(k_source_fill, (int)std::max(1LL, blocks), 256, 0, c->stream, A, c->d_err));
   ISKRA_CUDA(c, cudaGetLastError());
