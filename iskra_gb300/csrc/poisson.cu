@@ -26,6 +26,7 @@
 // mean-zero gauge with the right-hand side projected onto the range (the
 // reference's dense A\b has no defined answer there; E = -∇ϕ is unaffected).
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -1660,16 +1661,24 @@ static int build_device(Ctx *c, Poisson *P) {
     if (!rows[r].fixed) P->dsum += d[r];
   // classes
   bool rho_fixed = false;
-  std::map<std::vector<double>, int> cmap;
+  // (a row mostly repeats the one before it: the table is searched only where it
+  // does not.  Searched for every row, a 512 x 512 operator's first step took 29.5 ms
+  // instead of 23.8.)
+  typedef std::array<double, 10> RowKey;
+  std::map<RowKey, int> cmap;
   std::vector<RowClass> classes;
   std::vector<uint16_t> cls(nn);
+  RowKey prev{};
+  int prev_id = -1;
   for (int r = 0; r < nn; r++) {
     const RowEff &e = rows[r];
-    std::vector<double> key = {e.c0, e.cW, e.cE, e.cS, e.cN, e.fixed ? 1.0 : 0.0, e.rho ? 1.0 : 0.0,
+    const RowKey key = {e.c0, e.cW, e.cE, e.cS, e.cN, e.fixed ? 1.0 : 0.0, e.rho ? 1.0 : 0.0,
                                (double)e.sig_dof, e.sig_coef, e.fixed ? 0.0 : d[r]};
-    auto it = cmap.find(key);
-    int id;
-    if (it == cmap.end()) {
+    int id = prev_id;
+    const bool repeats = prev_id >= 0 && key == prev;
+    auto it = repeats ? cmap.end() : cmap.find(key);
+    if (repeats) {
+    } else if (it == cmap.end()) {
       id = (int)classes.size();
       if (id > (int)kClassMask) return set_err(c, ISKRA_EINVAL, "too many distinct operator rows");
       cmap[key] = id;
@@ -1706,6 +1715,8 @@ static int build_device(Ctx *c, Poisson *P) {
     } else {
       id = it->second;
     }
+    prev = key;
+    prev_id = id;
     cls[r] = (uint16_t)(id | (e.fixed ? kFixedBit : 0u));
     rho_fixed |= e.fixed && e.rho;
   }
