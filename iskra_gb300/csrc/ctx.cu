@@ -322,6 +322,7 @@ int iskra_ctx_create(const iskra_grid_t *g, uint64_t stream, iskra_ctx **out) {
             cudaMalloc(&c->vol_inv_df, nn * sizeof(float2)) == cudaSuccess &&
             cudaMalloc(&c->d_err, sizeof(int)) == cudaSuccess &&
             cudaMallocHost(&c->h_err, sizeof(int)) == cudaSuccess &&
+            cudaMallocHost(&c->h_status, sizeof(StepStatus)) == cudaSuccess &&
             cudaMalloc(&c->cell_count, ((size_t)c->nkeys_cap + 1) * sizeof(int)) == cudaSuccess &&
             cudaMalloc(&c->cell_cursor, ((size_t)c->nkeys_cap + 1) * sizeof(int)) == cudaSuccess &&
             cudaMalloc(&c->scan_tmp, ((size_t)c->nkeys_cap / 4096 + 2) * sizeof(int)) == cudaSuccess &&
@@ -396,6 +397,7 @@ int iskra_ctx_destroy(iskra_ctx *h) {
   cudaFree(c->bg_df);
   cudaFree(c->d_err);
   if (c->h_err) cudaFreeHost(c->h_err);
+  if (c->h_status) cudaFreeHost(c->h_status);
   cudaFree(c->cell_count);
   cudaFree(c->cell_cursor);
   cudaFree(c->scan_tmp);

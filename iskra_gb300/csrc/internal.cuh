@@ -357,6 +357,10 @@ int mg_queue_cycle(struct Ctx *c, Mg *m, const double *r, double *z, const int *
                    bool *dots_done);
 int mg_levels(const Mg *m);
 void mg_destroy(Mg *m);
+struct StepStatus {            // what a step reports to the host as soon as its solve has ended (pinned memory)
+  int err;                     // the error flag
+  int there;                   // set after err
+};
 struct CircuitDev {            // device-resident circuit state (FP64)
   double R, L, C, amp, freq, dc, area, scale;
   double t, i, q, vext;
@@ -457,6 +461,7 @@ struct Ctx {
   bool rho_df_valid = false;   // rho_df holds ρ
   int *d_err = nullptr;        // device error flags
   int *h_err = nullptr;        // pinned mirror
+  StepStatus *h_status = nullptr;  // pinned
   // scratch for scans / sort
   int *cell_count = nullptr;   // (nkeys + 1)
   int *cell_cursor = nullptr;  // (nkeys + 1)

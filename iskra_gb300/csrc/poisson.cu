@@ -2441,7 +2441,8 @@ struct FieldBlock {
   EOut eo;
   MgBlock mg;
   double idx2, idx1, idy2, idy1;  // 1/(2Δx), ... of the CG path's FP64 field
-  int *err, *notconv;
+  int *err;
+  StepStatus *status;          // for the host, which waits for it, or nullptr
 };
 constexpr int kFieldThreads = 512, kFieldMgIterations = 10000;
 // MODE: 0 ny = 2, 1 ny another power of two, 2 any other ny (direct solves); 3
@@ -2561,7 +2562,10 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
     int it = 0;
     bool done = (rhs2 > 0 && res2 <= P.rtol2 * rhs2) || res2 == 0.0;
     const MgSh q = mg_sh(lev, P.mg.lv[0]);
-    while (!done && it < kFieldMgIterations) {
+    // (a residual that is no number, or a direction without energy, stays so: the
+    // rest of the iterations would only hold the device)
+    bool stuck = !isfinite(res2);
+    while (!done && !stuck && it < kFieldMgIterations) {
       for (int k = tid; k < nn; k += T) q.b[k] = (float)r64[k];
       __syncthreads();
       mg_bottom_cycle(lev, P.mg.lv, 0, P.mg.L, ci);
@@ -2609,6 +2613,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
       res2 = t1[0];
       it++;
       done = (rhs2 > 0 && res2 <= P.rtol2 * rhs2) || res2 == 0.0;
+      stuck = alpha == 0 || !isfinite(res2);
     }
     if (tid == 0) {
       sc->rhs2 = rhs2;
@@ -2617,7 +2622,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
       sc->iters = it;
       sc->done = done;
       sc->e_pending = 0;
-      if (!done) atomicOr(P.notconv, DERR_NOTCONV);
+      if (!done) atomicOr(P.err, DERR_NOTCONV);
     }
   }
   for (int s = 0; !MG; s++) {
@@ -2649,7 +2654,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
         sc->iters = s;
         sc->done = done;
         sc->e_pending = 0;
-        if (!done) atomicOr(P.notconv, DERR_NOTCONV);
+        if (!done) atomicOr(P.err, DERR_NOTCONV);
       }
       break;
     }
@@ -2681,6 +2686,13 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
       fft_inv_item<DF, ODD>(0, spec, nx, P.F, TP, P.op.cls, xd, x64, fbuf);
     }
     __syncthreads();
+  }
+  // Every flag of the step is set: its kernels ended before this one, and the
+  // block's own flags were set before barriers above or by this thread.
+  if (P.status && tid == 0) {
+    P.status->err = *(volatile int *)P.err;
+    __threadfence_system();
+    *(volatile int *)&P.status->there = 1;
   }
   // E, and ϕ to memory
   for (int k = tid; k < nn; k += T) {
@@ -2779,8 +2791,8 @@ int launch_field_block(Ctx *c, double rtol) {
   B.nn = P->nn;
   B.eo = eout(c, true);
   B.err = c->d_err;
-  B.notconv = c->d_err;
   if (!P->separable) {
+    B.status = c->h_status;
     mg_block_view(P->mg, &B.mg);
     B.idx2 = 1.0 / (2 * c->g.dx);
     B.idx1 = 1.0 / c->g.dx;
