@@ -328,17 +328,29 @@ __global__ void k_lambda(const double *__restrict__ part, int nparts, double dsu
   if (threadIdx.x == 0) sc->lambda = dsum > 0 ? s / dsum : 0.0;
 }
 
+static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
+
 // Optional E = -∇ϕ output of k_residual (generalized_poisson.jl:398-410):
 // FP32 node values: the MCC target term and, staged per tile, the gather.
 // The node differences are taken in FP64 (ϕ is ~10^2-10^3 V while neighbour
-// differences are ~10^-1 V) and scaled in FP32.
+// differences are ~10^-1 V) and scaled in FP32, or wholly in FP64 (exact).
 struct EOut {
   float2 *E32;
   float idx2, idx1, idy2, idy1;  // 1/(2Δx), 1/Δx, 1/(2Δy), 1/Δy
+  int exact;                     // FP64 down to the last rounding, as k_efield
+  double dx2, dx1, dy2, dy1;     // (exact) the same
 };
 
 __device__ __forceinline__ void efield_at(const double *__restrict__ x, int k, int i, int j, int nx, int ny,
                                           const EOut &eo) {
+  if (eo.exact) {
+    const double ex = i == 0 ? (x[k] - x[k + 1]) * eo.dx1
+                             : i == nx - 1 ? (x[k - 1] - x[k]) * eo.dx1 : (x[k - 1] - x[k + 1]) * eo.dx2;
+    const double ey = j == 0 ? (x[k] - x[k + nx]) * eo.dy1
+                             : j == ny - 1 ? (x[k - nx] - x[k]) * eo.dy1 : (x[k - nx] - x[k + nx]) * eo.dy2;
+    eo.E32[k] = make_float2((float)ex, (float)ey);
+    return;
+  }
   float ex, ey;
   if (i == 0) ex = (float)(x[k] - x[k + 1]) * eo.idx1;
   else if (i == nx - 1) ex = (float)(x[k - 1] - x[k]) * eo.idx1;
@@ -1549,7 +1561,7 @@ static int fft_smem_attr(Ctx *c);
 // of the recomputed one, and so does a context with a learned warm start,
 // which works on CG solves.
 static bool direct_solve(Ctx *c, const Poisson *P, double rtol) {
-  return P->sep_form && ((P->ny & (P->ny - 1)) == 0 || (!c->lws && rtol >= 1e-9));
+  return P->sep_form && (power_of_two(P->ny) || (!c->lws && rtol >= 1e-9));
 }
 
 // Effective rows and the symmetrising scale d of the free rows (breadth-first
@@ -2092,6 +2104,11 @@ static EOut eout(Ctx *c, bool on) {
   e.idx1 = (float)(1.0 / c->g.dx);
   e.idy2 = (float)(1.0 / (2 * c->g.dy));
   e.idy1 = (float)(1.0 / c->g.dy);
+  e.exact = !c->ps->separable || !power_of_two(c->ny);
+  e.dx2 = 1.0 / (2 * c->g.dx);
+  e.dx1 = 1.0 / c->g.dx;
+  e.dy2 = 1.0 / (2 * c->g.dy);
+  e.dy1 = 1.0 / c->g.dy;
   return e;
 }
 
@@ -2150,7 +2167,6 @@ static int fft_smem_attr(Ctx *c) {
   constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
   if (P->odd > 1) {
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_fwd<true>, kAttr, smem));
-    ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<true, true>, kAttr, smem));
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_inv_update<false, true>, kAttr, smem));
   } else {
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_fft_fwd<false>, kAttr, smem));
@@ -2295,9 +2311,8 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
                                  (const float *)P->q, (const float *)P->gk, (int)P->cyclic, P->pin_k0, sc));
       }
       if (P->df_mode) {
-        ISKRA_CUDA(c, launch_pdl(odd ? k_fft_inv_update<true, true> : k_fft_inv_update<true, false>, sh.fb, 256,
-                                 sh.smem, st, (const float2 *)P->spec, P->nx, F, sh.TP, (const uint16_t *)P->cls,
-                                 P->xd, (double *)nullptr, sc));
+        ISKRA_CUDA(c, launch_pdl(k_fft_inv_update<true, false>, sh.fb, 256, sh.smem, st, (const float2 *)P->spec,
+                                 P->nx, F, sh.TP, (const uint16_t *)P->cls, P->xd, (double *)nullptr, sc));
         ISKRA_CUDA(c, launch_pdl(k_residual_df<false, true>, B, T, 0, st, op, (const float2 *)P->xd,
                                  (const double *)nullptr, (const float2 *)nullptr, make_float2(0.f, 0.f), nie,
                                  P->bd, P->scal, P->r32, P->part, nn,
@@ -2440,7 +2455,6 @@ struct FieldBlock {
   CrArgs C;
   EOut eo;
   MgBlock mg;
-  double idx2, idx1, idy2, idy1;  // 1/(2Δx), ... of the CG path's FP64 field
   int *err;
   StepStatus *status;          // for the host, which waits for it, or nullptr
 };
@@ -2697,14 +2711,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
   // E, and ϕ to memory
   for (int k = tid; k < nn; k += T) {
     const int j = k / nx, i = k - j * nx;
-    if (MG) {  // in FP64 as k_efield
-      const double ex = i == 0 ? (x64[k] - x64[k + 1]) * P.idx1
-                               : i == nx - 1 ? (x64[k - 1] - x64[k]) * P.idx1 : (x64[k - 1] - x64[k + 1]) * P.idx2;
-      const double ey = j == 0 ? (x64[k] - x64[k + nx]) * P.idy1
-                               : j == ny - 1 ? (x64[k - nx] - x64[k]) * P.idy1 : (x64[k - nx] - x64[k + nx]) * P.idy2;
-      P.eo.E32[k] = make_float2((float)ex, (float)ey);
-      P.x[k] = x64[k];
-    } else if (DF) {
+    if (DF) {
       const int w = i > 0 ? k - 1 : k + nx - 1, e = i < nx - 1 ? k + 1 : k - nx + 1;
       const int so = j > 0 ? k - nx : k + nx * (ny - 1), no = j < ny - 1 ? k + nx : k - nx * (ny - 1);
       efield_df5(xd[k], xd[w], xd[e], xd[so], xd[no], k, i, j, nx, ny, P.eo);
@@ -2794,10 +2801,6 @@ int launch_field_block(Ctx *c, double rtol) {
   if (!P->separable) {
     B.status = c->h_status;
     mg_block_view(P->mg, &B.mg);
-    B.idx2 = 1.0 / (2 * c->g.dx);
-    B.idx1 = 1.0 / c->g.dx;
-    B.idy2 = 1.0 / (2 * c->g.dy);
-    B.idy1 = 1.0 / c->g.dy;
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_field_block<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kFieldSmem));
     ISKRA_CUDA(c, launch_pdl(k_field_block<false, 3>, 1, kFieldThreads, 40 * (size_t)P->nn + B.mg.bytes, c->stream, B));
@@ -2807,7 +2810,7 @@ int launch_field_block(Ctx *c, double rtol) {
   B.F = FftPlan{P->N, P->log2p, P->odd, P->tw, P->tw + P->N / 2};
   B.C = cr_args(P, P->K);
   const int mode = P->N == 2 ? 0 : P->odd > 1 ? 2 : 1;
-  auto kern = df ? (mode == 0 ? k_field_block<true, 0> : mode == 1 ? k_field_block<true, 1> : k_field_block<true, 2>)
+  auto kern = df ? (mode == 0 ? k_field_block<true, 0> : k_field_block<true, 1>)
                  : (mode == 0 ? k_field_block<false, 0> : mode == 1 ? k_field_block<false, 1> : k_field_block<false, 2>);
   ISKRA_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFieldSmem));
   ISKRA_CUDA(c, launch_pdl(kern, 1, kFieldThreads, field_block_bytes(P), c->stream, B));
@@ -3039,8 +3042,11 @@ int poisson_sync_x(Ctx *c) {
 // keeps ϕ to ~48 bits; its residual floor (~2^-47 |A||x| / ||rhs||, 5e-13
 // measured at 512^2) is far below 1e-9, so tolerances from 1e-9 up run on
 // the FP32 pipes.  Tighter tolerances and operators with σ dofs (whose rows
-// mix 1/Δx and 1/Δx^2 scales) keep the FP64 state.
-static bool want_df(const Poisson *P, double rtol) { return P->separable && P->nsig == 0 && rtol >= 1e-9; }
+// mix 1/Δx and 1/Δx^2 scales) keep the FP64 state, and so do operators whose ny
+// is no power of two: they were CG solves, in FP64.
+static bool want_df(const Poisson *P, double rtol) {
+  return P->separable && power_of_two(P->ny) && P->nsig == 0 && rtol >= 1e-9;
+}
 
 // Puts the solver that direct_solve picks in effect (outside stream capture);
 // the multigrid hierarchy is built when CG first needs it.
