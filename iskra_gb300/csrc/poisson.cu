@@ -337,8 +337,8 @@ static bool power_of_two(int n) { return (n & (n - 1)) == 0; }
 struct EOut {
   float2 *E32;
   float idx2, idx1, idy2, idy1;  // 1/(2Δx), 1/Δx, 1/(2Δy), 1/Δy
-  int exact;                     // FP64 down to the last rounding, as k_efield
-  double dx2, dx1, dy2, dy1;     // (exact) the same
+  int exact = 0;                 // FP64 down to the last rounding, as k_efield
+  double dx2 = 0, dx1 = 0, dy2 = 0, dy1 = 0;  // (exact) the same
 };
 
 __device__ __forceinline__ void efield_at(const double *__restrict__ x, int k, int i, int j, int nx, int ny,
