@@ -89,6 +89,7 @@ struct Poisson {
   // ---- device representation ----
   bool separable = false, singular = false, cyclic = false;
   bool sep_form = false;        // the operator separates (direct_solve decides whether it is solved so)
+  double stalled = 0;           // largest tolerance at which a direct solve stalled
   int nclass = 0;
   uint16_t *cls = nullptr;      // nn
   RowClass *classes = nullptr;
@@ -377,8 +378,18 @@ constexpr int kSmemClasses = 128;  // row-class table held in shared memory up t
 // In a step graph the residual of the last sweep flags DERR_NOTCONV (in
 // *notconv) when the solve stops above tolerance.
 struct SweepLoop {
-  int *notconv;
+  int *notconv;        // the last pass of a step graph: where an unmet tolerance is flagged
+  StepStatus *status;  // where the pass that ends the solve reports to the host, or nullptr
+  const int *err;      // (status) the error flag
 };
+
+// The step's error flag to the host, by one thread, when every kernel or phase that
+// may set it has ended.
+__device__ __forceinline__ void report_step(StepStatus *status, const int *err) {
+  status->err = *(const volatile int *)err;
+  __threadfence_system();
+  *(volatile int *)&status->there = 1;
+}
 
 // Residual of free row k: res = b - λ - A x, returned scaled as -d res in
 // FP32 (r64 != nullptr also receives it in FP64); 0 on fixed rows.  The
@@ -477,6 +488,7 @@ __device__ __forceinline__ void finish_norms(PoissonScal *sc, double *__restrict
     sc->done = done;
     if (FIRST) sc->e_pending = done;
     if (loop.notconv && !done) atomicOr(loop.notconv, DERR_NOTCONV);
+    if (loop.status && (done || loop.notconv)) report_step(loop.status, loop.err);
   }
 }
 
@@ -1559,9 +1571,11 @@ static int fft_smem_attr(Ctx *c);
 // 3.66 ms with multigrid CG, 0.10 ms directly); tighter ones keep CG, whose
 // recursively updated residual reaches tolerances below the rounding floor
 // of the recomputed one, and so does a context with a learned warm start,
-// which works on CG solves.
+// which works on CG solves, and an operator whose direct solve has stalled at this
+// tolerance (solve_sync): the floor of the recomputed residual grows with nx^2 for a
+// smooth ρ (uniform ρ: 6e-10 at 4096 columns, 4.6e-9 at 12000).
 static bool direct_solve(Ctx *c, const Poisson *P, double rtol) {
-  return P->sep_form && (power_of_two(P->ny) || (!c->lws && rtol >= 1e-9));
+  return P->sep_form && (power_of_two(P->ny) || (!c->lws && rtol >= 1e-9 && rtol > P->stalled));
 }
 
 // Effective rows and the symmetrising scale d of the free rows (breadth-first
@@ -1758,6 +1772,7 @@ static int build_device(Ctx *c, Poisson *P) {
     }
   }
   P->sep_form = sep;
+  P->stalled = 0;
   P->separable = direct_solve(c, P, 1.0);
   // ---- multigrid preconditioner of the CG path ----
   mg_destroy(P->mg);
@@ -2291,7 +2306,8 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
   const double nie = -1.0 / P->eps0;
   const double rtol2 = rtol * rtol;
   cudaStream_t st = c->stream;
-  const SweepLoop none{};
+  SweepLoop mid = loop;  // all but the last pass
+  mid.notconv = nullptr;
   if (P->separable) {
     const SepShape sh = sep_shape(c);
     const int K = P->K;
@@ -2316,14 +2332,14 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
         ISKRA_CUDA(c, launch_pdl(k_residual_df<false, true>, B, T, 0, st, op, (const float2 *)P->xd,
                                  (const double *)nullptr, (const float2 *)nullptr, make_float2(0.f, 0.f), nie,
                                  P->bd, P->scal, P->r32, P->part, nn,
-                                 (int)P->singular, rtol2, eout(c, true), last ? loop : none));
+                                 (int)P->singular, rtol2, eout(c, true), last ? loop : mid));
       } else {
         ISKRA_CUDA(c, launch_pdl(odd ? k_fft_inv_update<false, true> : k_fft_inv_update<false, false>, sh.fb, 256,
                                  sh.smem, st, (const float2 *)P->spec, P->nx, F, sh.TP, (const uint16_t *)P->cls,
                                  (float2 *)nullptr, P->x, sc));
         ISKRA_CUDA(c, launch_pdl(k_residual<false, true>, B, T, 0, st, op, (const double *)P->x,
                                  (const double *)c->rho, nie, P->scal, (double *)nullptr, P->r32, P->part, nn,
-                                 (int)P->singular, rtol2, eout(c, true), last ? loop : none));
+                                 (int)P->singular, rtol2, eout(c, true), last ? loop : mid));
       }
     }
   } else if (P->mg) {  // flexible PCG, one multigrid V-cycle per iteration
@@ -2372,11 +2388,10 @@ static int queue_sweeps(Ctx *c, double rtol, int count, bool reset_cg, SweepLoop
 
 // Sweeps a step graph runs per solve (each skipped on the device once the
 // residual meets rtol): one FP32 correction reduces the residual by about
-// 10^-5 (cold start) and the step starts from the previous potential.  One
-// more with an odd factor in ny (CG, which solved those operators before,
-// had no such limit).
-static int graph_sweeps(const Poisson *P, double rtol) {
-  const int n = (int)std::ceil(std::log(rtol) / std::log(1e-5)) + (P->odd > 1 ? 1 : 0);
+// 10^-5 (cold start) and the step starts from the previous potential.  (ny with
+// an odd factor: the host goes on with the solve where these are not enough.)
+static int graph_sweeps(double rtol) {
+  const int n = (int)std::ceil(std::log(rtol) / std::log(1e-5));
   return std::max(2, std::min(8, n));
 }
 
@@ -2399,17 +2414,21 @@ static int finish_solve(Ctx *c) {
   return launch_efield_from(c, P->x);
 }
 
+// Whether the host looks at a step's errors before it launches the next one: CG
+// operators, and the direct solves of other ny, which were CG solves.
+bool poisson_step_checked(Ctx *c) { return !c->ps->separable || !power_of_two(c->ps->ny); }
+
 // Solve queued inside a step capture (separable operators).
 int poisson_solve_graph(Ctx *c, double rtol) {
   int rc = poisson_prepare(c);
   if (rc) return rc;
   Poisson *P = c->ps;
   if (!P->separable) return set_err(c, ISKRA_EINVAL, "graph solve needs a separable operator");
-  const int n = graph_sweeps(P, rtol);
-  const SweepLoop none{}, last{c->d_err};
-  rc = queue_prologue(c, rtol, c->graph_dt, none, true);
+  const int n = graph_sweeps(rtol);
+  StepStatus *status = poisson_step_checked(c) ? c->h_status : nullptr;
+  rc = queue_prologue(c, rtol, c->graph_dt, SweepLoop{nullptr, status, c->d_err}, true);
   if (rc) return rc;
-  rc = queue_sweeps(c, rtol, n, false, last);
+  rc = queue_sweeps(c, rtol, n, false, SweepLoop{c->d_err, status, c->d_err});
   if (rc) return rc;
   return finish_solve(c);
 }
@@ -2703,11 +2722,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_block(FieldBlock P) {
   }
   // Every flag of the step is set: its kernels ended before this one, and the
   // block's own flags were set before barriers above or by this thread.
-  if (P.status && tid == 0) {
-    P.status->err = *(volatile int *)P.err;
-    __threadfence_system();
-    *(volatile int *)&P.status->there = 1;
-  }
+  if (P.status && tid == 0) report_step(P.status, P.err);
   // E, and ϕ to memory
   for (int k = tid; k < nn; k += T) {
     const int j = k / nx, i = k - j * nx;
@@ -2794,12 +2809,12 @@ int launch_field_block(Ctx *c, double rtol) {
   B.bfix = P->bfix_d;
   B.singular = P->singular;
   B.rho_fixed = P->rho_fixed;
-  B.sweeps = std::min(8, graph_sweeps(P, rtol) + 2);  // (sweeps not needed cost nothing here)
+  B.sweeps = std::min(8, graph_sweeps(rtol) + 2);  // (sweeps not needed cost nothing here)
   B.nn = P->nn;
   B.eo = eout(c, true);
   B.err = c->d_err;
+  B.status = poisson_step_checked(c) ? c->h_status : nullptr;
   if (!P->separable) {
-    B.status = c->h_status;
     mg_block_view(P->mg, &B.mg);
     ISKRA_CUDA(c, cudaFuncSetAttribute(k_field_block<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kFieldSmem));
@@ -2894,6 +2909,7 @@ static int lws_line_search(Ctx *c, const float *y, const double *scale) {
 // step graphs).  step: the solve of an iskra_step (CG operators), which
 // starts from ϕ extrapolated in time like the graph path; other solves
 // start from ϕ and end the extrapolation history.
+static int choose_solver(Ctx *c, double rtol);
 static int solve_sync(Ctx *c, double rtol, int maxit, int *iters, double *relres, bool step = false) {
   int rc = poisson_prepare(c);
   if (rc) return rc;
@@ -2905,6 +2921,7 @@ static int solve_sync(Ctx *c, double rtol, int maxit, int *iters, double *relres
                              (void *)P->x, P->xh, P->nn, P->scal));
   bool first = true, lws_pending = false;
   int done_it = 0;
+  double last_relres = INFINITY;
   const SweepLoop none{};
   for (;;) {
     // (multigrid CG: as many iterations as the last solve took before the
@@ -2980,6 +2997,21 @@ static int solve_sync(Ctx *c, double rtol, int maxit, int *iters, double *relres
     ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
     done_it = P->scal_h->iters;
     if (P->scal_h->done || done_it >= maxit) break;
+    if (P->separable && !power_of_two(P->ny)) {
+      // two corrections that gain less than a factor of 10: the rounding floor is
+      // above the tolerance, which CG, as it was before these operators were solved
+      // directly, meets with its updated residual
+      const double now = P->scal_h->relres;
+      if (!std::isfinite(now)) break;
+      if (!(now < 0.1 * last_relres)) {
+        P->stalled = rtol;
+        rc = choose_solver(c, rtol);
+        if (rc) return rc;
+        first = true;
+        done_it = 0;
+      }
+      last_relres = now;
+    }
   }
   rc = finish_solve(c);
   if (rc) return rc;

@@ -18,6 +18,7 @@ const double *poisson_x_ptr(Ctx *c);
 const float2 *poisson_xd_ptr(Ctx *c);
 void poisson_mark_x_stale(Ctx *c);
 bool poisson_separable(Ctx *c);
+bool poisson_step_checked(Ctx *c);
 int poisson_solve_blocking(Ctx *c, double rtol, int maxit);
 int poisson_solve_graph(Ctx *c, double rtol);
 
@@ -130,12 +131,13 @@ static int update_sort_periods(Ctx *c, double dt) {
 static bool tail_wants_sort(const Species &s) { return s.tail >= 4096 && 8 * s.tail >= s.cap; }
 
 // Waits until the launched step's solve has ended and returns the step's errors.  The
-// field kernel reports through pinned memory before it writes E and ϕ, so that the
-// next step's launch overlaps its end (10 x 10 nodes, µs per step: 66; waiting for
-// the stream: 70; no look before the call ends: 64).  A solve short of its
-// tolerance comes first and leaves the other flags to the next call, as in
+// solve's last kernel reports through pinned memory before it writes E and ϕ, so that
+// the next step's launch overlaps its end (10 x 10 nodes, µs per step: 66; waiting
+// for the stream: 70; no look before the call ends: 64).  A direct solve short of
+// its tolerance goes on under the host's checks; a CG solve that is ends the step,
+// before the other flags, which it leaves to the next call, as in
 // poisson_solve_blocking.
-static int step_errors(Ctx *c) {
+static int step_errors(Ctx *c, double rtol) {
   volatile int *there = &c->h_status->there;
   for (unsigned n = 1; !*there; n++)
     if (n % 1024 == 0) {  // (a launch that failed never reports)
@@ -152,6 +154,7 @@ static int step_errors(Ctx *c) {
   *c->h_err = f & ~DERR_NOTCONV;
   ISKRA_CUDA(c, cudaMemcpyAsync(c->d_err, c->h_err, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   ISKRA_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (poisson_separable(c)) return poisson_solve_blocking(c, rtol, 10000);
   return set_err(c, ISKRA_ENOTCONV, "Poisson solve did not reach the tolerance");
 }
 
@@ -317,8 +320,7 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
       rc = launch_sort(c, s);
       if (rc) return rc;
     }
-  const bool direct = poisson_separable(c);
-  if (!direct && !poisson_one_block(c)) {
+  if (!poisson_separable(c) && !poisson_one_block(c)) {
     // eager path: CG needs host-side convergence checks
     for (int n = 0; n < nsteps; n++) {
       rc = queue_step(c, dt, seed, rtol, true);
@@ -364,28 +366,36 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
     c->species[s].n64_valid = c->g_n64[s];
     c->species[s].n_df_valid = c->g_n_df[s];
   }
+  const bool checked = poisson_step_checked(c);
   for (int n = 0; n < nsteps; n++) {
-    c->h_status->there = 0;
+    if (checked) c->h_status->there = 0;
     ISKRA_CUDA(c, cudaGraphLaunch(c->graph, c->stream));
     c->launches += c->graph_kernels;
     c->e_from_phi = true;
     poisson_mark_x_stale(c);
-    // a step of a CG operator is checked before the next one is launched, so that the
-    // call ends at the step that failed, as it does where the host runs the solve
-    if (!direct) {
-      rc = step_errors(c);
+    // checked before the next one is launched: the call ends at the step that failed,
+    // as it does where the host runs the solve
+    if (checked) {
+      rc = step_errors(c, rtol);
       if (rc) return rc;
     }
     c->step++;
     c->d_step_known = c->step;
     for (int s = 0; s < (int)c->species.size(); s++) {
       if (c->sort_period[s] > 0 && c->step % c->sort_period[s] == 0) {
+        if (!c->sort_graph[s]) {
+          rc = launch_sort(c, s);
+          if (rc) return rc;
+          continue;
+        }
         ISKRA_CUDA(c, cudaGraphLaunch(c->sort_graph[s], c->stream));
         c->launches += c->sort_graph_kernels[s];
       }
     }
+    // a solve that went over to CG dropped the captured step: the rest starts anew
+    if (!c->graph && n + 1 < nsteps) return iskra_step(h, dt, nsteps - n - 1, seed, rtol);
   }
-  return direct || !c->dl_pending ? ISKRA_OK : collect_device_errors(c);
+  return checked && c->dl_pending ? collect_device_errors(c) : ISKRA_OK;
 }
 
 // Sort-cadence autotuner: runs `trial` steps of the caller's own simulation
