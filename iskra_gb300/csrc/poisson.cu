@@ -1574,6 +1574,18 @@ static int fft_smem_attr(Ctx *c);
 // which works on CG solves, and an operator whose direct solve has stalled at this
 // tolerance (solve_sync): the floor of the recomputed residual grows with nx^2 for a
 // smooth ρ (uniform ρ: 6e-10 at 4096 columns, 4.6e-9 at 12000).
+//   The dense DFTs of the odd factor cost its square: up to kMaxOdd.  Steps at
+// 1e-8, 200 k particles, µs direct (corrections) / multigrid CG: nx = 301: 74 (1)
+// / 482 at ny = 255, 200 (2) / 580 at 1023, 349 (1) / 719 at 1533, 478 (1) / 768 at
+// 2039, 1558 (1) / 1184 at 4093; nx = 2048: 246 (2) / 834, 1286 (2) / 1804, 2098 (1)
+// / 2617, 2748 (1) / 2653.  A second correction would cost more than CG from about
+// 1500 on.  Singular operators, whose CG has no multigrid, win at any factor (ny =
+// 4093: 3.3-20 ms a solve against 117-1450).
+constexpr int kMaxOdd = 1024;
+static int odd_factor(int n) {
+  while (n % 2 == 0) n /= 2;
+  return n;
+}
 static bool direct_solve(Ctx *c, const Poisson *P, double rtol) {
   return P->sep_form && (power_of_two(P->ny) || (!c->lws && rtol >= 1e-9 && rtol > P->stalled));
 }
@@ -1749,7 +1761,7 @@ static int build_device(Ctx *c, Poisson *P) {
   P->nclass = (int)classes.size();
   P->rho_fixed = rho_fixed;
   // ---- separability: per column i, every j gives the same scaled row ----
-  bool sep = P->method == 0 && ny >= 2 && ny <= 4096;
+  bool sep = P->method == 0 && ny >= 2 && ny <= 4096 && (singular || odd_factor(ny) <= kMaxOdd);
   std::vector<double> s0(nx), sW(nx), sE(nx), ey(nx);
   std::vector<int> colfixed(nx);
   for (int i = 0; i < nx && sep; i++) {
