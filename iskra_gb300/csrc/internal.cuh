@@ -343,6 +343,7 @@ struct Species {
   bool acc_zero = true;        // acc is all zero
   bool n_valid = true;         // n matches the current positions
   long long tail = 0;          // at most this many particles sampled outside steps since the last sort
+  unsigned long long tail_next = 0;  // no sort for their sake before this step
 };
 
 struct Poisson;                // poisson.cu

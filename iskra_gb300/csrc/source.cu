@@ -190,7 +190,8 @@ int iskra_source_sample(iskra_ctx *h, int src, double dt, uint64_t seed) {
   // one-off samples take their call number as the step word, with the top
   // bit set so they never share a key with a step's sample
   const int rc = launch_source(c, src, dt, seed, nullptr, (1ull << 63) | S.calls++);
-  if (rc == ISKRA_OK) c->species[S.sid].tail += std::max(0LL, (long long)std::floor(S.rate * dt));
+  Species &s = c->species[S.sid];
+  if (rc == ISKRA_OK) s.tail = std::min(s.cap, s.tail + std::max(0LL, (long long)std::floor(S.rate * dt)));
   return rc;
 }
 

@@ -127,8 +127,14 @@ static int update_sort_periods(Ctx *c, double dt) {
 // later, against 0.9 ms sorted) and a sort costs ~0.045 ns per particle of
 // the species and its launches (~20 us; the tail push of 20 k particles on 10 x
 // 10 nodes takes 13 us longer than the tiles'), so a tail of at least an eighth
-// of the capacity pays within a few steps; a smaller one waits for the period.
-static bool tail_wants_sort(const Species &s) { return s.tail >= 4096 && 8 * s.tail >= s.cap; }
+// of the capacity pays within a few steps; a smaller one waits for the period.  At
+// most one such sort per period: the count is an upper bound (a source at the
+// species' capacity appends nothing, which only the device knows), so a program that
+// samples into a full species before every step pays no more than its periodic sorts
+// again.
+static bool tail_wants_sort(const Ctx *c, const Species &s, int period) {
+  return period > 0 && s.tail >= 4096 && 8 * s.tail >= s.cap && c->step >= s.tail_next;
+}
 
 // Waits until the launched step's solve has ended and returns the step's errors.  The
 // solve's last kernel reports through pinned memory before it writes E and ϕ, so that
@@ -184,6 +190,15 @@ static int capture(Ctx *c, cudaGraphExec_t *out, unsigned long long *kernels, F 
   cudaGraphDestroy(g);
   ISKRA_CUDA(c, ei);
   *kernels = k;
+  return ISKRA_OK;
+}
+
+// A sort of a step: the captured one, where there is one.
+static int step_sort(Ctx *c, int s) {
+  if (!c->sort_graph[s]) return launch_sort(c, s);
+  ISKRA_CUDA(c, cudaGraphLaunch(c->sort_graph[s], c->stream));
+  c->launches += c->sort_graph_kernels[s];
+  c->species[s].tail = 0;
   return ISKRA_OK;
 }
 
@@ -315,13 +330,19 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
   // particles sampled since the last sort lie in the unsorted tail, whose
   // push scatters its deposits in global memory: sort once before the steps
   // when the tail is a good part of the species
-  for (int s = 0; s < (int)c->species.size(); s++)
-    if (c->sort_period[s] > 0 && tail_wants_sort(c->species[s])) {
-      rc = launch_sort(c, s);
-      if (rc) return rc;
-    }
+  auto sort_tails = [&]() -> int {
+    for (int s = 0; s < (int)c->species.size(); s++)
+      if (tail_wants_sort(c, c->species[s], c->sort_period[s])) {
+        const int r = step_sort(c, s);
+        if (r) return r;
+        c->species[s].tail_next = c->step + c->sort_period[s];
+      }
+    return ISKRA_OK;
+  };
   if (!poisson_separable(c) && !poisson_one_block(c)) {
     // eager path: CG needs host-side convergence checks
+    rc = sort_tails();
+    if (rc) return rc;
     for (int n = 0; n < nsteps; n++) {
       rc = queue_step(c, dt, seed, rtol, true);
       if (rc) return rc;
@@ -356,10 +377,14 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
   }
   for (int s = 0; s < (int)c->species.size(); s++) {
     if (!c->sort_graph[s] && c->sort_period[s] > 0) {
+      const long long tail = c->species[s].tail;  // (the capture sorts nothing)
       rc = capture(c, &c->sort_graph[s], &c->sort_graph_kernels[s], [&]() { return launch_sort(c, s); });
+      c->species[s].tail = tail;
       if (rc) return rc;
     }
   }
+  rc = sort_tails();
+  if (rc) return rc;
   c->rho64_valid = c->g_rho64;
   c->rho_df_valid = c->g_rho_df;
   for (int s = 0; s < (int)c->species.size(); s++) {
@@ -383,13 +408,8 @@ int iskra_step(iskra_ctx *h, double dt, int nsteps, uint64_t seed, double rtol) 
     c->d_step_known = c->step;
     for (int s = 0; s < (int)c->species.size(); s++) {
       if (c->sort_period[s] > 0 && c->step % c->sort_period[s] == 0) {
-        if (!c->sort_graph[s]) {
-          rc = launch_sort(c, s);
-          if (rc) return rc;
-          continue;
-        }
-        ISKRA_CUDA(c, cudaGraphLaunch(c->sort_graph[s], c->stream));
-        c->launches += c->sort_graph_kernels[s];
+        rc = step_sort(c, s);
+        if (rc) return rc;
       }
     }
     // a solve that went over to CG dropped the captured step: the rest starts anew
