@@ -1154,9 +1154,11 @@ static void make_maps(Lws *L) {
 // microseconds each, which the host could not queue as fast as they run (256 x
 // 192: forward, then forward and backward with the copies around them 496 -> 332 us,
 // with the weight gradients beside the chain and their loads in flight).
-// Inside another capture the launches are queued as they are.
+// Inside another capture, and on the legacy default stream, which cannot be
+// captured, the launches are queued as they are.
 template <class F>
 int lws_replay(Ctx *c, cudaGraphExec_t *exec, F queue) {
+  if (c->stream == cudaStreamLegacy) return queue();
   cudaStreamCaptureStatus cs;
   ISKRA_CUDA(c, cudaStreamIsCapturing(c->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone) return queue();
