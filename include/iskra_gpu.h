@@ -257,7 +257,9 @@ int iskra_poisson_set_warm_start(iskra_ctx *ctx, int mode);
  * 1 = CG with Jacobi scaling only, 2 = multigrid-preconditioned CG even for
  * a separable operator.  Every method iterates to the same FP64 relative
  * residual.  Returns the method in effect through *active when non-NULL
- * (0 separable, 1 Jacobi CG, 2 multigrid CG). */
+ * (0 separable, 1 Jacobi CG, 2 multigrid CG): that of a solve to 1e-8 --
+ * operators whose ny is no power of two are solved directly from 1e-9 up and
+ * by CG to tighter tolerances. */
 int iskra_poisson_set_method(iskra_ctx *ctx, int method, int *active);
 
 /* ---- Monte Carlo collisions (Chemistry/src/mcc.jl) ----------------------- */

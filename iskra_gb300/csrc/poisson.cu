@@ -1582,6 +1582,7 @@ static int fft_smem_attr(Ctx *c);
 // 1500 on.  Singular operators, whose CG has no multigrid, win at any factor (ny =
 // 4093: 3.3-20 ms a solve against 117-1450).
 constexpr int kMaxOdd = 1024;
+constexpr double kReportRtol = 1e-8;  // the solver before a tolerance is known: that of the default one
 static int odd_factor(int n) {
   while (n % 2 == 0) n /= 2;
   return n;
@@ -1785,7 +1786,7 @@ static int build_device(Ctx *c, Poisson *P) {
   }
   P->sep_form = sep;
   P->stalled = 0;
-  P->separable = direct_solve(c, P, 1.0);
+  P->separable = direct_solve(c, P, kReportRtol);
   // ---- multigrid preconditioner of the CG path ----
   mg_destroy(P->mg);
   P->mg = nullptr;
@@ -3546,10 +3547,12 @@ int iskra_poisson_set_method(iskra_ctx *h, int method, int *active) {
     c->ps->method = method;
     c->ps->dirty = true;
   }
-  int rc = poisson_prepare(c);
-  if (!rc) rc = choose_solver(c, 1.0);
+  const int rc = poisson_prepare(c);
   if (rc) return rc;
-  if (active) *active = c->ps->separable ? 0 : (c->ps->mg ? 2 : 1);
+  // (the solver itself changes with the next solve, whose tolerance decides; the
+  // hierarchy of an operator solved directly so far is built when CG first needs it)
+  const Poisson *P = c->ps;
+  if (active) *active = direct_solve(c, P, kReportRtol) ? 0 : (P->method != 1 && !P->singular ? 2 : 1);
   return ISKRA_OK;
 }
 
