@@ -84,7 +84,7 @@ struct Poisson {
   bool dirty = true;
   int method = 0;               // 0 auto, 1 CG (Jacobi), 2 CG with the multigrid preconditioner
   Mg *mg = nullptr;             // multigrid hierarchy of a non-separable operator (multigrid.cu)
-  cudaGraphExec_t pcg_graph = nullptr;  // one multigrid-CG iteration (~70 kernels), replayed
+  cudaGraphExec_t pcg_graph = nullptr;  // one multigrid-CG iteration (9 to 13 kernels), replayed
   double pcg_graph_rtol = 0;
   // ---- device representation ----
   bool separable = false, singular = false, cyclic = false;
@@ -1274,11 +1274,6 @@ __global__ void k_cg_rz0(const double *__restrict__ part, int nparts, PoissonSca
 // direction and S p kernels it replaces took 43 us.
 constexpr int kApX = 32, kApY = 16, kApW = kApX + 2, kApH = kApY + 2;
 constexpr int kApThreads = (kApW * kApH + 31) / 32 * 32;
-__device__ __forceinline__ int tile_node(int i, int n) {
-  if ((unsigned)i < (unsigned)n) return i;
-  const int m = i % n;
-  return m < 0 ? m + n : m;
-}
 __global__ void __launch_bounds__(kApThreads) k_pcg_ap(OpView op, const double *__restrict__ z,
                                                        double *__restrict__ pa, double *__restrict__ pb,
                                                        double *__restrict__ ap, double *__restrict__ part,
@@ -1298,7 +1293,7 @@ __global__ void __launch_bounds__(kApThreads) k_pcg_ap(OpView op, const double *
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int ty = tile / tiles_x;
     const int gx = (tile - ty * tiles_x) * kApX - 1 + lx, gy = ty * kApY - 1 + ly;
-    const int k = tile_node(gx, nx) + nx * tile_node(gy, ny);
+    const int k = wrap_any(gx, nx) + nx * wrap_any(gy, ny);
     const bool own = lx >= 1 && lx <= kApX && ly >= 1 && ly <= kApY && gx < nx && gy < ny;
     const RowClass &C = op.classes[op.cls[k] & kClassMask];
     double p = z[k];
@@ -1565,6 +1560,21 @@ static RowEff effective_row(const Poisson *P, int r) {
 
 static int fft_smem_attr(Ctx *c);
 
+// Largest odd factor of ny solved directly: its dense DFTs cost the square.  Steps
+// at 1e-8, 200 k particles, µs direct (corrections) / multigrid CG: nx = 301: 74 (1)
+// / 482 at ny = 255, 200 (2) / 580 at 1023, 349 (1) / 719 at 1533, 478 (1) / 768 at
+// 2039, 1558 (1) / 1184 at 4093; nx = 2048: 246 (2) / 834, 1286 (2) / 1804, 2098 (1)
+// / 2617, 2748 (1) / 2653.  A second correction would cost more than CG from about
+// 1500 on.  Singular operators, whose CG has no multigrid, win at any factor (ny =
+// 4093: 3.3-20 ms a solve against 117-1450).
+constexpr int kMaxOdd = 1024;
+static int odd_factor(int n) {
+  while (n % 2 == 0) n /= 2;
+  return n;
+}
+
+constexpr double kReportRtol = 1e-8;  // stands for a tolerance that is not known yet: the default one
+
 // Whether a separable operator is solved directly (FFT along y, cyclic
 // reduction along x) for tolerance rtol.  A power-of-two ny always is.  Any
 // other ny is down to a tolerance of 1e-9 (301 x 97 slab: a step took
@@ -1574,19 +1584,6 @@ static int fft_smem_attr(Ctx *c);
 // which works on CG solves, and an operator whose direct solve has stalled at this
 // tolerance (solve_sync): the floor of the recomputed residual grows with nx^2 for a
 // smooth ρ (uniform ρ: 6e-10 at 4096 columns, 4.6e-9 at 12000).
-//   The dense DFTs of the odd factor cost its square: up to kMaxOdd.  Steps at
-// 1e-8, 200 k particles, µs direct (corrections) / multigrid CG: nx = 301: 74 (1)
-// / 482 at ny = 255, 200 (2) / 580 at 1023, 349 (1) / 719 at 1533, 478 (1) / 768 at
-// 2039, 1558 (1) / 1184 at 4093; nx = 2048: 246 (2) / 834, 1286 (2) / 1804, 2098 (1)
-// / 2617, 2748 (1) / 2653.  A second correction would cost more than CG from about
-// 1500 on.  Singular operators, whose CG has no multigrid, win at any factor (ny =
-// 4093: 3.3-20 ms a solve against 117-1450).
-constexpr int kMaxOdd = 1024;
-constexpr double kReportRtol = 1e-8;  // the solver before a tolerance is known: that of the default one
-static int odd_factor(int n) {
-  while (n % 2 == 0) n /= 2;
-  return n;
-}
 static bool direct_solve(Ctx *c, const Poisson *P, double rtol) {
   return P->sep_form && (power_of_two(P->ny) || (!c->lws && rtol >= 1e-9 && rtol > P->stalled));
 }
@@ -2449,8 +2446,8 @@ int poisson_solve_graph(Ctx *c, double rtol) {
 // ---- a step's field part in one block ------------------------------------------
 // On grids of up to kFieldBlockNodes nodes the circuit, the density pass, the warm
 // start, the driven rows, the residuals and corrections (or the whole multigrid
-// CG, up to ~1200 nodes), and E run as phases of one 512-thread block with ϕ, the right-hand side, the residual and the spectrum
-// in shared memory: at these sizes each of the 9 (double-float) to 18 (FP64,
+// CG, up to ~1300 nodes), and E run as phases of one 512-thread block with ϕ, the
+// right-hand side, the residual and the spectrum in shared memory: at these sizes each of the 9 (double-float) to 18 (FP64,
 // singular) launches they took costs 3-10 us of launch and memory latency for
 // well under a microsecond of work.  The phases are the multi-launch path's own
 // node and line functions, so ϕ, ρ and E are the same bits; only the norms'
