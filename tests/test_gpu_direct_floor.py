@@ -87,3 +87,28 @@ def test_errors_end_the_call(lib):
         assert e.value.code == 9  # ISKRA_ENOTCONV
         assert ctx.kernel_launches() == 3 * per_step
         ctx.close()
+
+
+@pytest.mark.parametrize("every", [0, 2])
+def test_going_over_to_cg_inside_a_call(lib, every):
+    """A call whose first solve stalls does the rest of its steps through CG: the same
+    bits as one call per step."""
+    nx, ny, rtol = 12000, 12, 1e-9
+    out = []
+    for calls in ([4], [1, 1, 1, 1]):
+        ctx = _ctx(nx, ny)
+        s = ctx.species_create(-QE, ME, 1e-3, 100)
+        ctx.set_boundary(s, lib.BND_WRAP, lib.BND_WRAP)
+        ctx.upload(s, *rand_particles(np.random.default_rng(nx), 100, nx, ny, 1e-3, 1e-3, 1e3))
+        ctx.set_background(np.full((nx, ny), RHO))
+        ctx.set_sort_every(every)
+        for n in calls:
+            ctx.step(1e-12, n, seed=1, rtol=rtol)
+        it, rr = ctx.solve_info()
+        assert rr <= rtol
+        x, v, ids = ctx.download(s)
+        o = np.argsort(ids)
+        out.append((ctx.field(lib.FIELD_PHI), x[o], v[o]))
+        ctx.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
